@@ -44,6 +44,8 @@ __device__ __forceinline__ float sample_z(float mn, float off, int j, float rnd)
 // last hit whose range starts at or before q (starts are non-decreasing and
 // strictly increasing over hits that get samples).  Returns #samples.
 // b: the ray's frame; S: its sample count (<= p.S, the row stride of rands).
+// IDS: node ids are written too (si); without it si is not touched.
+template <bool IDS = true>
 __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, int b, int S, int nh,
                                                float rand_const, float *sz, int *si, SampleScratch &sc) {
   const int lane = lane_id();
@@ -91,7 +93,7 @@ __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, in
       sc.start[lane] = start;
       sc.mn[lane] = mn;
       sc.off[lane] = (mx - mn) / (float)(ne + 1);
-      sc.id[lane] = id;
+      if (IDS) sc.id[lane] = id;
       __syncwarp();
       const int end = min(has + __shfl_sync(SG_FULL, incl, 31), S);
       // owners are among the lanes with samples; lanes past the last of
@@ -106,7 +108,7 @@ __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, in
           else up = mid - 1;
         }
         sz[q] = sample_z(sc.mn[lo], sc.off[lo], q - sc.start[lo], jitter(q));
-        si[q] = sc.id[lo];
+        if (IDS) si[q] = sc.id[lo];
       }
       __syncwarp();
       has = end;
@@ -116,19 +118,18 @@ __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, in
     const int left = S - has;
     const int cnt = left < nvalid ? left : nvalid;
     for (int i = lane; i < cnt; i += 32) {
-      const int id = __ldg(hi + i);
       const float mn = __ldg(h0 + i), mx = __ldg(h1 + i);
       const float off = (mx - mn) * 0.5f;
       const float base = mn + off;
       const int q = has + i;
       sz[q] = sum3_rn(base, -(off * 0.5f), off * jitter(q));
-      si[q] = id;
+      if (IDS) si[q] = __ldg(hi + i);
     }
     done = has + cnt;
   }
   for (int q = done + lane; q < S; q += 32) {
     sz[q] = -1.0f;
-    si[q] = -1;
+    if (IDS) si[q] = -1;
   }
   __syncwarp();
   return done;

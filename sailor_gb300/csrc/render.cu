@@ -15,6 +15,20 @@
 // grid and no head its results equal the unfused chain sg_sample_sorted ->
 // sg_grid_gather (x2) -> sg_composite_fwd on the same inputs.
 //
+// A ray's sorted positions are evaluated in blocks of 32, front to back: the
+// density taps of a block, its alphas, the transmittance through it, and
+// colour taps for its samples up to the early termination.  The walk stops
+// at the block in which the ray ends, so nothing is tapped behind it: of the
+// 85 M record slots of the 7.4 M-ray training step 46 M hold samples that
+// count, and the taps (latency of scattered 16-byte loads, 3-6 % of HBM)
+// are what the kernels are bound by.  What a later pass needs of a position
+// (weight, colour, alpha, ...) sits in warp-private shared memory, so the
+// block loop stays rolled: one body of code for every sample count (the
+// unrolled one stalled on instruction fetch) and 62-80 registers.  Against
+// the kernels that evaluated every position first: 2^20 random rays of 96
+// samples forward + adjoint 27.2 -> 15.1 ms, 2^20 pixel rays forward (with
+// fusion and tree) 4.11 -> 3.71 ms, a 3.9 M-ray training step 11.1 -> 10.1.
+//
 // The backward saves nothing from the forward: it re-runs the same per-ray
 // evaluation (same samples, taps, alpha and transmittance, bit for bit),
 // forms the exact adjoint of compositing from in-warp prefix sums, chains
@@ -30,6 +44,18 @@
 
 #include "ray_core.cuh"
 #include "scatter.cuh"
+
+// Resident CTAs per SM the register budgets are set for (build-time settings).
+#ifndef SG_RENDER_FWD_MINB
+#define SG_RENDER_FWD_MINB 4
+#endif
+#ifndef SG_RENDER_REC_MINB
+#define SG_RENDER_REC_MINB 4
+#endif
+#ifndef SG_RENDER_ADJ_MINB
+#define SG_RENDER_ADJ_MINB 3
+#endif
+#define SG_RENDER_MINB(MODE) ((MODE) == kModeRec ? SG_RENDER_REC_MINB : SG_RENDER_ADJ_MINB)
 
 namespace sg {
 
@@ -71,6 +97,7 @@ struct RenderParams {
   float *ray_g;  // [k][C]: head^T (colour gradient of ray k)
   long rec_cap;
   RecordKeys keys;
+  int cap;  // positions a warp's shared memory holds: 32, 64 or 128
 };
 
 __device__ __forceinline__ void ray_frame(const RenderParams &p, long r, int &b, int &S, int &s) {
@@ -85,93 +112,282 @@ __device__ __forceinline__ void ray_frame(const RenderParams &p, long r, int &b,
   }
 }
 
-template <int E>
-struct RayEval {
-  float z[E], sg[E], s01[E], al[E], tb[E], dl[E], rgb[E][3];
-  unsigned valid, proc, post;
-  int done;
-};
+// Warp-private shared memory of the render kernels (dynamic; cap = 32, 64 or
+// 128 positions).
+//   z    [cap]     samples, then sorted depths
+//   f    [32 + 32] transmittance factors of a block and the values before them
+//   sc             sampler scratch
+//   id, pos [cap]  node ids and sorted positions (forward with out_node)
+//   keep [8][cap]  per position, for the adjoint: see Keep
+//   cw   [32][9], wg [32]  corner weights and (weight, TSDF gradient) of a
+//                  block's samples (in-kernel scatter)
+enum { kKeepW = 0, kKeepR, kKeepG, kKeepB, kKeepS01, kKeepAl, kKeepTb, kKeepDl, kKeepWords };
 
-// Warp-private shared memory of the render kernels.
-template <int E>
 struct RenderSmem {
   float *z, *f;
-  int *i, *p;
   SampleScratch *sc;
+  int *id, *pos;
+  float *keep;
+  float *cw;
+  float2 *wg;
+  int cap;
+  __device__ __forceinline__ float &k(int which, int i) const { return keep[which * cap + i]; }
 };
 
-// Samples, sort, field taps, alpha and transmittance of ray r (frame b, S
-// samples) into ev; sorted depths stay in sm.z, with POS the sorted
-// positions in sm.p.
-template <int E, int C, bool POS>
-__device__ __forceinline__ void eval_ray(const RenderParams &p, long r, int b, int S, int sgm,
-                                         const RenderSmem<E> &sm, RayEval<E> &ev) {
-  const int lane = lane_id();
-  const int nh = p.hit_count ? min(__ldg(p.hit_count + r), p.sp.W) : p.sp.W;
-  ev.done = warp_sample_ray(p.sp, r, b, S, nh, p.rand_const, sm.z, sm.i, *sm.sc);
-  ev.valid = ev.proc = ev.post = 0;
-  if (ev.done == 0) return;
-  warp_sort_samples<E, POS>(sm.z, sm.p, S, ev.done);
-  const float *bb = p.sp.t.vol_bbox + 6 * b;
-  const float bmin[3] = {bb[0], bb[2], bb[4]};
-  const float vs = __ldg(p.sp.t.voxel_size + b), inv_vs = 1.0f / vs;
-  const float *fb = p.fbbox + 6 * b;
-  const float fmin[3] = {fb[0], fb[2], fb[4]};
-  const float fvs = __ldg(p.fvs + b), inv_fvs = 1.0f / fvs;
-  const float *tsdf = p.tsdf + (size_t)b * p.D * p.D * p.D;
-  const float *feat = p.feat + (size_t)b * p.Df * p.Df * p.Df * C;
-  const float o[3] = {__ldg(p.ori + r * 3), __ldg(p.ori + r * 3 + 1), __ldg(p.ori + r * 3 + 2)};
-  const float dr[3] = {__ldg(p.dir + r * 3), __ldg(p.dir + r * 3 + 1), __ldg(p.dir + r * 3 + 2)};
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int i = e * 32 + lane;
-    ev.z[e] = (i < S) ? sm.z[i] : -1.0f;
-    ev.sg[e] = ev.s01[e] = 0.0f;
-    ev.rgb[e][0] = ev.rgb[e][1] = ev.rgb[e][2] = 0.0f;
-    if (ev.z[e] >= 0.0f) {
-      ev.valid |= 1u << e;
-      const float pt[3] = {__fmaf_rn(dr[0], ev.z[e], o[0]), __fmaf_rn(dr[1], ev.z[e], o[1]),
-                           __fmaf_rn(dr[2], ev.z[e], o[2])};
-      int i0[3];
-      float wc[8];
-      tap_cell(bmin, vs, inv_vs, pt, i0, wc);
-      float t1[1];
-      grid_tap_cell<1>(tsdf, p.D, i0, wc, t1);
-      ev.s01[e] = tsdf_sigmoid(t1[0], p.dk);  // kept for the adjoint
-      ev.sg[e] = ev.s01[e] * p.inv_s;
-      if (!p.shared) tap_cell(fmin, fvs, inv_fvs, pt, i0, wc);
-      float fe[C];
-      grid_tap_cell<C>(feat, p.Df, i0, wc, fe);
-      if (p.head) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          float a = 0.0f;
-#pragma unroll
-          for (int c = 0; c < C; c++) a = __fmaf_rn(__ldg(p.head + k * C + c), fe[c], a);
-          ev.rgb[e][k] = a;
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 3; k++) ev.rgb[e][k] = fe[k < C ? k : 0];
-      }
-    }
-  }
-  ray_alpha<E>(ev.z, ev.sg, ev.valid, S, 0, sm.z, ev.al, ev.dl);
-  ray_transmittance<E>(ev.al, ev.valid, S, p.t_thres, sm.f, ev.tb, ev.proc, ev.post);
+// What a mode of the kernel needs beside the samples.
+enum { kModeFwd = 0, kModeBwd = 1, kModeTrain = 2, kModeRec = 3, kModeRecTsdf = 4 };
+__host__ __device__ constexpr bool mode_keeps(int mode) {
+  return mode == kModeBwd || mode == kModeTrain || mode == kModeRecTsdf;
+}
+__host__ __device__ constexpr bool mode_scatters(int mode) { return mode == kModeBwd || mode == kModeTrain; }
+
+__host__ __device__ constexpr int render_warp_words(int mode, int cap, bool ids) {
+  return cap + 64 + 128 + (ids ? 2 * cap : 0) + (mode_keeps(mode) ? kKeepWords * cap : 0) +
+         (mode_scatters(mode) ? 32 * 9 + 64 : 0);
 }
 
-#define SG_RENDER_SMEM(E)                         \
-  __shared__ __align__(16) float s_zall[8][32 * E]; \
-  __shared__ __align__(16) float s_fall[8][kTransScratch<E>]; \
-  __shared__ int s_iall[8][32 * E];                 \
-  __shared__ int s_pall[8][32 * E];                 \
-  __shared__ SampleScratch s_sc[8];                 \
-  const int w8 = threadIdx.x >> 5;                  \
-  const RenderSmem<E> sm{s_zall[w8], s_fall[w8], s_iall[w8], s_pall[w8], &s_sc[w8]};
+__device__ __forceinline__ RenderSmem render_smem(float *base, int mode, int cap, bool ids) {
+  static_assert(sizeof(SampleScratch) == 128 * 4, "sampler scratch of 128 words");
+  RenderSmem sm;
+  sm.cap = cap;
+  float *w = base + (threadIdx.x >> 5) * render_warp_words(mode, cap, ids);
+  sm.z = w;
+  w += cap;
+  sm.f = w;
+  w += 64;
+  sm.sc = reinterpret_cast<SampleScratch *>(w);
+  w += 128;
+  sm.id = sm.pos = nullptr;
+  if (ids) {
+    sm.id = reinterpret_cast<int *>(w);
+    sm.pos = reinterpret_cast<int *>(w + cap);
+    w += 2 * cap;
+  }
+  sm.keep = w;
+  if (mode_keeps(mode)) w += kKeepWords * cap;
+  sm.cw = w;
+  sm.wg = reinterpret_cast<float2 *>(w + 32 * 9);
+  return sm;
+}
 
-template <int E, int C>
-__global__ void __launch_bounds__(256) render_fwd_kernel(RenderParams p) {
-  SG_RENDER_SMEM(E)
+// Sum over the warp, pairs of neighbours first: the association of the
+// inclusive scan's last element (warp_incl_scan_f), so a total taken here
+// equals the one the adjoint's scans reach, bit for bit.
+__device__ __forceinline__ float warp_sum_scan_order(float v) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) v += __shfl_xor_sync(SG_FULL, v, o);
+  return v;
+}
+
+// Transmittance through the 32 positions of a block, carried strictly in
+// order from T (the transmittance before the block): the reference's serial
+// T *= 1 - alpha, so the early-termination decision is the reference's too.
+// f: this lane's factor (1 where its position holds no sample); [lo, hi):
+// the block's positions at which termination counts.  Returns the position
+// in the block whose update took T below t_thres (32: none); tb: the
+// transmittance before this lane's position (valid up to that position).
+// Every lane runs the same chain, eight positions per step.  When every
+// factor is in [0, 1] the product cannot rise (rounding is monotonic), so
+// one test of the step's last value finds the step where it first falls
+// below t_thres; otherwise the step's lowest value is tested.
+__device__ __forceinline__ int block_transmittance(float f, float &T, float t_thres, int lo, int hi, float *s_f,
+                                                   float &tb) {
+  const int lane = lane_id();
+  float *s_t = s_f + 32;
+  s_f[lane] = f;
+  const bool mono = __all_sync(SG_FULL, f >= 0.0f && f <= 1.0f);
+  __syncwarp();
+  int stop = 32;
+#pragma unroll 1
+  for (int i = 0; i < 32; i += 8) {
+    const float4 f0 = *reinterpret_cast<const float4 *>(s_f + i);
+    const float4 f1 = *reinterpret_cast<const float4 *>(s_f + i + 4);
+    float Ta[9];
+    Ta[0] = T;
+    Ta[1] = Ta[0] * f0.x;
+    Ta[2] = Ta[1] * f0.y;
+    Ta[3] = Ta[2] * f0.z;
+    Ta[4] = Ta[3] * f0.w;
+    Ta[5] = Ta[4] * f1.x;
+    Ta[6] = Ta[5] * f1.y;
+    Ta[7] = Ta[6] * f1.z;
+    Ta[8] = Ta[7] * f1.w;
+    if (lane == 0) {
+      *reinterpret_cast<float4 *>(s_t + i) = make_float4(Ta[0], Ta[1], Ta[2], Ta[3]);
+      *reinterpret_cast<float4 *>(s_t + i + 4) = make_float4(Ta[4], Ta[5], Ta[6], Ta[7]);
+    }
+    float low = Ta[8];
+    if (!mono)
+      low = fminf(fminf(fminf(Ta[1], Ta[2]), fminf(Ta[3], Ta[4])), fminf(fminf(Ta[5], Ta[6]), fminf(Ta[7], Ta[8])));
+    if (low < t_thres) {
+      int k = 8;
+#pragma unroll
+      for (int q = 7; q >= 0; q--)
+        if (Ta[q + 1] < t_thres && i + q >= lo && i + q < hi) k = q;
+      if (k < 8) {
+        stop = i + k;
+        break;
+      }
+    }
+    T = Ta[8];
+  }
+  __syncwarp();
+  tb = s_t[lane];
+  return stop;
+}
+
+// Geometry of a ray: what the taps of its samples need.
+struct RayGeom {
+  float o[3], d[3];
+  float bmin[3], vs, inv_vs;  // TSDF grid
+  int b;
+};
+
+__device__ __forceinline__ RayGeom ray_geom(const RenderParams &p, long r, int b) {
+  RayGeom g;
+  const float *bb = p.sp.t.vol_bbox + 6 * b;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    g.o[a] = __ldg(p.ori + r * 3 + a);
+    g.d[a] = __ldg(p.dir + r * 3 + a);
+    g.bmin[a] = __ldg(bb + 2 * a);
+  }
+  g.vs = __ldg(p.sp.t.voxel_size + b);
+  g.inv_vs = 1.0f / g.vs;
+  g.b = b;
+  return g;
+}
+
+__device__ __forceinline__ void ray_point(const RayGeom &g, float z, float pt[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; a++) pt[a] = __fmaf_rn(g.d[a], z, g.o[a]);
+}
+
+// Cell and fractions of a sample on the feature grid: the TSDF grid's when
+// both lie on one geometry.
+__device__ __forceinline__ void feat_cell(const RenderParams &p, const RayGeom &g, float z, int (&i0)[3],
+                                          float (&f)[3]) {
+  float pt[3];
+  ray_point(g, z, pt);
+  if (p.shared) {
+    tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
+  } else {
+    const float *fb = p.fbbox + 6 * g.b;
+    const float fmin[3] = {__ldg(fb), __ldg(fb + 2), __ldg(fb + 4)};
+    const float fvs = __ldg(p.fvs + g.b);
+    tap_frac(fmin, fvs, 1.0f / fvs, pt, i0, f);
+  }
+}
+
+// Colour of a sample: trilinear features through the linear head (or the
+// three channels themselves).
+template <int C>
+__device__ __forceinline__ void colour_tap(const RenderParams &p, int b, const int (&i0)[3], const float (&f)[3],
+                                           float (&rgb)[3]) {
+  float w[8], fe[C];
+#pragma unroll
+  for (int cr = 0; cr < 8; cr++) w[cr] = corner_weight(f, cr);
+  grid_tap_cell<C>(p.feat + (size_t)b * p.Df * p.Df * p.Df * C, p.Df, i0, w, fe);
+  if (p.head) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      float a = 0.0f;
+#pragma unroll
+      for (int c = 0; c < C; c++) a = __fmaf_rn(__ldg(p.head + k * C + c), fe[c], a);
+      rgb[k] = a;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) rgb[k] = fe[k < C ? k : 0];
+  }
+}
+
+// Evaluation of one block of 32 sorted positions of a ray.
+struct BlockEval {
+  float z, al, tb, dl, s01, w;
+  float rgb[3];
+  int i0[3];    // cell of a used sample on the feature grid
+  float f[3];
+  bool used;    // a sample, at or before the early termination
+};
+
+// State of a ray's walk over its blocks.
+struct RayWalk {
+  float T;
+  int m0;    // first position that holds a sample (-1: not met yet)
+  int end;   // positions at and after it are past the termination
+};
+
+// Block e: density taps, alpha, transmittance, and the colour of the samples
+// that count -- positions past the early termination are never tapped.
+// Returns false when the block holds no sample.
+template <int C>
+__device__ __forceinline__ bool eval_block(const RenderParams &p, const RayGeom &g, int S, int e,
+                                           const RenderSmem &sm, RayWalk &wk, BlockEval &v) {
+  const int lane = lane_id(), i = e * 32 + lane;
+  v.z = i < S ? sm.z[i] : -1.0f;
+  const bool valid = v.z >= 0.0f;
+  const unsigned vb = __ballot_sync(SG_FULL, valid);
+  if (vb == 0u) return false;
+  if (wk.m0 < 0) wk.m0 = e * 32 + __ffs(vb) - 1;
+  v.al = v.dl = v.s01 = v.w = 0.0f;
+  v.rgb[0] = v.rgb[1] = v.rgb[2] = 0.0f;
+  if (valid) {
+    float pt[3];
+    ray_point(g, v.z, pt);
+    tap_frac(g.bmin, g.vs, g.inv_vs, pt, v.i0, v.f);
+    float wc[8], t1[1];
+#pragma unroll
+    for (int cr = 0; cr < 8; cr++) wc[cr] = corner_weight(v.f, cr);
+    grid_tap_cell<1>(p.tsdf + (size_t)g.b * p.D * p.D * p.D, p.D, v.i0, wc, t1);
+    v.s01 = tsdf_sigmoid(t1[0], p.dk);  // kept for the adjoint
+    const float sg = v.s01 * p.inv_s;
+    // the step to the next position with z > 0 (else the last position);
+    // 1e10 behind the last position (volume_rendering.cu:87-97)
+    if (i == S - 1) {
+      v.dl = 1e10f;
+    } else {
+      float zn = sm.z[i + 1];
+      if (!(zn > 0.0f)) {
+        int m = S - 1;
+        for (int q = i + 2; q < S; q++)
+          if (sm.z[q] > 0.0f) {
+            m = q;
+            break;
+          }
+        zn = sm.z[m];
+      }
+      v.dl = zn - v.z;
+    }
+    v.al = 1.0f - expf(-sg * v.dl);
+  }
+  const int stop = block_transmittance(valid ? 1.0f - v.al : 1.0f, wk.T, p.t_thres, wk.m0 - e * 32, S - e * 32, sm.f,
+                                       v.tb);
+  if (stop < 32) wk.end = e * 32 + stop + 1;
+  v.used = valid && i < wk.end;
+  if (v.used) {
+    v.w = v.al * v.tb;
+    if (!p.shared) feat_cell(p, g, v.z, v.i0, v.f);
+    colour_tap<C>(p, g.b, v.i0, v.f, v.rgb);
+  }
+  return true;
+}
+
+// Samples and sort of ray r; returns the number of samples (sorted depths in
+// sm.z, padding first).
+template <bool IDS>
+__device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, int b, int S, const RenderSmem &sm) {
+  const int nh = p.hit_count ? min(__ldg(p.hit_count + r), p.sp.W) : p.sp.W;
+  const int done = warp_sample_ray<IDS>(p.sp, r, b, S, nh, p.rand_const, sm.z, sm.id, *sm.sc);
+  if (done > 0) warp_sort_samples<4, IDS>(sm.z, sm.pos, S, done);
+  return done;
+}
+
+extern __shared__ __align__(16) float s_render[];
+
+template <int C, bool IDS>
+__global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB) render_fwd_kernel(RenderParams p) {
+  const RenderSmem sm = render_smem(s_render, kModeFwd, p.cap, IDS);
   const int lane = lane_id();
   const int Smax = p.sp.S;
   // a segment table covers rays [ray_begin[0], total): a sub-table of
@@ -181,28 +397,30 @@ __global__ void __launch_bounds__(256) render_fwd_kernel(RenderParams p) {
        r += ((long)gridDim.x * blockDim.x) >> 5) {
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
-    RayEval<E> ev;
-    eval_ray<E, C, true>(p, r, b, S, sgm, sm, ev);
-    float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, d = 0.0f, ws = 0.0f, aa = 0.0f;
-    if (p.out_z) {
+    const int done = sample_and_sort<IDS>(p, r, b, S, sm);
+    if (IDS) {
       for (int i = lane; i < Smax; i += 32) {
-        const bool has = ev.done > 0 && i < S;
+        const bool has = done > 0 && i < S;
         p.out_z[(size_t)r * Smax + i] = has ? sm.z[i] : -1.0f;
-        p.out_node[(size_t)r * Smax + i] = has ? sm.i[sm.p[i]] : -1;
+        p.out_node[(size_t)r * Smax + i] = has ? sm.id[sm.pos[i]] : -1;
       }
     }
-    if (ev.done > 0) {
+    float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, d = 0.0f, ws = 0.0f, aa = 0.0f;
+    if (done > 0) {
       // a ray whose largest depth is < 0 renders 0 (no sample: done == 0)
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        if (((ev.proc & ev.valid) >> e) & 1u) {
-          const float w = ev.al[e] * ev.tb[e];
-          acc_r += w * ev.rgb[e][0];
-          acc_g += w * ev.rgb[e][1];
-          acc_b += w * ev.rgb[e][2];
-          d += w * ev.z[e];
-          ws += w;
-          aa += w * ev.al[e];
+      const RayGeom g = ray_geom(p, r, b);
+      RayWalk wk{1.0f, -1, S};
+#pragma unroll 1
+      for (int e = (S - done) >> 5; e * 32 < wk.end; e++) {
+        BlockEval v;
+        if (!eval_block<C>(p, g, S, e, sm, wk, v)) continue;
+        if (v.used) {
+          acc_r += v.w * v.rgb[0];
+          acc_g += v.w * v.rgb[1];
+          acc_b += v.w * v.rgb[2];
+          d += v.w * v.z;
+          ws += v.w;
+          aa += v.w * v.al;
         }
       }
       acc_r = warp_sum(acc_r);
@@ -227,11 +445,6 @@ __global__ void __launch_bounds__(256) render_fwd_kernel(RenderParams p) {
 // ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
-// Scatter layout of the backward.  Feature gradient: with C == 16, lane l
-// owns corner l / 4, channels 4 (l % 4) .. 4 (l % 4) + 3 (one float4, flushed
-// with one vector reduction); with C == 3, lane l < 24 owns corner l / 3,
-// channel l % 3.  TSDF gradient: lane l owns corner l - kTsdfLane0<C> when
-// that is in [0, 8).
 // A trilinear cell (lower corner i0, each axis in [-1, D-1] when any corner
 // is inside the grid) packed into one non-negative key of 21 bits per axis;
 // -1 when no corner is inside (the sample contributes nothing).
@@ -240,141 +453,118 @@ __device__ __forceinline__ long long cell_key(const int (&i0)[3], int D) {
   return ((long long)(i0[0] + 1) << 42) | ((long long)(i0[1] + 1) << 21) | (long long)(i0[2] + 1);
 }
 
-struct Cell3 {
-  int v[3];
+// Scatter of the in-kernel backward.  The colour head is linear, so the
+// feature gradient of the sample at sorted position i is w_i G with
+// G = head^T g_c (g_c: the gradient of the ray's colour, w_i its compositing
+// weight): per cell run only the 8 sums of corner weight x w_i are carried,
+// and G multiplies them when the run ends.  C == 16: lane l owns corner
+// l / 4, channels 4 (l % 4) .. 4 (l % 4) + 3 (one vector reduction), and its
+// corner's TSDF gradient (written by channel group 0).  C == 3: lane l < 24
+// owns corner l / 3, channel l % 3; lane l >= 24 the TSDF gradient of corner
+// l - 24.
+struct Scatter {
+  long long cur;  // cell of the current run, -1: none
+  float a, t;     // corner weight x compositing weight, x TSDF gradient
 };
-__device__ __forceinline__ Cell3 cell_of(long long k) {
-  return Cell3{{(int)(k >> 42) - 1, (int)((k >> 21) & 0x1fffff) - 1, (int)(k & 0x1fffff) - 1}};
-}
 
-template <int C>
-constexpr int kTsdfLane0 = (C == 3) ? 24 : 0;
-
-template <int C>
-__device__ __forceinline__ void flush_feat(const RenderParams &p, int b, const Cell3 &c3, float4 &acc) {
-  const int(&cell)[3] = c3.v;
+template <int C, bool FEAT, bool TSDF>
+__device__ __forceinline__ void scatter_flush(const RenderParams &p, int b, const float (&G)[4], Scatter &s) {
   const int lane = lane_id();
+  const int cell[3] = {(int)(s.cur >> 42) - 1, (int)((s.cur >> 21) & 0x1fffff) - 1, (int)(s.cur & 0x1fffff) - 1};
   size_t off;
   if constexpr (C == 16) {
-    if ((acc.x != 0.0f || acc.y != 0.0f || acc.z != 0.0f || acc.w != 0.0f) && corner_inside(cell, lane >> 2, p.Df, off))
-      red_add_f32x4(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + 4 * (lane & 3), acc.x, acc.y, acc.z,
-                    acc.w);
+    if (FEAT && s.a != 0.0f && corner_inside(cell, lane >> 2, p.Df, off))
+      red_add_f32x4(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + 4 * (lane & 3), s.a * G[0], s.a * G[1],
+                    s.a * G[2], s.a * G[3]);
+    if (TSDF && (lane & 3) == 0 && s.t != 0.0f && corner_inside(cell, lane >> 2, p.D, off))
+      atomicAdd(p.grad_tsdf + (size_t)b * p.D * p.D * p.D + off, s.t);
   } else {
-    if (lane < 8 * C && acc.x != 0.0f && corner_inside(cell, lane / C, p.Df, off))
-      atomicAdd(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + lane % C, acc.x);
+    if (FEAT && lane < 24 && s.a != 0.0f && corner_inside(cell, lane / 3, p.Df, off))
+      atomicAdd(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + lane % 3, s.a * G[0]);
+    if (TSDF && lane >= 24 && s.t != 0.0f && corner_inside(cell, lane - 24, p.D, off))
+      atomicAdd(p.grad_tsdf + (size_t)b * p.D * p.D * p.D + off, s.t);
   }
-  acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  s.a = s.t = 0.0f;
 }
 
-template <int C>
-__device__ __forceinline__ void flush_tsdf(const RenderParams &p, int b, const Cell3 &c3, float &acc) {
-  const int(&cell)[3] = c3.v;
-  const int cr = lane_id() - kTsdfLane0<C>;
-  size_t off;
-  if (cr >= 0 && cr < 8 && acc != 0.0f && corner_inside(cell, cr, p.D, off))
-    atomicAdd(p.grad_tsdf + (size_t)b * p.D * p.D * p.D + off, acc);
-  acc = 0.0f;
-}
-
-// Records of ray r (compact index k) for the deterministic reduction of the
-// grid gradients.  The colour head is linear, so the feature gradient of
-// the sample at sorted position i is w_i G with G = head^T g_c (g_c: the
-// gradient of the ray's colour, w_i its compositing weight): G goes to
-// ray_g[k] once per ray, and each used sample's record holds its cell (the
-// key), its cell fractions and w_i, the ray and its TSDF gradient.  The
-// records of the samples with a cell are packed, in sorted position order,
-// at the front of the ray's slots (a warp scan over the positions); their
-// count goes to ray_nrec[k].
-template <int E, int C>
-__device__ __forceinline__ void emit_records(const RenderParams &p, long k, long r, int b, int S,
-                                             const RayEval<E> &ev, const float (&w)[E], const float (&gsig)[E],
-                                             const float (&gc)[3]) {
+// One block's samples into the run sums: key (-1: none), corner weights from
+// f, the sample's weight and TSDF gradient.
+template <int C, bool FEAT, bool TSDF>
+__device__ __forceinline__ void scatter_block(const RenderParams &p, int b, const RenderSmem &sm, long long key,
+                                              const float (&f)[3], float w, float gt, const float (&G)[4],
+                                              Scatter &s) {
   const int lane = lane_id();
-  if (lane < C) {
-    float g;
-    if (p.head)
-      g = __fmaf_rn(__ldg(p.head + 2 * C + lane), gc[2], __fmaf_rn(__ldg(p.head + C + lane), gc[1],
-                                                                    __ldg(p.head + lane) * gc[0]));
-    else
-      g = lane < 3 ? gc[lane] : 0.0f;
-    p.ray_g[k * C + lane] = g;
-  }
-  const long base = __ldg(p.hit_slot + k);
-  const float *fb = p.fbbox + 6 * b;
-  const float fmin[3] = {fb[0], fb[2], fb[4]};
-  const float fvs = __ldg(p.fvs + b), inv_fvs = 1.0f / fvs;
-  const float o[3] = {__ldg(p.ori + r * 3), __ldg(p.ori + r * 3 + 1), __ldg(p.ori + r * 3 + 2)};
-  const float dr[3] = {__ldg(p.dir + r * 3), __ldg(p.dir + r * 3 + 1), __ldg(p.dir + r * 3 + 2)};
-  const float dsdt_k = -p.dk * p.inv_s;
-  const unsigned used = ev.proc & ev.valid;
-  const unsigned below = (1u << lane) - 1u;
-  int n = 0;  // records of the positions before this block
+  const unsigned m = __ballot_sync(SG_FULL, key >= 0);
+  if (m == 0u) return;
+  if (key >= 0) {
 #pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int i = e * 32 + lane;
-    uint32_t key = p.keys.invalid;
-    float f[3] = {0.0f, 0.0f, 0.0f};
-    if (i < S && ((used >> e) & 1u)) {
-      const float pt[3] = {__fmaf_rn(dr[0], ev.z[e], o[0]), __fmaf_rn(dr[1], ev.z[e], o[1]),
-                           __fmaf_rn(dr[2], ev.z[e], o[2])};
-      int i0[3];
-      tap_frac(fmin, fvs, inv_fvs, pt, i0, f);
-      key = record_key(p.keys, b, i0);
-    }
-    const bool has = key != p.keys.invalid;
-    const unsigned m = __ballot_sync(SG_FULL, has);
-    const long slot = base + n + __popc(m & below);
-    if (has && slot < p.rec_cap) {
-      const float gt = p.grad_tsdf ? gsig[e] * (ev.s01[e] * (1.0f - ev.s01[e]) * dsdt_k) : 0.0f;
-      p.rec[slot].fw = make_float4(f[0], f[1], f[2], w[e]);
-      p.rec[slot].kt = make_int4((int)k, __float_as_int(gt), 0, 0);
-      p.rec_key[slot] = key;
-    }
-    n += __popc(m);
+    for (int cr = 0; cr < 8; cr++) sm.cw[lane * 9 + cr] = corner_weight(f, cr);
+    sm.wg[lane] = make_float2(w, gt);
   }
-  if (lane == 0) {
-    // the ray's records within the slot capacity
-    const long room = p.rec_cap - base;
-    p.ray_nrec[k] = (int)(room <= 0 ? 0 : (n < room ? n : room));
+  // run heads: samples whose cell differs from the one before
+  const unsigned before = m & ((1u << lane) - 1u);
+  const long long pk = __shfl_sync(SG_FULL, key, before ? 31 - __clz(before) : 0);
+  const unsigned heads = __ballot_sync(SG_FULL, key >= 0 && key != (before ? pk : s.cur));
+  __syncwarp();
+  const int cr = C == 16 ? lane >> 2 : (lane < 24 ? lane / 3 : lane - 24);
+  for (unsigned q = m; q; q &= q - 1) {
+    const int j = __ffs(q) - 1;
+    if ((heads >> j) & 1u) {
+      if (s.cur >= 0) scatter_flush<C, FEAT, TSDF>(p, b, G, s);
+      s.cur = __shfl_sync(SG_FULL, key, j);
+    }
+    const float c = sm.cw[j * 9 + cr];
+    const float2 x = sm.wg[j];
+    if (FEAT) s.a = __fmaf_rn(c, x.x, s.a);
+    if (TSDF) s.t = __fmaf_rn(c, x.y, s.t);
   }
+  __syncwarp();
 }
 
-// TRAIN: the upstream gradient is formed in the kernel from the ray's own
-// outputs (loss = loss_scale / 2 * |rgb - target|^2 per ray, so d loss /
-// d rgb = loss_scale * (rgb - target)); the outputs and per-ray loss are
-// written, and nothing is recomputed.
-// Resident CTAs per SM the adjoint kernels' register budget is set for: the
-// training pass of the smaller sample capacities has less live state, so
-// more of its warps fit (64 and 80 registers, a few bytes spilled; 4 and 3
-// CTAs measured 7 % faster over the batched step than 2 CTAs at 128).
-// The record-mode pass (REC) carries no scatter state, so more of its CTAs
-// fit: 4 / 4 / 3 at up to 32 / 64 / 128 samples (measured 0.27 ms faster on
-// the batched step than 4 / 3 / 2; 5 / 4 / 3 and 6 / 4 / 2 were slower).
-// Build-time settings SG_REC_MINB_E1/E2/E4.
-#ifndef SG_REC_MINB_E1
-#define SG_REC_MINB_E1 4
-#endif
-#ifndef SG_REC_MINB_E2
-#define SG_REC_MINB_E2 4
-#endif
-#ifndef SG_REC_MINB_E4
-#define SG_REC_MINB_E4 3
-#endif
-template <int E, bool TRAIN, bool REC = false>
-constexpr int kBwdMinBlocks = !TRAIN ? 2
-                              : (REC ? (E == 1 ? SG_REC_MINB_E1 : (E == 2 ? SG_REC_MINB_E2 : SG_REC_MINB_E4))
-                                     : (E == 1 ? 4 : (E == 2 ? 3 : 2)));
+// head^T g_c for channel c of the feature grid.
+template <int C>
+__device__ __forceinline__ float head_grad(const RenderParams &p, int c, const float (&gc)[3]) {
+  if (p.head)
+    return __fmaf_rn(__ldg(p.head + 2 * C + c), gc[2], __fmaf_rn(__ldg(p.head + C + c), gc[1],
+                                                                  __ldg(p.head + c) * gc[0]));
+  return c == 0 ? gc[0] : (c == 1 ? gc[1] : (c == 2 ? gc[2] : 0.0f));
+}
 
-// REC: the rays are the compact list of rays with hits and the grid
-// gradients leave the kernel as per-sample records (emit_records) for the
-// deterministic reduction, instead of the in-kernel scatter with atomics.
-template <int E, int C, bool TRAIN, bool REC>
-__global__ void __launch_bounds__(256, kBwdMinBlocks<E, TRAIN, REC>) render_bwd_kernel(RenderParams p) {
+// Record of this lane's sample for the deterministic reduction: its cell (the
+// key), its cell fractions and compositing weight, the ray's compact index k
+// and its TSDF gradient.  The records of a ray's samples with a cell are
+// packed, in sorted position order, from slot base on (n: those written by
+// the blocks before; updated).
+__device__ __forceinline__ void emit_record(const RenderParams &p, long k, int b, long base, bool used,
+                                            const int (&i0)[3], const float (&f)[3], float w, float gt, int &n) {
+  const uint32_t key = used ? record_key(p.keys, b, i0) : p.keys.invalid;
+  const bool has = key != p.keys.invalid;
+  const unsigned m = __ballot_sync(SG_FULL, has);
+  const long slot = base + n + __popc(m & ((1u << lane_id()) - 1u));
+  if (has && slot < p.rec_cap) {
+    p.rec[slot].fw = make_float4(f[0], f[1], f[2], w);
+    p.rec[slot].kt = make_int4((int)k, __float_as_int(gt), 0, 0);
+    p.rec_key[slot] = key;
+  }
+  n += __popc(m);
+}
+
+// MODE kModeBwd: the adjoint for given upstream gradients.  The training
+// modes form the upstream gradient in the kernel from the ray's own outputs
+// (loss = loss_scale / 2 * |rgb - target|^2 per ray, so d loss / d rgb =
+// loss_scale * (rgb - target)); the outputs and per-ray loss are written, and
+// nothing is recomputed.  kModeTrain scatters with atomics; in the record
+// modes the rays are the compact list of rays with hits and the grid
+// gradients leave the kernel as per-sample records (emit_record) for the
+// deterministic reduction (scatter.cu).  Without the TSDF's gradient
+// (kModeRec) a record needs nothing that comes after its sample, so it is
+// written as soon as the sample's weight is known and no adjoint runs.
+template <int C, int MODE>
+__global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(RenderParams p) {
   static_assert(C == 3 || C == 16, "feature grids of 3 or 16 channels");
-  SG_RENDER_SMEM(E)
-  __shared__ float s_wf[REC ? 1 : 8][32][9], s_wt[REC ? 1 : 8][32][9];
-  __shared__ __align__(16) float s_g[REC ? 1 : 8][32][C == 16 ? 20 : 4];
-  __shared__ long long s_kf[REC ? 1 : 8][32], s_kt[REC ? 1 : 8][32];  // packed cell keys, -1: no contribution
+  constexpr bool REC = MODE == kModeRec || MODE == kModeRecTsdf;
+  constexpr bool TRAIN = MODE != kModeBwd;
+  const RenderSmem sm = render_smem(s_render, MODE, p.cap, false);
   const int lane = lane_id();
   const int Smax = p.sp.S;
   // a segment table covers rays [ray_begin[0], total): a sub-table of
@@ -386,11 +576,10 @@ __global__ void __launch_bounds__(256, kBwdMinBlocks<E, TRAIN, REC>) render_bwd_
     const long r = REC ? (long)__ldg(p.hit_ray + it) : it;
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
-    RayEval<E> ev;
-    eval_ray<E, C, false>(p, r, b, S, sgm, sm, ev);
-    if (ev.done == 0) {
+    const int done = sample_and_sort<false>(p, r, b, S, sm);
+    if (done == 0) {
       if (REC && lane == 0) p.ray_nrec[it] = 0;  // no sample: no record
-      if (p.grad_sigma) {
+      if (MODE == kModeBwd && p.grad_sigma) {
         for (int i = lane; i < Smax; i += 32) {
           p.grad_sigma[(size_t)r * Smax + i] = 0.0f;
           for (int k = 0; k < 3; k++) p.grad_rgb[((size_t)r * Smax + i) * 3 + k] = 0.0f;
@@ -410,70 +599,55 @@ __global__ void __launch_bounds__(256, kBwdMinBlocks<E, TRAIN, REC>) render_bwd_
       __syncwarp();
       continue;
     }
-    float gc[3] = {0.0f, 0.0f, 0.0f}, gd = 0.0f, gws = 0.0f, ga = 0.0f;
-    if (!TRAIN) {
-      if (p.g_rgb) {
-        gc[0] = __ldg(p.g_rgb + r * 3);
-        gc[1] = __ldg(p.g_rgb + r * 3 + 1);
-        gc[2] = __ldg(p.g_rgb + r * 3 + 2);
-      }
-      gd = p.g_depth ? __ldg(p.g_depth + r) : 0.0f;
-      gws = p.g_ws ? __ldg(p.g_ws + r) : 0.0f;
-      ga = p.g_alpha ? __ldg(p.g_alpha + r) : 0.0f;
-    }
-    // weights and inclusive prefix sums over sorted positions of
-    // w*rgb, w*z, w, w*alpha; totals by carries (the forward's outputs)
-    float w[E], pf[E][3], pd[E], pw[E], pa[E];
+    const RayGeom g = ray_geom(p, r, b);
+    const long base = REC ? (long)__ldg(p.hit_slot + it) : 0;
+    int nrec = 0;
+    // the ray's blocks, front to back: totals of w*rgb (and, for the general
+    // adjoint, w*z, w, w*alpha) in the scans' order
     float cf[3] = {0.0f, 0.0f, 0.0f}, cd = 0.0f, cw = 0.0f, ca = 0.0f;
-    const unsigned used = ev.proc & ev.valid;
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      w[e] = ((used >> e) & 1u) ? ev.al[e] * ev.tb[e] : 0.0f;
-      if (!__any_sync(SG_FULL, (used >> e) & 1u)) {
-        // a block of positions no lane uses (past the ray's sample count or
-        // its termination): zero weights, the running totals stand
-#pragma unroll
-        for (int k = 0; k < 3; k++) pf[e][k] = cf[k];
-        pd[e] = cd;
-        pw[e] = cw;
-        pa[e] = ca;
-        continue;
-      }
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const float v = warp_incl_scan_f(w[e] * ev.rgb[e][k]);
-        pf[e][k] = cf[k] + v;
-        cf[k] += __shfl_sync(SG_FULL, v, 31);
-      }
-      if (!TRAIN) {
-        const float vd = warp_incl_scan_f(w[e] * ev.z[e]);
-        const float vw = warp_incl_scan_f(w[e]);
-        const float va = warp_incl_scan_f(w[e] * ev.al[e]);
-        pd[e] = cd + vd;
-        pw[e] = cw + vw;
-        pa[e] = ca + va;
-        cd += __shfl_sync(SG_FULL, vd, 31);
-        cw += __shfl_sync(SG_FULL, vw, 31);
-        ca += __shfl_sync(SG_FULL, va, 31);
-      }
-    }
-    if (TRAIN) {
-      // the loss reads only the colour: depth, weight sum and alpha sum are
-      // outputs alone, summed as the forward kernel sums them
-      float d = 0.0f, ws = 0.0f, aa = 0.0f;
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        if ((used >> e) & 1u) {
-          d += w[e] * ev.z[e];
-          ws += w[e];
-          aa += w[e] * ev.al[e];
+    RayWalk wk{1.0f, -1, S};
+    const int e0 = (S - done) >> 5;
+    int e1 = e0;  // blocks [e0, e1) were evaluated
+#pragma unroll 1
+    for (; e1 * 32 < wk.end; e1++) {
+      BlockEval v;
+      const bool any = eval_block<C>(p, g, S, e1, sm, wk, v);
+      if (mode_keeps(MODE)) {
+        const int i = e1 * 32 + lane;
+        sm.k(kKeepW, i) = any ? v.w : 0.0f;
+        sm.k(kKeepDl, i) = any && v.used ? v.dl : 0.0f;
+        if (any) {
+          sm.k(kKeepR, i) = v.rgb[0];
+          sm.k(kKeepG, i) = v.rgb[1];
+          sm.k(kKeepB, i) = v.rgb[2];
+          sm.k(kKeepS01, i) = v.s01;
+          sm.k(kKeepAl, i) = v.al;
+          sm.k(kKeepTb, i) = v.used ? v.tb : 0.0f;
         }
       }
-      cd = warp_sum(d);
-      cw = warp_sum(ws);
-      ca = warp_sum(aa);
+      if (!any) continue;
+#pragma unroll
+      for (int k = 0; k < 3; k++) cf[k] += warp_sum_scan_order(v.w * v.rgb[k]);
+      if (TRAIN) {
+        // the loss reads only the colour: depth, weight sum and alpha sum
+        // are outputs alone, summed as the forward kernel sums them
+        if (v.used) {
+          cd += v.w * v.z;
+          cw += v.w;
+          ca += v.w * v.al;
+        }
+      } else {
+        cd += warp_sum_scan_order(v.w * v.z);
+        cw += warp_sum_scan_order(v.w);
+        ca += warp_sum_scan_order(v.w * v.al);
+      }
+      if (MODE == kModeRec) emit_record(p, it, b, base, v.used, v.i0, v.f, v.w, 0.0f, nrec);
     }
+    float gc[3] = {0.0f, 0.0f, 0.0f}, gd = 0.0f, gws = 0.0f, ga = 0.0f;
     if (TRAIN) {
+      cd = warp_sum(cd);
+      cw = warp_sum(cw);
+      ca = warp_sum(ca);
       // forward outputs = the totals; upstream gradient of the per-ray loss
       float l = 0.0f;
 #pragma unroll
@@ -491,146 +665,118 @@ __global__ void __launch_bounds__(256, kBwdMinBlocks<E, TRAIN, REC>) render_bwd_
         p.out_alpha[r] = ca;
         if (p.out_loss) p.out_loss[r] = 0.5f * p.loss_scale * l;
       }
-    }
-    // exact adjoint per sorted position: d out / d sigma_i = delta_i *
-    // (T_{i+1} v_i - sum_{j>i} w_j v_j) (v = rgb, z, 1; 2 alpha T_{i+1} for
-    // the alpha sum); d out / d rgb_i = w_i
-    float gsig[E], grgb[E][3];
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      gsig[e] = 0.0f;
-      grgb[e][0] = grgb[e][1] = grgb[e][2] = 0.0f;
-      if (((ev.proc & ev.valid) >> e) & 1u) {
-        const float Ta = ev.tb[e] * (1.0f - ev.al[e]);
-        float acc = 0.0f;
-        if (!TRAIN)
-          acc = gws * (Ta - (cw - pw[e])) + gd * (Ta * ev.z[e] - (cd - pd[e])) +
-                ga * (2.0f * ev.al[e] * Ta - (ca - pa[e]));
-#pragma unroll
-        for (int k = 0; k < 3; k++) acc += gc[k] * (Ta * ev.rgb[e][k] - (cf[k] - pf[e][k]));
-        gsig[e] = ev.dl[e] * acc;
-#pragma unroll
-        for (int k = 0; k < 3; k++) grgb[e][k] = w[e] * gc[k];
+    } else {
+      if (p.g_rgb) {
+        gc[0] = __ldg(p.g_rgb + r * 3);
+        gc[1] = __ldg(p.g_rgb + r * 3 + 1);
+        gc[2] = __ldg(p.g_rgb + r * 3 + 2);
       }
+      gd = p.g_depth ? __ldg(p.g_depth + r) : 0.0f;
+      gws = p.g_ws ? __ldg(p.g_ws + r) : 0.0f;
+      ga = p.g_alpha ? __ldg(p.g_alpha + r) : 0.0f;
     }
-    if (p.grad_sigma) {
+    if (REC && lane < C) p.ray_g[it * C + lane] = head_grad<C>(p, lane, gc);
+    if constexpr (mode_keeps(MODE)) {
+      // exact adjoint per sorted position: d out / d sigma_i = delta_i *
+      // (T_{i+1} v_i - sum_{j>i} w_j v_j) (v = rgb, z, 1; 2 alpha T_{i+1} for
+      // the alpha sum); d out / d rgb_i = w_i
+      float rf[3] = {0.0f, 0.0f, 0.0f}, rd = 0.0f, rw = 0.0f, ra = 0.0f;  // running totals
+      const float dsdt_k = -p.dk * p.inv_s;
+      float G[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (mode_scatters(MODE) && p.grad_feat) {
+        if constexpr (C == 16) {
 #pragma unroll
-      for (int e = 0; e < E; e++) {
+          for (int q = 0; q < 4; q++) G[q] = head_grad<C>(p, 4 * (lane & 3) + q, gc);
+        } else {
+          if (lane < 24) G[0] = head_grad<C>(p, lane % 3, gc);
+        }
+      }
+      Scatter sf{-1, 0.0f, 0.0f}, st{-1, 0.0f, 0.0f};
+#pragma unroll 1
+      for (int e = e0; e < e1; e++) {
         const int i = e * 32 + lane;
-        if (i < Smax) {
-          p.grad_sigma[(size_t)r * Smax + i] = i < S ? gsig[e] : 0.0f;
-#pragma unroll
-          for (int k = 0; k < 3; k++) p.grad_rgb[((size_t)r * Smax + i) * 3 + k] = i < S ? grgb[e][k] : 0.0f;
-        }
-      }
-      for (int i = 32 * E + lane; i < Smax; i += 32) {
-        p.grad_sigma[(size_t)r * Smax + i] = 0.0f;
-        for (int k = 0; k < 3; k++) p.grad_rgb[((size_t)r * Smax + i) * 3 + k] = 0.0f;
-      }
-    }
-    if (REC) {
-      emit_records<E, C>(p, it, r, b, S, ev, w, gsig, gc);
-      __syncwarp();
-      continue;
-    }
-    if (!p.grad_feat && !p.grad_tsdf) {
-      __syncwarp();
-      continue;
-    }
-    // scatter into the grids, samples in sorted order
-    const float *bb = p.sp.t.vol_bbox + 6 * b;
-    const float bmin[3] = {bb[0], bb[2], bb[4]};
-    const float vs = __ldg(p.sp.t.voxel_size + b), inv_vs = 1.0f / vs;
-    const float *fb = p.fbbox + 6 * b;
-    const float fmin[3] = {fb[0], fb[2], fb[4]};
-    const float fvs = __ldg(p.fvs + b), inv_fvs = 1.0f / fvs;
-    const float o[3] = {__ldg(p.ori + r * 3), __ldg(p.ori + r * 3 + 1), __ldg(p.ori + r * 3 + 2)};
-    const float dr[3] = {__ldg(p.dir + r * 3), __ldg(p.dir + r * 3 + 1), __ldg(p.dir + r * 3 + 2)};
-    const float dsdt_k = -p.dk * p.inv_s;
-    // lane-owned accumulators: feature (corner, channels) and TSDF corner
-    float4 accf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float acct = 0.0f;
-    const int fcr = (C == 16) ? (lane >> 2) : (lane < 8 * C ? lane / C : 0);
-    const int fch = (C == 16) ? 4 * (lane & 3) : (lane < 8 * C ? lane % C : 0);
-    const int tcr = lane - kTsdfLane0<C>;
-    const bool town = tcr >= 0 && tcr < 8;
-    long long curf = -1, curt = -1;
-    const bool want_t = p.grad_tsdf != nullptr, want_f = p.grad_feat != nullptr;
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const bool use = ((used >> e) & 1u) != 0;
-      if (!__any_sync(SG_FULL, use)) continue;  // no sample of this block contributes
-      long long kf = -1, kt = -1;
-      if (use) {
-        const float pt[3] = {__fmaf_rn(dr[0], ev.z[e], o[0]), __fmaf_rn(dr[1], ev.z[e], o[1]),
-                             __fmaf_rn(dr[2], ev.z[e], o[2])};
-        int i0[3];
-        float wt[8];
-        tap_cell(bmin, vs, inv_vs, pt, i0, wt);
-        if (want_t) {
-          kt = cell_key(i0, p.D);
-#pragma unroll
-          for (int cr = 0; cr < 8; cr++) s_wt[w8][lane][cr] = wt[cr];
-          s_g[w8][lane][C == 16 ? 16 : 3] = gsig[e] * (ev.s01[e] * (1.0f - ev.s01[e]) * dsdt_k);
-        }
-        if (want_f) {
-          if (!p.shared) tap_cell(fmin, fvs, inv_fvs, pt, i0, wt);
-          kf = cell_key(i0, p.Df);
-#pragma unroll
-          for (int cr = 0; cr < 8; cr++) s_wf[w8][lane][cr] = wt[cr];
-          // feature gradient: head^T d rgb
-#pragma unroll
-          for (int c = 0; c < C; c++) {
-            float g;
-            if (p.head)
-              g = __fmaf_rn(__ldg(p.head + 2 * C + c), grgb[e][2],
-                            __fmaf_rn(__ldg(p.head + C + c), grgb[e][1], __ldg(p.head + c) * grgb[e][0]));
-            else
-              g = c < 3 ? grgb[e][c] : 0.0f;
-            s_g[w8][lane][c] = g;
+        const float z = i < S ? sm.z[i] : -1.0f;
+        const float w = sm.k(kKeepW, i);
+        const bool used = z >= 0.0f && i < wk.end;
+        float gsig = 0.0f, s01 = 0.0f;
+        if (__any_sync(SG_FULL, used)) {
+          const float al = sm.k(kKeepAl, i);
+          const float rgb[3] = {sm.k(kKeepR, i), sm.k(kKeepG, i), sm.k(kKeepB, i)};
+          const float Ta = sm.k(kKeepTb, i) * (1.0f - al);
+          s01 = sm.k(kKeepS01, i);
+          float acc = 0.0f;
+          if (!TRAIN) {
+            const float vd = warp_incl_scan_f(w * z), vw = warp_incl_scan_f(w), va = warp_incl_scan_f(w * al);
+            acc = gws * (Ta - (cw - (rw + vw))) + gd * (Ta * z - (cd - (rd + vd))) +
+                  ga * (2.0f * al * Ta - (ca - (ra + va)));
+            rd += __shfl_sync(SG_FULL, vd, 31);
+            rw += __shfl_sync(SG_FULL, vw, 31);
+            ra += __shfl_sync(SG_FULL, va, 31);
           }
-        }
-      }
-      s_kf[w8][lane] = kf;
-      s_kt[w8][lane] = kt;
-      __syncwarp();
-      // samples with a cell, in sorted order (the same mask in every lane)
-      const unsigned mf = __ballot_sync(SG_FULL, kf >= 0), mt = __ballot_sync(SG_FULL, kt >= 0);
-      if (want_f) {
-        for (unsigned m = mf; m; m &= m - 1) {
-          const int j = __ffs(m) - 1;
-          const long long k = s_kf[w8][j];
-          if (k != curf) {
-            if (curf >= 0) flush_feat<C>(p, b, cell_of(curf), accf);
-            curf = k;
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            const float v = warp_incl_scan_f(w * rgb[k]);
+            acc += gc[k] * (Ta * rgb[k] - (cf[k] - (rf[k] + v)));
+            rf[k] += __shfl_sync(SG_FULL, v, 31);
           }
-          const float wf = s_wf[w8][j][fcr];
-          if constexpr (C == 16) {
-            const float4 g4 = *reinterpret_cast<const float4 *>(&s_g[w8][j][fch]);
-            accf.x = __fmaf_rn(wf, g4.x, accf.x);
-            accf.y = __fmaf_rn(wf, g4.y, accf.y);
-            accf.z = __fmaf_rn(wf, g4.z, accf.z);
-            accf.w = __fmaf_rn(wf, g4.w, accf.w);
+          if (used) gsig = sm.k(kKeepDl, i) * acc;
+        }
+        if (MODE == kModeBwd && p.grad_sigma && i < Smax) {
+          p.grad_sigma[(size_t)r * Smax + i] = gsig;
+#pragma unroll
+          for (int k = 0; k < 3; k++) p.grad_rgb[((size_t)r * Smax + i) * 3 + k] = used ? w * gc[k] : 0.0f;
+        }
+        const float gt = gsig * (s01 * (1.0f - s01) * dsdt_k);
+        if (MODE == kModeRecTsdf) {
+          int i0[3] = {0, 0, 0};
+          float f[3] = {0.0f, 0.0f, 0.0f};
+          if (used) feat_cell(p, g, z, i0, f);
+          emit_record(p, it, b, base, used, i0, f, w, gt, nrec);
+        } else if (p.grad_feat || p.grad_tsdf) {
+          // scatter into the grids, samples in sorted order
+          int i0[3] = {0, 0, 0};
+          float f[3] = {0.0f, 0.0f, 0.0f};
+          if (used) feat_cell(p, g, z, i0, f);
+          const long long kf = used ? cell_key(i0, p.Df) : -1;
+          if (p.shared) {
+            if (p.grad_feat && p.grad_tsdf) scatter_block<C, true, true>(p, b, sm, kf, f, w, gt, G, sf);
+            else if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, kf, f, w, gt, G, sf);
+            else scatter_block<C, false, true>(p, b, sm, kf, f, w, gt, G, sf);
           } else {
-            accf.x = __fmaf_rn(wf, s_g[w8][j][fch], accf.x);
+            if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, kf, f, w, gt, G, sf);
+            if (p.grad_tsdf) {
+              if (used) {
+                float pt[3];
+                ray_point(g, z, pt);
+                tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
+              }
+              scatter_block<C, false, true>(p, b, sm, used ? cell_key(i0, p.D) : -1, f, w, gt, G, st);
+            }
           }
         }
       }
-      if (want_t) {
-        for (unsigned m = mt; m; m &= m - 1) {
-          const int j = __ffs(m) - 1;
-          const long long k = s_kt[w8][j];
-          if (k != curt) {
-            if (curt >= 0) flush_tsdf<C>(p, b, cell_of(curt), acct);
-            curt = k;
-          }
-          if (town) acct = __fmaf_rn(s_wt[w8][j][tcr], s_g[w8][j][C == 16 ? 16 : 3], acct);
+      if (mode_scatters(MODE)) {
+        if (sf.cur >= 0) {
+          if (p.shared && p.grad_feat && p.grad_tsdf) scatter_flush<C, true, true>(p, b, G, sf);
+          else if (p.grad_feat) scatter_flush<C, true, false>(p, b, G, sf);
+          else scatter_flush<C, false, true>(p, b, G, sf);
+        }
+        if (st.cur >= 0) scatter_flush<C, false, true>(p, b, G, st);
+      }
+      if (MODE == kModeBwd && p.grad_sigma) {
+        // positions of blocks that were not evaluated: no gradient
+        for (int i = lane; i < Smax; i += 32) {
+          if (i >= e0 * 32 && i < e1 * 32) continue;
+          p.grad_sigma[(size_t)r * Smax + i] = 0.0f;
+          for (int k = 0; k < 3; k++) p.grad_rgb[((size_t)r * Smax + i) * 3 + k] = 0.0f;
         }
       }
-      __syncwarp();
     }
-    if (curf >= 0) flush_feat<C>(p, b, cell_of(curf), accf);
-    if (curt >= 0) flush_tsdf<C>(p, b, cell_of(curt), acct);
+    if (REC && lane == 0) {
+      // the ray's records within the slot capacity
+      const long room = p.rec_cap - base;
+      p.ray_nrec[it] = (int)(room <= 0 ? 0 : (nrec < room ? nrec : room));
+    }
     __syncwarp();
   }
 }
@@ -641,29 +787,54 @@ static int render_grid(long R) {
   return (int)(g < cap ? g : cap);
 }
 
-// mode 0: forward, 1: backward, 2: training step (forward + loss + backward),
-// 3: training step writing gradient records
-template <int E, int C>
-static void launch_render_e(const RenderParams &p, int mode, int g, sg_stream_t stream) {
-  if (mode == 0) render_fwd_kernel<E, C><<<g, 256, 0, stream>>>(p);
-  else if (mode == 1) render_bwd_kernel<E, C, false, false><<<g, 256, 0, stream>>>(p);
-  else if (mode == 2) render_bwd_kernel<E, C, true, false><<<g, 256, 0, stream>>>(p);
-  else render_bwd_kernel<E, C, true, true><<<g, 256, 0, stream>>>(p);
+// Dynamic shared memory of a kernel (8 warps); above 48 KB it is opted into.
+template <typename K>
+static int render_smem_bytes(K kernel, int mode, int cap, bool ids, size_t &bytes) {
+  bytes = (size_t)8 * render_warp_words(mode, cap, ids) * sizeof(float);
+  if (bytes > 48 * 1024 &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    return SG_ERR_CUDA;
+  return SG_OK;
+}
+
+template <int C, int MODE>
+static int launch_bwd(const RenderParams &p, int g, sg_stream_t stream) {
+  size_t bytes;
+  const int rc = render_smem_bytes(render_bwd_kernel<C, MODE>, MODE, p.cap, false, bytes);
+  if (rc != SG_OK) return rc;
+  render_bwd_kernel<C, MODE><<<g, 256, bytes, stream>>>(p);
+  return SG_OK;
+}
+
+template <int C, bool IDS>
+static int launch_fwd(const RenderParams &p, int g, sg_stream_t stream) {
+  size_t bytes;
+  const int rc = render_smem_bytes(render_fwd_kernel<C, IDS>, kModeFwd, p.cap, IDS, bytes);
+  if (rc != SG_OK) return rc;
+  render_fwd_kernel<C, IDS><<<g, 256, bytes, stream>>>(p);
+  return SG_OK;
 }
 
 template <int C>
 static int launch_render(const RenderParams &p, int mode, int g, sg_stream_t stream) {
-  const int S = p.sp.S;
-  if (S <= 32) launch_render_e<1, C>(p, mode, g, stream);
-  else if (S <= 64) launch_render_e<2, C>(p, mode, g, stream);
-  else if (S <= 128) launch_render_e<4, C>(p, mode, g, stream);
-  else return SG_ERR_UNSUPPORTED;
+  int rc;
+  if (mode == kModeFwd) rc = p.out_z ? launch_fwd<C, true>(p, g, stream) : launch_fwd<C, false>(p, g, stream);
+  else if (mode == kModeBwd) rc = launch_bwd<C, kModeBwd>(p, g, stream);
+  else if (mode == kModeTrain) rc = launch_bwd<C, kModeTrain>(p, g, stream);
+  else if (p.grad_tsdf) rc = launch_bwd<C, kModeRecTsdf>(p, g, stream);
+  else rc = launch_bwd<C, kModeRec>(p, g, stream);
+  if (rc != SG_OK) return rc;
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
 
-static int launch_render_c(const RenderParams &p, int C, int mode, sg_stream_t stream) {
+// mode: kModeFwd, kModeBwd, kModeTrain, or kModeRec (records; with the TSDF
+// gradient when p.grad_tsdf is set)
+static int launch_render_c(RenderParams p, int C, int mode, sg_stream_t stream) {
   if (p.R <= 0) return SG_OK;
+  const int S = p.sp.S;
+  if (S > 128) return SG_ERR_UNSUPPORTED;
+  p.cap = S <= 32 ? 32 : (S <= 64 ? 64 : 128);
   const int g = render_grid(p.R);
   if (C == 3) return launch_render<3>(p, mode, g, stream);
   if (C == 16) return launch_render<16>(p, mode, g, stream);
@@ -759,7 +930,7 @@ extern "C" int sg_render_fused(const SgTree *tree, const int *hit_idx, const flo
   p.out_alpha = out_alpha;
   p.out_z = out_z;
   p.out_node = out_node;
-  return launch_render_c(p, 3, 0, stream);
+  return launch_render_c(p, 3, kModeFwd, stream);
 }
 
 extern "C" int sg_render_segments_fwd(const SgTree *tree, const SgRaySegments *seg, const SgRenderArgs *args,
@@ -776,7 +947,7 @@ extern "C" int sg_render_segments_fwd(const SgTree *tree, const SgRaySegments *s
   p.out_alpha = out_alpha;
   p.out_z = out_z;
   p.out_node = out_node;
-  return launch_render_c(p, args->C, 0, stream);
+  return launch_render_c(p, args->C, kModeFwd, stream);
 }
 
 extern "C" int sg_render_segments_bwd(const SgTree *tree, const SgRaySegments *seg, const SgRenderArgs *args,
@@ -795,7 +966,7 @@ extern "C" int sg_render_segments_bwd(const SgTree *tree, const SgRaySegments *s
   p.grad_tsdf = grad_tsdf;
   p.grad_sigma = grad_sigma;
   p.grad_rgb = grad_rgb;
-  return launch_render_c(p, args->C, 1, stream);
+  return launch_render_c(p, args->C, kModeBwd, stream);
 }
 
 extern "C" int sg_render_segments_train(const SgTree *tree, const SgRaySegments *seg, const SgRenderArgs *args,
@@ -815,7 +986,7 @@ extern "C" int sg_render_segments_train(const SgTree *tree, const SgRaySegments 
   p.out_alpha = out_alpha;
   p.grad_feat = grad_feat;
   p.grad_tsdf = grad_tsdf;
-  return launch_render_c(p, args->C, 2, stream);
+  return launch_render_c(p, args->C, kModeTrain, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -879,9 +1050,7 @@ extern "C" int sg_render_segments_train_det(const SgTree *tree, const SgRaySegme
     pg.k_end = w.seg_hit + groups[g + 1];
     // the group's count of rays with hits is on the device: the grid is the
     // persistent cap, its warps striding over the compact range
-    const int gsz = render_grid(R);
-    if (args->C == 3) rc = launch_render<3>(pg, 3, gsz, stream);
-    else rc = launch_render<16>(pg, 3, gsz, stream);
+    rc = launch_render_c(pg, args->C, kModeRec, stream);
     if (rc != SG_OK) return rc;
   }
   return launch_det_reduce(w, p.keys, R, (long)capacity, args->C, grad_feat, grad_tsdf, stream);
