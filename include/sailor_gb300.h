@@ -739,6 +739,51 @@ int sg_render_segments_train_det(const SgTree *tree, const SgRaySegments *seg,
                                  long long capacity, SgStatus *status,
                                  sg_stream_t stream);
 
+/* ---- packed fields ---------------------------------------------------- */
+
+/* Colour and TSDF of the voxels near the tree's nodes, packed for the renders
+ * below: packed [B,D,D,D,4] float32 (16-byte aligned) receives, for every
+ * voxel in a top node's brick or within one voxel of one, head * features (or
+ * the three channels) and the TSDF value; other voxels are left as they are.
+ * Needs the feature grid on the TSDF grid's geometry (Df == D == tree->Db,
+ * feat_bbox == tree->vol_bbox, feat_vs == tree->voxel_size), C of 3 or 16 and a
+ * brick edge that is a power of two (else SG_ERR_UNSUPPORTED). */
+int sg_pack_fields(const SgTree *tree, const SgRaySegments *seg,
+                   const SgRenderArgs *args, float *packed, sg_stream_t stream);
+
+/* sg_render_segments_fwd / _bwd / _train / _train_det with the samples tapped
+ * from fields that sg_pack_fields packed from the same tree and args (NULL:
+ * from the grids themselves, as those calls do).  Samples whose cell is not
+ * packed read the grids; the outputs are the same, bit for bit. */
+int sg_render_packed_fwd(const SgTree *tree, const SgRaySegments *seg,
+                         const SgRenderArgs *args, const float *packed,
+                         float *out_rgb, float *out_depth, float *out_ws,
+                         float *out_alpha, float *out_z, int *out_node,
+                         sg_stream_t stream);
+int sg_render_packed_bwd(const SgTree *tree, const SgRaySegments *seg,
+                         const SgRenderArgs *args, const float *packed,
+                         const float *g_rgb, const float *g_depth,
+                         const float *g_ws, const float *g_alpha,
+                         float *grad_feat, float *grad_tsdf, float *grad_sigma,
+                         float *grad_rgb, sg_stream_t stream);
+int sg_render_packed_train(const SgTree *tree, const SgRaySegments *seg,
+                           const SgRenderArgs *args, const float *packed,
+                           const float *target_rgb, float loss_scale,
+                           float *out_rgb, float *out_depth, float *out_ws,
+                           float *out_alpha, float *out_loss, float *grad_feat,
+                           float *grad_tsdf, sg_stream_t stream);
+int sg_render_packed_train_det(const SgTree *tree, const SgRaySegments *seg,
+                               const SgRenderArgs *args, const float *packed,
+                               int ngroups, const int *groups,
+                               const int *group_S, const float *target_rgb,
+                               float loss_scale, float *out_rgb,
+                               float *out_depth, float *out_ws,
+                               float *out_alpha, float *out_loss,
+                               float *grad_feat, float *grad_tsdf,
+                               void *workspace, size_t workspace_bytes,
+                               long long capacity, SgStatus *status,
+                               sg_stream_t stream);
+
 /* Stable sort of (keys[i], i), i < *count (a device int, at most capacity),
  * by the low key_bits bits of the keys: the sorted keys and the indices
  * into keys_out / vals_out ([capacity] each); keys_tmp / vals_tmp are

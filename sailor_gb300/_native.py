@@ -31,6 +31,8 @@ EXPORTS = (
     "sg_project_sampled_xyz", "sg_project_gather", "sg_train_det_workspace_bytes", "sg_render_segments_train_det",
     "sg_sort_pairs_scratch_bytes", "sg_sort_pairs", "sg_octree_scratch_bytes", "sg_octree_build",
     "sg_octree_nodes", "sg_octree_traversal", "sg_sample_fine", "sg_nerf_param_count", "sg_nerf_density",
+    "sg_pack_fields", "sg_render_packed_fwd", "sg_render_packed_bwd", "sg_render_packed_train",
+    "sg_render_packed_train_det",
 )
 
 
@@ -131,6 +133,11 @@ def _load():
     lib.sg_train_det_workspace_bytes.argtypes = [ll, i, i, ll]
     lib.sg_train_det_workspace_bytes.restype = sz
     lib.sg_render_segments_train_det.argtypes = [T, G, A, i, p, p, p, f, p, p, p, p, p, p, p, p, sz, ll, p, p]
+    lib.sg_pack_fields.argtypes = [T, G, A, p, p]
+    lib.sg_render_packed_fwd.argtypes = [T, G, A, p, p, p, p, p, p, p, p]
+    lib.sg_render_packed_bwd.argtypes = [T, G, A, p, p, p, p, p, p, p, p, p, p]
+    lib.sg_render_packed_train.argtypes = [T, G, A, p, p, f, p, p, p, p, p, p, p, p]
+    lib.sg_render_packed_train_det.argtypes = [T, G, A, p, i, p, p, p, f, p, p, p, p, p, p, p, p, sz, ll, p, p]
     lib.sg_sort_pairs_scratch_bytes.argtypes = [ll]
     lib.sg_sort_pairs_scratch_bytes.restype = sz
     lib.sg_sort_pairs.argtypes = [p, p, ll, i, p, p, p, p, p, sz, p]
