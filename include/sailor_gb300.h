@@ -492,6 +492,12 @@ typedef struct SgProjGather {
 
 int sg_project_gather(const SgProjGather *args, sg_stream_t stream);
 
+/* A map [n,C,H,W] read through its element strides (4, host) into dst
+ * [n,H,W,C]: sg_project_gather reads channels-last maps in whole texel rows,
+ * which pays from about a quarter as many points per image as pixels. */
+int sg_channels_last(const float *src, const long long *stride, int n, int C, int H,
+                     int W, float *dst, sg_stream_t stream);
+
 /* Node-corner trilinear aggregation.  Replaces
  * MultiLayerOctree::trilinear_aggregate_features(_backward)
  * (sampling_kernel.cu:162-327, 1384-1462).  ori/dir [B,N,3],

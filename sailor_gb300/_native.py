@@ -32,7 +32,7 @@ EXPORTS = (
     "sg_sort_pairs_scratch_bytes", "sg_sort_pairs", "sg_octree_scratch_bytes", "sg_octree_build",
     "sg_octree_nodes", "sg_octree_traversal", "sg_sample_fine", "sg_nerf_param_count", "sg_nerf_density",
     "sg_pack_fields", "sg_render_packed_fwd", "sg_render_packed_bwd", "sg_render_packed_train",
-    "sg_render_packed_train_det",
+    "sg_render_packed_train_det", "sg_channels_last",
 )
 
 
@@ -147,6 +147,7 @@ def _load():
     lib.sg_zero_near_nodes.argtypes = [C.POINTER(SgTree), p, i, p]
     lib.sg_project_sampled_xyz.argtypes = [C.POINTER(SgTree), p, p, p, p, p, p, i, i, i, i, i, i, i, p, p, p]
     lib.sg_project_gather.argtypes = [C.POINTER(SgProjGather), p]
+    lib.sg_channels_last.argtypes = [p, C.POINTER(ll), i, i, i, i, p, p]
     lib.sg_tune_set.argtypes = [i, i]
     lib.sg_tune_get.argtypes = [i]
     O = C.POINTER(SgOctree)

@@ -17,11 +17,15 @@
 // maps bilinearly (align_corners=True, zero padding) straight into the
 // channel-last [view image, point, C] layout the reference produces with
 // permute + contiguous.  Maps are read through strides, so NCHW and
-// channels-last tensors both work; channels-last maps with C % 4 == 0 are
-// gathered by lane groups with 16-byte loads of whole texel rows and
-// 16-byte stores of whole output rows (a warp covers 32 items, four at a
-// time), the others item by item.
+// channels-last tensors both work.  Maps whose channels are contiguous are
+// gathered by lane groups, texel rows and output rows in vectors of 16, 8 or
+// 4 bytes (gather_rows); maps of up to 4 channels and maps of any other
+// layout by a thread per item (gather_map).
+//
+// sg_channels_last writes a map into channels-last order, for callers that
+// gather many points from a map in another layout.
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -164,7 +168,8 @@ constexpr int kMaxMaps = 4;
 struct GatherMap {
   const float *data;
   long sn, sc, sy, sx;  // element strides of [view image, channel, y, x]
-  int C, H, W, vec4;    // vec4: channels contiguous, C % 4 == 0, 16-byte aligned
+  int C, H, W;
+  int rows;             // floats per vector of the row gather (4, 2, 1); 0: a thread per item
   float *out;           // [view image, N, C]
 };
 
@@ -181,7 +186,6 @@ struct ProjGatherParams {
   float *ori_pts, *grids, *depth;  // [BV, 3, N], [BV, 2, N], [BV, 1, N]; each may be null
   GatherMap maps[kMaxMaps];
   int n_maps;
-  int groups;                      // channels-last maps share map 0's size: lane-group gathers
   int psdf_map;                    // map holding depth for psdf (-1: none)
   float psdf_clip, psdf_scale;
   float *psdf;                     // [BV, N, 1]
@@ -219,21 +223,50 @@ __device__ __forceinline__ long corner_off(const GatherMap &m, int img, int x0, 
   return (long)img * m.sn + (long)(y0 + (i >> 1)) * m.sy + (long)(x0 + (i & 1)) * m.sx;
 }
 
-// Per-item gather of a map that is not read in lane groups: channel by
-// channel through the channel stride.  Returns channel 0.
-__device__ __forceinline__ float gather_map(const GatherMap &m, int img, long k, const Foot &f) {
-  float *out = m.out + k * m.C;
-  long off[4];
+// Per-item gather of NC channels of a map that is not read in lane groups, all
+// their loads in flight together; the first channel's value is returned.
+// off: element offset of the footprint's first corner in the first channel.
+template <int NC, typename Off>
+__device__ __forceinline__ float gather_channels(const GatherMap &m, Off off, float *out, const Foot &f) {
+  const Off sx = (Off)m.sx, sy = (Off)m.sy, sc = (Off)m.sc;
+  float v[NC][4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) off[i] = corner_off(m, img, f.x0, f.y0, i);
-  float first = 0.0f;
-  for (int c = 0; c < m.C; c++) {
-    float a = 0.0f;
+  for (int i = 0; i < 4; i++) {
+    const float *at = m.data + (off + ((i & 2) ? sy : 0) + ((i & 1) ? sx : 0));
+    const bool in = (f.mask >> i) & 1;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      v[c][i] = 0.0f;
+      if (in) v[c][i] = __ldg(at);
+      at += sc;
+    }
+  }
+  float a[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    a[c] = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; i++)
-      if ((f.mask >> i) & 1) a = __fmaf_rn(__ldg(m.data + off[i] + (long)c * m.sc), f.w[i], a);
-    __stcs(out + c, a);
-    if (c == 0) first = a;
+      if ((f.mask >> i) & 1) a[c] = __fmaf_rn(v[c][i], f.w[i], a[c]);
+    __stcs(out + c, a[c]);
+  }
+  return a[0];
+}
+
+// Per-item gather of a whole map through its channel stride.  Returns channel 0.
+template <bool SMALL>
+__device__ __forceinline__ float gather_map(const GatherMap &m, int img, long k, const Foot &f) {
+  using Off = typename std::conditional<SMALL, int, long>::type;
+  float *out = m.out + k * m.C;
+  Off off = (Off)img * (Off)m.sn + (Off)f.y0 * (Off)m.sy + (Off)f.x0 * (Off)m.sx;
+  if (m.C == 1) return gather_channels<1>(m, off, out, f);
+  if (m.C == 3) return gather_channels<3>(m, off, out, f);
+  float first = 0.0f;
+#pragma unroll 1
+  for (int c = 0; c < m.C; c++) {
+    const float v = gather_channels<1>(m, off, out + c, f);
+    if (c == 0) first = v;
+    off += (Off)m.sc;
   }
   return first;
 }
@@ -278,49 +311,136 @@ __device__ __forceinline__ void persp_point(const ProjGatherParams &p, long img,
 
 // Footprints of a warp's 32 items, for the lane groups.
 struct WarpFoot {
-  float4 w;
-  int4 a;  // x0, y0, mask, image
+  float4 w;  // corner weights, 0 for corners outside the image
+  int4 a;    // x0, y0, mask, image
 };
 
-// Gather of one channels-last map (vec4) for the 32 items of a warp: lane
-// groups of 8 take the items four at a time, lane (group, q) the channel
-// quads q, q + 8, ..., so each load reads whole 16-byte quads of one texel
-// row and each store writes a contiguous part of the item's output row.
-// The items' footprints come from the warp's shared array.
+// V consecutive floats, and their multiply-add by one weight in pairs
+// (fma.rn.f32x2: the roundings of two fma.rn.f32).
+__device__ __forceinline__ unsigned long long pair_of(float w) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(w));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long x, unsigned long long w,
+                                                       unsigned long long acc) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(w), "l"(acc));
+  return r;
+}
+template <int V> struct FloatVec;
+template <> struct FloatVec<1> {
+  using Raw = float;
+  using W = float;
+  static __device__ __forceinline__ W weight(float w) { return w; }
+  static __device__ __forceinline__ Raw zero() { return 0.0f; }
+  static __device__ __forceinline__ Raw fma(Raw x, W w, Raw acc) { return __fmaf_rn(x, w, acc); }
+};
+template <> struct FloatVec<2> {
+  using Raw = unsigned long long;
+  using W = unsigned long long;
+  static __device__ __forceinline__ W weight(float w) { return pair_of(w); }
+  static __device__ __forceinline__ Raw zero() { return 0ull; }
+  static __device__ __forceinline__ Raw fma(Raw x, W w, Raw acc) { return fma_pair(x, w, acc); }
+};
+template <> struct FloatVec<4> {
+  using Raw = ulonglong2;
+  using W = unsigned long long;
+  static __device__ __forceinline__ W weight(float w) { return pair_of(w); }
+  static __device__ __forceinline__ Raw zero() { return make_ulonglong2(0ull, 0ull); }
+  static __device__ __forceinline__ Raw fma(Raw x, W w, Raw acc) {
+    return make_ulonglong2(fma_pair(x.x, w, acc.x), fma_pair(x.y, w, acc.y));
+  }
+};
+
+// Gather of one map with contiguous channels for the 32 items of a warp: lane
+// groups of GW (8, or 4 and 2 where a row has no more vectors) take the items,
+// kRowItems at a time, lane (group, q) the V-float vectors q, q + GW, ..., so
+// each load reads whole vectors of one texel row and each store writes a
+// contiguous part of the item's output row.  The items' footprints come from
+// the warp's shared array.
+//
+// Bound by the L1 data path (four texel rows of 128 bytes an item: 82 % busy)
+// and by issue, so the loop is kept short: 32-bit offsets where every map allows it (SMALL), two items per
+// group with 8 loads in flight a lane, paired multiply-adds, and (WHOLE) no
+// test per corner where every footprint of the warp lies wholly inside the
+// image or wholly outside it: an item outside reads texel (0, 0)'s corners
+// and writes zeros.  33.5 M items of 32 + 32 + 3 + 1 channels: 4.25 -> 3.26 ms
+// (of it the projection alone 0.32, a 32-channel map 1.15, the depth map
+// 0.17, the colours 0.31).
+constexpr int kRowItems = 2;
+
+template <int V, int GW, bool SMALL, bool WHOLE>
 __device__ __forceinline__ void gather_rows(const GatherMap &m, long k0, long total, const WarpFoot *sf) {
-  const int lane = lane_id(), grp = lane >> 3, q0 = lane & 7;
-  const int nq = m.C >> 2;
-  for (int r = 0; r < 8; r++) {
-    const int src = r * 4 + grp;
-    if (k0 + src >= total) break;  // items past the end are the warp's last ones
-    const float4 w = sf[src].w;
-    const int4 a = sf[src].a;
-    const float wt[4] = {w.x, w.y, w.z, w.w};
-    long off[4];
+  using T = FloatVec<V>;
+  using Raw = typename T::Raw;
+  using Off = typename std::conditional<SMALL, int, long>::type;
+  const int lane = lane_id(), grp = lane / GW, q0 = lane % GW;
+  constexpr int kGroups = 32 / GW;
+  const int C = m.C;
+  const int left = total - k0 < 32 ? (int)(total - k0) : 32;  // items past the end are the warp's last ones
+  const float *const data = m.data + V * q0;
+  float *out = m.out + k0 * C + (grp * C + V * q0);
+  const Off sy = (Off)m.sy, sx = (Off)m.sx, sn = (Off)m.sn;
+#pragma unroll 1
+  for (int r = grp; r < left; r += kGroups * kRowItems, out += kGroups * kRowItems * C) {
+    typename T::W w[kRowItems][4];
+    int mask[kRowItems];
+    const float *at[kRowItems][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++) off[i] = corner_off(m, a.w, a.x, a.y, i);
-    float4 *out = reinterpret_cast<float4 *>(m.out + (k0 + src) * m.C);
-    for (int q = q0; q < nq; q += 8) {
-      float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int u = 0; u < kRowItems; u++) {
+      const int it = r + kGroups * u;
+      const float4 ww = sf[it].w;
+      const int4 a = sf[it].a;
+      w[u][0] = T::weight(ww.x);
+      w[u][1] = T::weight(ww.y);
+      w[u][2] = T::weight(ww.z);
+      w[u][3] = T::weight(ww.w);
+      mask[u] = a.z;
+      at[u][0] = data + ((Off)a.w * sn + (Off)a.y * sy + (Off)a.x * sx);
+      at[u][1] = at[u][0] + sy;
+    }
+#pragma unroll 1
+    for (int q = V * q0; q < C; q += V * GW) {
+      Raw v[kRowItems][4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (!((a.z >> i) & 1)) continue;
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(m.data + off[i]) + q);
-        acc.x = __fmaf_rn(v.x, wt[i], acc.x);
-        acc.y = __fmaf_rn(v.y, wt[i], acc.y);
-        acc.z = __fmaf_rn(v.z, wt[i], acc.z);
-        acc.w = __fmaf_rn(v.w, wt[i], acc.w);
+      for (int u = 0; u < kRowItems; u++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const Raw *const a = reinterpret_cast<const Raw *>(at[u][i >> 1] + ((i & 1) ? sx : 0) + (q - V * q0));
+          if constexpr (WHOLE) {
+            v[u][i] = __ldg(a);
+          } else {
+            v[u][i] = T::zero();
+            if ((mask[u] >> i) & 1) v[u][i] = __ldg(a);
+          }
+        }
+#pragma unroll
+      for (int u = 0; u < kRowItems; u++) {
+        Raw acc = T::zero();
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc = T::fma(v[u][i], w[u][i], acc);
+        if (WHOLE && mask[u] == 0) acc = T::zero();
+        // streaming: the maps, not the output, should stay in L2
+        if (r + kGroups * u < left)
+          __stcs(reinterpret_cast<Raw *>(out + kGroups * u * C + (q - V * q0)), acc);
       }
-      __stcs(out + q, acc);  // streaming: the maps, not the output, should stay in L2
     }
   }
 }
 
+template <int V, int GW, bool SMALL>
+__device__ __forceinline__ void gather_rows_for(const GatherMap &m, long k0, long total, const WarpFoot *sf, bool whole) {
+  if (whole) gather_rows<V, GW, SMALL, true>(m, k0, total, sf);
+  else gather_rows<V, GW, SMALL, false>(m, k0, total, sf);
+}
+
 // Warp per 32 consecutive (image, point) items: lane = item for the
 // projection, the bilinear footprint (once per item; maps of one size share
-// it) and the maps that are not channels-last with C % 4 == 0; channels-last
-// maps in lane groups (gather_rows).
-__global__ void __launch_bounds__(256) project_gather_kernel(ProjGatherParams p) {
+// it) and the maps gathered item by item; the others in lane groups
+// (gather_rows).
+template <bool SMALL>
+__global__ void __launch_bounds__(256, 4) project_gather_kernel(ProjGatherParams p) {
   __shared__ WarpFoot s_foot[8][32];
   const long total = (long)p.BV * p.N;
   const int lane = lane_id(), w8 = threadIdx.x >> 5;
@@ -342,32 +462,81 @@ __global__ void __launch_bounds__(256) project_gather_kernel(ProjGatherParams p)
         persp_point(p, img, n, gx, gy, dep);
       }
     }
-    const Foot f0 = footprint(p.maps[0].H, p.maps[0].W, gx, gy);
-    if (p.groups) {
-      __syncwarp();  // the previous items' readers are done
-      s_foot[w8][lane].w = make_float4(f0.w[0], f0.w[1], f0.w[2], f0.w[3]);
-      s_foot[w8][lane].a = make_int4(f0.x0, f0.y0, live ? f0.mask : 0, img);
-      __syncwarp();
-    }
+    int fh = -1, fw = -1;     // size of the map the current footprint is of
+    bool staged = false;      // it is in the shared array
+    bool whole = false;       // every footprint of the warp is wholly inside the image or wholly outside
+    Foot f{};
     for (int mi = 0; mi < p.n_maps; mi++) {
       const GatherMap &m = p.maps[mi];
+      if (m.H != fh || m.W != fw) {
+        f = footprint(m.H, m.W, gx, gy);
+        if (!live) f.mask = 0;
+        fh = m.H;
+        fw = m.W;
+        staged = false;
+      }
       float first = 0.0f;
-      if (m.vec4 && p.groups) {
-        gather_rows(m, k0, total, s_foot[w8]);
+      if (m.rows) {
+        if (!staged) {
+          __syncwarp();  // the previous footprints' readers are done
+          s_foot[w8][lane].w = make_float4((f.mask & 1) ? f.w[0] : 0.0f, (f.mask & 2) ? f.w[1] : 0.0f,
+                                           (f.mask & 4) ? f.w[2] : 0.0f, (f.mask & 8) ? f.w[3] : 0.0f);
+          s_foot[w8][lane].a = make_int4(f.x0, f.y0, f.mask, img);
+          __syncwarp();
+          staged = true;
+          whole = __all_sync(SG_FULL, f.mask == 0 || f.mask == 15) && m.H > 1 && m.W > 1;
+        }
+        if (m.rows == 4) {
+          if (m.C <= 8) gather_rows_for<4, 2, SMALL>(m, k0, total, s_foot[w8], whole);
+          else if (m.C <= 16) gather_rows_for<4, 4, SMALL>(m, k0, total, s_foot[w8], whole);
+          else gather_rows_for<4, 8, SMALL>(m, k0, total, s_foot[w8], whole);
+        } else if (m.rows == 2) {
+          gather_rows_for<2, 8, SMALL>(m, k0, total, s_foot[w8], whole);
+        } else {
+          gather_rows_for<1, 8, SMALL>(m, k0, total, s_foot[w8], whole);
+        }
         if (mi == p.psdf_map && live) {  // channel 0 for the depth difference
 #pragma unroll
           for (int i = 0; i < 4; i++)
-            if ((f0.mask >> i) & 1) first = __fmaf_rn(__ldg(m.data + corner_off(m, img, f0.x0, f0.y0, i)), f0.w[i],
-                                                      first);
+            if ((f.mask >> i) & 1) first = __fmaf_rn(__ldg(m.data + corner_off(m, img, f.x0, f.y0, i)), f.w[i], first);
         }
       } else if (live) {
-        first = gather_map(m, img, k, m.H == p.maps[0].H && m.W == p.maps[0].W ? f0 : footprint(m.H, m.W, gx, gy));
+        first = gather_map<SMALL>(m, img, k, f);
       }
       if (mi == p.psdf_map && live) {
         const float dd = fminf(fmaxf(dep - first, -p.psdf_clip), p.psdf_clip);
         p.psdf[k] = dd * p.psdf_scale;
       }
     }
+  }
+}
+
+// A map [n, C, H, W] through its strides into [n, H, W, C]: a CTA moves 64
+// pixels x 32 channels through shared memory, read along x and written along
+// the channels, 128 bytes a warp either way: 4 x 32 x 512^2 floats in 85 us
+// cold (3.1 TB/s in and out; latency of the strided reads).
+constexpr int kClPix = 64, kClChan = 32;
+
+__global__ void __launch_bounds__(256) channels_last_kernel(const float *__restrict__ src, long sn, long sc, long sy,
+                                                            long sx, int C, int H, int W, float *__restrict__ dst) {
+  __shared__ float s[kClChan][kClPix + 1];
+  const int HW = H * W;
+  const int p0 = blockIdx.x * kClPix, c0 = blockIdx.y * kClChan;
+  const long n = blockIdx.z;
+  const bool lin = sy == (long)W * sx;
+#pragma unroll
+  for (int i = 0; i < kClPix * kClChan / 256; i++) {
+    const int j = i * 256 + threadIdx.x, c = j / kClPix, px = j % kClPix, q = p0 + px;
+    if (q < HW && c0 + c < C) {
+      const long at = lin ? (long)q * sx : (long)(q / W) * sy + (long)(q % W) * sx;
+      s[c][px] = __ldg(src + n * sn + (long)(c0 + c) * sc + at);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kClPix * kClChan / 256; i++) {
+    const int j = i * 256 + threadIdx.x, px = j / kClChan, c = j % kClChan, q = p0 + px;
+    if (q < HW && c0 + c < C) dst[(n * HW + q) * C + c0 + c] = s[c][px];
   }
 }
 
@@ -446,6 +615,7 @@ extern "C" int sg_project_gather(const SgProjGather *a, sg_stream_t stream) {
   p.grids = a->grids;
   p.depth = a->depth;
   p.n_maps = a->n_maps;
+  bool small = true;
   for (int i = 0; i < a->n_maps; i++) {
     const SgFeatureMap &m = a->maps[i];
     if (!m.data || !m.out || m.C <= 0 || m.H <= 0 || m.W <= 0) return SG_ERR_INVALID_ARG;
@@ -459,14 +629,20 @@ extern "C" int sg_project_gather(const SgProjGather *a, sg_stream_t stream) {
     g.H = m.H;
     g.W = m.W;
     g.out = m.out;
-    g.vec4 = (m.stride[1] == 1 && m.C % 4 == 0 && m.stride[0] % 4 == 0 && m.stride[2] % 4 == 0 &&
-              m.stride[3] % 4 == 0 && ((uintptr_t)m.data) % 16 == 0 && ((uintptr_t)m.out) % 16 == 0)
-                 ? 1
-                 : 0;
+    // rows: channels contiguous, more of them than a thread per item reads
+    // well (4), vectors as wide as the count, the strides and the addresses allow
+    g.rows = 0;
+    if (m.stride[1] == 1 && m.C > 4) {
+      auto fits = [&](int v) {
+        return m.C % v == 0 && m.stride[0] % v == 0 && m.stride[2] % v == 0 && m.stride[3] % v == 0 &&
+               ((uintptr_t)m.data) % (4 * v) == 0 && ((uintptr_t)m.out) % (4 * v) == 0;
+      };
+      g.rows = fits(4) ? 4 : (fits(2) ? 2 : 1);
+    }
+    auto mag = [](long long v) { return (double)(v < 0 ? -v : v); };
+    if (mag(m.stride[0]) * a->n_images + mag(m.stride[2]) * (m.H + 1.0) + mag(m.stride[3]) * (m.W + 1.0) + m.C >= 2147483647.0)
+      small = false;
   }
-  p.groups = a->n_maps > 0 ? 1 : 0;
-  for (int i = 0; i < a->n_maps; i++)
-    if (p.maps[i].vec4 && (p.maps[i].H != p.maps[0].H || p.maps[i].W != p.maps[0].W)) p.groups = 0;
   p.psdf_map = a->psdf_map;
   p.psdf_clip = a->psdf_clip;
   p.psdf_scale = a->psdf_scale;
@@ -476,7 +652,22 @@ extern "C" int sg_project_gather(const SgProjGather *a, sg_stream_t stream) {
   if (total > (1L << 40)) return SG_ERR_UNSUPPORTED;
   long g = (total + 255) / 256;
   if (g > (long)num_sms() * 64) g = (long)num_sms() * 64;
-  project_gather_kernel<<<(int)g, 256, 0, stream>>>(p);
+  if (small) project_gather_kernel<true><<<(int)g, 256, 0, stream>>>(p);
+  else project_gather_kernel<false><<<(int)g, 256, 0, stream>>>(p);
+  SG_LAUNCH_CHECK();
+  return SG_OK;
+}
+
+extern "C" int sg_channels_last(const float *src, const long long *stride, int n, int C, int H, int W, float *dst,
+                                sg_stream_t stream) {
+  if (n < 0 || C <= 0 || H <= 0 || W <= 0) return SG_ERR_INVALID_ARG;
+  if (n == 0) return SG_OK;
+  if (!src || !stride || !dst) return SG_ERR_INVALID_ARG;
+  const long hw = (long)H * W;
+  const long gy = (C + kClChan - 1) / kClChan;
+  if (hw > INT_MAX - kClPix || gy > 65535 || n > 65535) return SG_ERR_UNSUPPORTED;
+  const dim3 g((unsigned)((hw + kClPix - 1) / kClPix), (unsigned)gy, (unsigned)n);
+  channels_last_kernel<<<g, 256, 0, stream>>>(src, stride[0], stride[1], stride[2], stride[3], C, H, W, dst);
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
