@@ -331,7 +331,10 @@ class BatchPipeline:
                                            N.ptr(self.cams), N.stream()), "camera_params")
             N.check(N.lib.sg_segment_rays(C.byref(self.cam_seg), N.ptr(self.ori), N.ptr(self.dirs), N.stream()),
                     "segment_rays")
-        N.check(N.lib.sg_intersect_segments(C.byref(self.tree), C.byref(self.seg), N.ptr(self.ori),
+        # camera segments generate their rays again (the same bits), a warp per
+        # 8 x 4 pixels
+        seg = self.cam_seg if self.cameras else self.seg
+        N.check(N.lib.sg_intersect_segments(C.byref(self.tree), C.byref(seg), N.ptr(self.ori),
                                             N.ptr(self.dirs), self.W, N.ptr(self.hit_idx), N.ptr(self.hit_t0),
                                             N.ptr(self.hit_t1), N.ptr(self.valid_len), N.ptr(self.hit_count),
                                             N.ptr(self.status), N.stream()), "intersect_segments")
