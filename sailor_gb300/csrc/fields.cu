@@ -8,19 +8,26 @@
 // outside the grid contribute zero.  Sample point = ori + z * dir of its ray;
 // samples with z < 0 produce 0.
 //
-// grid_gather_kernel: one thread per sample; the eight corner reads of
-// neighbouring samples of a ray hit the same few cache lines (samples are
-// depth-sorted), so HBM traffic is about the touched grid bytes plus the
-// 4*C output bytes and 4-byte depth per sample.
+// grid_gather_kernel: a warp takes 32 consecutive samples: a lane per sample
+// finds its cell and corner weights; with C a multiple of 4, C / 4 lanes then
+// share each sample, a float4 of channels a lane, so that corner reads are
+// whole 64-byte texels and the output rows are written contiguously (a thread
+// per sample wrote its 16 channels 64 bytes apart from its neighbours': the
+// L1 data path was 73 % busy).  Sample -> ray -> frame by multiplication (two
+// 64-bit divisions a sample were a third of the 1- and 3-channel gathers).
+// 12.6 M samples x 16 channels of 256^3: 1.02 -> 0.74 ms; 16.8 M samples x 3
+// channels 122 -> 121 us, x 1 90 -> 78 us.
 //
-// grid_scatter_kernel (the adjoint): one warp per ray walks the ray's
-// samples in order; lane l owns the (corner, channel) slots l, l+32, ... of
-// the 8*C values a trilinear cell receives.  While consecutive samples stay in
-// one cell their contributions w_corner * g_channel accumulate in registers;
-// at a cell change (and at the end of the ray) the slots are flushed with one
-// atomic add each, C consecutive lanes covering one corner's C contiguous
-// channels.  Samples of a ray are depth-sorted and cluster in the few hit
-// voxels, so a flush carries many samples.
+// grid_scatter_kernel (the adjoint): 8 lanes per ray walk the ray's samples in
+// order, a lane per corner with its C channel sums in registers (four rays a
+// warp).  While consecutive samples stay in one trilinear cell their
+// contributions w_corner * g_channel accumulate; at a cell change (and at the
+// end of the ray) the lane adds its sums into the grid, four channels per
+// vector reduction where C is a multiple of 4.  Samples of a ray are
+// depth-sorted and cluster in the few hit voxels, so a flush carries many
+// samples.  A warp per ray, its lanes over the 8 C slots, took 88 warp
+// instructions a sample at C = 16 (staging through shared memory): 12.6 M
+// samples 1.16 -> 0.96 ms, at C = 1 0.69 -> 0.34 ms; now bound by the atomics.
 //
 // mode 1 turns a gathered normalised TSDF t (C == 1) into a density
 // sigma = sigmoid(-t * scale / s) / s  (scale = truncation margin in metres,
@@ -32,10 +39,28 @@
 
 namespace sg {
 
+// Division by a fixed d >= 1: q = (mulhi(n, m) + n) >> s for 0 <= n < 2^31
+// (T. Granlund, P. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994), the plain 64-bit quotient above that.
+struct FixedDiv {
+  uint32_t d, m, s;
+  int small;  // every dividend is below 2^31
+  static FixedDiv of(uint32_t d, long largest) {
+    FixedDiv f{d, 0u, 0u, largest < (1l << 31) ? 1 : 0};
+    while ((1ull << f.s) < d) f.s++;
+    f.m = (uint32_t)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
+    return f;
+  }
+  __device__ __forceinline__ long div(long n) const {
+    return small ? (long)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s) : n / (long)d;
+  }
+};
+
 struct GatherParams {
   const float *ori, *dir, *z;
   long R;
   int N, S;
+  FixedDiv by_S, by_N;
   const float *grid;
   int D, C;
   const float *vol_bbox, *voxel_size;
@@ -44,31 +69,117 @@ struct GatherParams {
   float *out;
 };
 
-template <int C>
-__global__ void __launch_bounds__(256) grid_gather_kernel(GatherParams p) {
-  const long n = p.R * p.S;
-  for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-    const long r = k / p.S;
-    const int b = (int)(r / p.N);
-    const float zz = __ldg(p.z + k);
-    float acc[C];
+// Geometry of a sample's frame, kept while the frame stays the same.
+struct FrameGeom {
+  int b = -1;
+  float bmin[3], vs, inv_vs;
+  __device__ __forceinline__ void load(const float *__restrict__ vol_bbox, const float *__restrict__ voxel_size, int frame) {
+    if (frame == b) return;
+    b = frame;
 #pragma unroll
-    for (int c = 0; c < C; c++) acc[c] = 0.0f;
-    if (zz >= 0.0f) {
-      const float *bb = p.vol_bbox + 6 * b;
-      const float bmin[3] = {bb[0], bb[2], bb[4]};
-      float pt[3];
-#pragma unroll
-      for (int a = 0; a < 3; a++) pt[a] = __fmaf_rn(__ldg(p.dir + r * 3 + a), zz, __ldg(p.ori + r * 3 + a));
-      grid_tap<C>(p.grid + (size_t)b * p.D * p.D * p.D * C, p.D, bmin, __ldg(p.voxel_size + b),
-                  1.0f / __ldg(p.voxel_size + b), pt, acc);
-      if (p.mode == 1) acc[0] = tsdf_density(acc[0], p.scale / p.s, 1.0f / p.s);
-    }
-#pragma unroll
-    for (int c = 0; c < C; c++) p.out[k * C + c] = acc[c];
+    for (int a = 0; a < 3; a++) bmin[a] = __ldg(vol_bbox + 6 * b + 2 * a);
+    vs = __ldg(voxel_size + b);
+    inv_vs = 1.0f / vs;
   }
+};
+
+// The 8 corners of a cell that lie in the grid, bit cr = (dx, dy, dz) of bits (2, 1, 0).
+__device__ __forceinline__ unsigned corners_inside(const int (&i0)[3], int D) {
+  unsigned m = 0xffu;
+  if (i0[0] < 0 || i0[0] >= D) m &= 0xf0u;
+  if (i0[0] + 1 < 0 || i0[0] + 1 >= D) m &= 0x0fu;
+  if (i0[1] < 0 || i0[1] >= D) m &= 0xccu;
+  if (i0[1] + 1 < 0 || i0[1] + 1 >= D) m &= 0x33u;
+  if (i0[2] < 0 || i0[2] >= D) m &= 0xaau;
+  if (i0[2] + 1 < 0 || i0[2] + 1 >= D) m &= 0x55u;
+  return m;
 }
 
+// VEC: grid and output are 16-byte aligned (C a multiple of 4).
+template <int C, bool VEC>
+__global__ void __launch_bounds__(256) grid_gather_kernel(GatherParams p) {
+  constexpr int L = VEC ? C / 4 : 1;  // lanes of a sample
+  const long n = p.R * p.S;
+  const int lane = lane_id();
+  const long dy = p.D, dx = (long)p.D * p.D;
+  FrameGeom g;
+  for (long k0 = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; k0 < n;
+       k0 += ((long)gridDim.x * blockDim.x >> 5) * 32) {
+    const long k = k0 + lane;
+    const float zz = k < n ? __ldg(p.z + k) : -1.0f;
+    unsigned in = 0u;
+    long off = 0;  // the lower corner's voxel, frame included
+    float f[3] = {0.0f, 0.0f, 0.0f};
+    if (zz >= 0.0f) {
+      const long r = p.by_S.div(k);
+      g.load(p.vol_bbox, p.voxel_size, (int)p.by_N.div(r));
+      float pt[3];
+      int i0[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) pt[a] = __fmaf_rn(__ldg(p.dir + r * 3 + a), zz, __ldg(p.ori + r * 3 + a));
+      tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
+      in = corners_inside(i0, p.D);
+      off = (((long)g.b * p.D + i0[0]) * p.D + i0[1]) * p.D + i0[2];
+    }
+    if constexpr (L == 1) {
+      float acc[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) acc[c] = 0.0f;
+#pragma unroll
+      for (int cr = 0; cr < 8; cr++) {
+        if (!((in >> cr) & 1u)) continue;
+        const float w = corner_weight(f, cr);
+        const float *v = p.grid + (off + ((cr & 4) ? dx : 0) + ((cr & 2) ? dy : 0) + (cr & 1)) * C;
+        if constexpr (VEC) {
+          const float4 q = __ldg(reinterpret_cast<const float4 *>(v));
+          acc[0] = __fmaf_rn(w, q.x, acc[0]);
+          acc[1] = __fmaf_rn(w, q.y, acc[1]);
+          acc[2] = __fmaf_rn(w, q.z, acc[2]);
+          acc[3] = __fmaf_rn(w, q.w, acc[3]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < C; c++) acc[c] = __fmaf_rn(w, __ldg(v + c), acc[c]);
+        }
+      }
+      if (p.mode == 1 && zz >= 0.0f) acc[0] = tsdf_density(acc[0], p.scale / p.s, 1.0f / p.s);
+      if (k < n) {
+        if constexpr (VEC) {
+          *reinterpret_cast<float4 *>(p.out + k * C) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < C; c++) p.out[k * C + c] = acc[c];
+        }
+      }
+    } else {
+      const int q = lane % L;
+#pragma unroll 1
+      for (int s0 = 0; s0 < 32; s0 += 32 / L) {
+        const int src = s0 + lane / L;
+        const unsigned m = __shfl_sync(SG_FULL, in, src);
+        const long o = __shfl_sync(SG_FULL, off, src);
+        const float fs[3] = {__shfl_sync(SG_FULL, f[0], src), __shfl_sync(SG_FULL, f[1], src),
+                             __shfl_sync(SG_FULL, f[2], src)};
+        const float4 *v = reinterpret_cast<const float4 *>(p.grid) + o * L + q;
+        float4 t[8];
+#pragma unroll
+        for (int cr = 0; cr < 8; cr++) {
+          t[cr] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if ((m >> cr) & 1u) t[cr] = __ldg(v + (((cr & 4) ? dx : 0) + ((cr & 2) ? dy : 0) + (cr & 1)) * L);
+        }
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int cr = 0; cr < 8; cr++) {
+          const float w = corner_weight(fs, cr);
+          acc.x = __fmaf_rn(w, t[cr].x, acc.x);
+          acc.y = __fmaf_rn(w, t[cr].y, acc.y);
+          acc.z = __fmaf_rn(w, t[cr].z, acc.z);
+          acc.w = __fmaf_rn(w, t[cr].w, acc.w);
+        }
+        if (k0 + src < n) __stcs(reinterpret_cast<float4 *>(p.out + (k0 + src) * C) + q, acc);
+      }
+    }
+  }
+}
 
 struct ScatterParams {
   const float *ori, *dir, *z;
@@ -83,96 +194,115 @@ struct ScatterParams {
   float *ggrid;        // [B, D, D, D, C], accumulated
 };
 
-template <int C>
-__device__ __forceinline__ void scatter_flush(const ScatterParams &p, int b, const int cell[3],
-                                              const float (&acc)[(8 * C + 31) / 32]) {
-  constexpr int NSLOT = (8 * C + 31) / 32;
-  const int lane = lane_id();
+// VEC: gradients and grid are 16-byte aligned (C a multiple of 4).
+template <int C, bool VEC>
+__device__ __forceinline__ void scatter_flush(const ScatterParams &p, long cell, int cr, unsigned in, float (&acc)[C]) {
+  if ((in >> cr) & 1u) {
+    float *g = p.ggrid + (cell + ((cr & 4) ? (long)p.D * p.D : 0) + ((cr & 2) ? p.D : 0) + (cr & 1)) * C;
+    if constexpr (VEC) {
 #pragma unroll
-  for (int q = 0; q < NSLOT; q++) {
-    const int slot = lane + 32 * q;
-    if (slot >= 8 * C || acc[q] == 0.0f) continue;
-    const int cr = slot / C, ch = slot - cr * C;
-    const int ix = cell[0] + ((cr >> 2) & 1), iy = cell[1] + ((cr >> 1) & 1), iz = cell[2] + (cr & 1);
-    if (ix < 0 || iy < 0 || iz < 0 || ix >= p.D || iy >= p.D || iz >= p.D) continue;
-    atomicAdd(p.ggrid + ((((size_t)b * p.D + ix) * p.D + iy) * p.D + iz) * C + ch, acc[q]);
+      for (int c = 0; c < C; c += 4)
+        if (acc[c] != 0.0f || acc[c + 1] != 0.0f || acc[c + 2] != 0.0f || acc[c + 3] != 0.0f)
+          red_add_f32x4(g + c, acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < C; c++)
+        if (acc[c] != 0.0f) atomicAdd(g + c, acc[c]);
+    }
   }
+#pragma unroll
+  for (int c = 0; c < C; c++) acc[c] = 0.0f;
 }
 
-template <int C>
+template <int C, bool VEC>
 __global__ void __launch_bounds__(256) grid_scatter_kernel(ScatterParams p) {
-  constexpr int NSLOT = (8 * C + 31) / 32;
-  __shared__ float s_w[8][32][9];      // padded rows: conflict-free per-lane writes
-  __shared__ float s_g[8][32][C + 1];
-  __shared__ int s_cell[8][32][5];
-  const int lane = lane_id(), w8 = threadIdx.x >> 5;
-  for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < p.R;
-       r += ((long)gridDim.x * blockDim.x) >> 5) {
-    const int b = (int)(r / p.N);
-    const float *bb = p.vol_bbox + 6 * b;
-    const float bmin[3] = {bb[0], bb[2], bb[4]};
-    const float vs = __ldg(p.voxel_size + b);
-    const float inv_vs = 1.0f / vs;
-    float acc[NSLOT];
+  const int cr = lane_id() & 7;  // corner, and sample of a step of 8
+  FrameGeom g;
+  const long nw = ((long)gridDim.x * blockDim.x) >> 5;
+  for (long r0 = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; r0 < p.R; r0 += nw * 4) {
+    const long r = r0 + (lane_id() >> 3);
+    const bool live = r < p.R;
+    float o[3] = {0.0f, 0.0f, 0.0f}, d[3] = {0.0f, 0.0f, 0.0f};
+    if (live) {
+      g.load(p.vol_bbox, p.voxel_size, (int)(r / p.N));
 #pragma unroll
-    for (int q = 0; q < NSLOT; q++) acc[q] = 0.0f;
-    int cur[3] = {INT_MIN, 0, 0};
-    for (int c0 = 0; c0 < p.S; c0 += 32) {
-      // per sample: cell, corner weights (as the forward tap forms them) and gradient
-      const int i = c0 + lane;
-      const float zz = i < p.S ? __ldg(p.z + r * p.S + i) : -1.0f;
-      int valid = 0;
+      for (int a = 0; a < 3; a++) {
+        o[a] = __ldg(p.ori + r * 3 + a);
+        d[a] = __ldg(p.dir + r * 3 + a);
+      }
+    }
+    float acc[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) acc[c] = 0.0f;
+    long cur = 0;        // lower corner's voxel of the current run
+    unsigned cur_in = 0u;
+    for (int c0 = 0; c0 < p.S; c0 += 8) {
+      // a lane per sample: cell, fractions (as the forward tap forms them) and,
+      // at one channel, the gradient
+      const int i = c0 + cr;
+      const float zz = live && i < p.S ? __ldg(p.z + r * p.S + i) : -1.0f;
+      unsigned in = 0u;
+      long cell = 0;
+      float f[3] = {0.0f, 0.0f, 0.0f}, g1 = 0.0f;
       if (zz >= 0.0f) {
-        float pt[3], wc[8];
+        float pt[3];
         int i0[3];
 #pragma unroll
-        for (int a = 0; a < 3; a++) pt[a] = __fmaf_rn(__ldg(p.dir + r * 3 + a), zz, __ldg(p.ori + r * 3 + a));
-        tap_cell(bmin, vs, inv_vs, pt, i0, wc);
+        for (int a = 0; a < 3; a++) pt[a] = __fmaf_rn(d[a], zz, o[a]);
+        tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
+        in = corners_inside(i0, p.D);
+        // with the corners that are inside, this names the cell (an index of -1
+        // on an axis wraps into the row before, whose own cells have other corners inside)
+        cell = (((long)g.b * p.D + i0[0]) * p.D + i0[1]) * p.D + i0[2];
+        if constexpr (C == 1) {
+          g1 = __ldg(p.gout + r * p.S + i);
+          if (p.mode == 1) {
+            // d sigma / d t of sigma = sigmoid(-t scale / s) / s at the gathered t
+            float t1[1], wc[8];
 #pragma unroll
-        for (int cr = 0; cr < 8; cr++) s_w[w8][lane][cr] = wc[cr];
-        s_cell[w8][lane][0] = i0[0];
-        s_cell[w8][lane][1] = i0[1];
-        s_cell[w8][lane][2] = i0[2];
-        const float *g = p.gout + ((size_t)r * p.S + i) * C;
-        if (p.mode == 1) {
-          // d sigma / d t of sigma = sigmoid(-t scale / s) / s at the gathered t
-          float t1[1];
-          grid_tap_cell<1>(p.grid + (size_t)b * p.D * p.D * p.D, p.D, i0, wc, t1);
-          const float k = p.scale / p.s;
-          const float sg = tsdf_sigmoid(t1[0], k);
-          s_g[w8][lane][0] = __ldg(g) * (-sg * (1.0f - sg) * (k * (1.0f / p.s)));
-        } else {
-#pragma unroll
-          for (int c = 0; c < C; c++) s_g[w8][lane][c] = __ldg(g + c);
-        }
-        valid = 1;
-      }
-      s_cell[w8][lane][3] = valid;
-      __syncwarp();
-      const int n = min(32, p.S - c0);
-      for (int j = 0; j < n; j++) {
-        if (!s_cell[w8][j][3]) continue;
-        const int cj[3] = {s_cell[w8][j][0], s_cell[w8][j][1], s_cell[w8][j][2]};
-        if (cj[0] != cur[0] || cj[1] != cur[1] || cj[2] != cur[2]) {
-          if (cur[0] != INT_MIN) scatter_flush<C>(p, b, cur, acc);
-#pragma unroll
-          for (int q = 0; q < NSLOT; q++) acc[q] = 0.0f;
-          cur[0] = cj[0];
-          cur[1] = cj[1];
-          cur[2] = cj[2];
-        }
-#pragma unroll
-        for (int q = 0; q < NSLOT; q++) {
-          const int slot = lane + 32 * q;
-          if (slot < 8 * C) {
-            const int cr = slot / C, ch = slot - cr * C;
-            acc[q] = __fmaf_rn(s_w[w8][j][cr], s_g[w8][j][ch], acc[q]);
+            for (int c = 0; c < 8; c++) wc[c] = corner_weight(f, c);
+            grid_tap_cell<1>(p.grid + (size_t)g.b * p.D * p.D * p.D, p.D, i0, wc, t1);
+            const float k = p.scale / p.s;
+            const float sg = tsdf_sigmoid(t1[0], k);
+            g1 = g1 * (-sg * (1.0f - sg) * (k * (1.0f / p.s)));
           }
         }
       }
-      __syncwarp();
+      const float *grow = p.gout + ((size_t)(live ? r : 0) * p.S + c0) * C;
+#pragma unroll 2
+      for (int j = 0; j < 8; j++) {
+        const unsigned inj = __shfl_sync(SG_FULL, in, j, 8);
+        const long cj = __shfl_sync(SG_FULL, cell, j, 8);
+        const float fj[3] = {__shfl_sync(SG_FULL, f[0], j, 8), __shfl_sync(SG_FULL, f[1], j, 8),
+                             __shfl_sync(SG_FULL, f[2], j, 8)};
+        float gj = 0.0f;
+        if constexpr (C == 1) gj = __shfl_sync(SG_FULL, g1, j, 8);
+        if (inj == 0u) continue;  // no sample, or no corner of it inside the grid
+        if (cj != cur || inj != cur_in) {
+          if (cur_in) scatter_flush<C, VEC>(p, cur, cr, cur_in, acc);
+          cur = cj;
+          cur_in = inj;
+        }
+        const float w = (((cr & 4) ? fj[0] : 1.0f - fj[0]) * ((cr & 2) ? fj[1] : 1.0f - fj[1])) *
+                        ((cr & 1) ? fj[2] : 1.0f - fj[2]);
+        if constexpr (C == 1) {
+          acc[0] = __fmaf_rn(w, gj, acc[0]);
+        } else if constexpr (VEC) {
+#pragma unroll
+          for (int c = 0; c < C; c += 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(grow + j * C + c));
+            acc[c] = __fmaf_rn(w, q.x, acc[c]);
+            acc[c + 1] = __fmaf_rn(w, q.y, acc[c + 1]);
+            acc[c + 2] = __fmaf_rn(w, q.z, acc[c + 2]);
+            acc[c + 3] = __fmaf_rn(w, q.w, acc[c + 3]);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < C; c++) acc[c] = __fmaf_rn(w, __ldg(grow + j * C + c), acc[c]);
+        }
+      }
     }
-    if (cur[0] != INT_MIN) scatter_flush<C>(p, b, cur, acc);
+    if (cur_in) scatter_flush<C, VEC>(p, cur, cr, cur_in, acc);
   }
 }
 
@@ -214,16 +344,27 @@ extern "C" int sg_grid_gather(const float *ori, const float *dir, const float *z
   if (!ori || !dir || !z || !grid || !vol_bbox || !voxel_size || !out) return SG_ERR_INVALID_ARG;
   if (B <= 0 || N <= 0 || S <= 0 || D <= 0 || C <= 0 || C > 16) return SG_ERR_INVALID_ARG;
   if (mode == 1 && (C != 1 || s == 0.0f)) return SG_ERR_INVALID_ARG;
-  GatherParams p{ori, dir, z, (long)B * N, N, S, grid, D, C, vol_bbox, voxel_size, mode, scale, s, out};
+  const long samples = (long)B * N * S;
+  GatherParams p{ori, dir, z, (long)B * N, N, S, FixedDiv::of(S, samples), FixedDiv::of(N, samples), grid, D, C, vol_bbox, voxel_size, mode, scale, s, out};
   long n = (long)B * N * S;
   int g = ceil_div(n, 256);
   if (g > num_sms() * 64) g = num_sms() * 64;
+  const bool vec = (((uintptr_t)grid) | ((uintptr_t)out)) % 16 == 0;
   switch (C) {
-    case 1: grid_gather_kernel<1><<<g, 256, 0, stream>>>(p); break;
-    case 3: grid_gather_kernel<3><<<g, 256, 0, stream>>>(p); break;
-    case 4: grid_gather_kernel<4><<<g, 256, 0, stream>>>(p); break;
-    case 8: grid_gather_kernel<8><<<g, 256, 0, stream>>>(p); break;
-    case 16: grid_gather_kernel<16><<<g, 256, 0, stream>>>(p); break;
+    case 1: grid_gather_kernel<1, false><<<g, 256, 0, stream>>>(p); break;
+    case 3: grid_gather_kernel<3, false><<<g, 256, 0, stream>>>(p); break;
+    case 4:
+      if (vec) grid_gather_kernel<4, true><<<g, 256, 0, stream>>>(p);
+      else grid_gather_kernel<4, false><<<g, 256, 0, stream>>>(p);
+      break;
+    case 8:
+      if (vec) grid_gather_kernel<8, true><<<g, 256, 0, stream>>>(p);
+      else grid_gather_kernel<8, false><<<g, 256, 0, stream>>>(p);
+      break;
+    case 16:
+      if (vec) grid_gather_kernel<16, true><<<g, 256, 0, stream>>>(p);
+      else grid_gather_kernel<16, false><<<g, 256, 0, stream>>>(p);
+      break;
     default: return SG_ERR_UNSUPPORTED;
   }
   SG_LAUNCH_CHECK();
@@ -241,14 +382,24 @@ extern "C" int sg_grid_scatter(const float *ori, const float *dir, const float *
   ScatterParams p{ori, dir, z, (long)B * N, N, S, grad_out, grid, D, vol_bbox, voxel_size, mode, scale, s,
                   grad_grid};
   long R = (long)B * N;
-  int g = ceil_div(R * 32, 256);
+  int g = ceil_div(R * 8, 256);
   if (g > num_sms() * 32) g = num_sms() * 32;
+  const bool vec = (((uintptr_t)grad_out) | ((uintptr_t)grad_grid)) % 16 == 0;
   switch (C) {
-    case 1: grid_scatter_kernel<1><<<g, 256, 0, stream>>>(p); break;
-    case 3: grid_scatter_kernel<3><<<g, 256, 0, stream>>>(p); break;
-    case 4: grid_scatter_kernel<4><<<g, 256, 0, stream>>>(p); break;
-    case 8: grid_scatter_kernel<8><<<g, 256, 0, stream>>>(p); break;
-    case 16: grid_scatter_kernel<16><<<g, 256, 0, stream>>>(p); break;
+    case 1: grid_scatter_kernel<1, false><<<g, 256, 0, stream>>>(p); break;
+    case 3: grid_scatter_kernel<3, false><<<g, 256, 0, stream>>>(p); break;
+    case 4:
+      if (vec) grid_scatter_kernel<4, true><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<4, false><<<g, 256, 0, stream>>>(p);
+      break;
+    case 8:
+      if (vec) grid_scatter_kernel<8, true><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<8, false><<<g, 256, 0, stream>>>(p);
+      break;
+    case 16:
+      if (vec) grid_scatter_kernel<16, true><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<16, false><<<g, 256, 0, stream>>>(p);
+      break;
     default: return SG_ERR_UNSUPPORTED;
   }
   SG_LAUNCH_CHECK();
