@@ -348,151 +348,110 @@ __device__ __forceinline__ void warp_sort_samples(float *sz, int *spos, int S, i
 }
 
 // ---------------------------------------------------------------------------
-// compositing (volume_rendering.cu:17-240)
+// compositing (volume_rendering.cu:17-240), a block of 32 positions at a time
 // ---------------------------------------------------------------------------
-// alpha per sorted position.  mode 0: 1 - exp(-sigma * delta) with delta to
-// the next position holding z > 0 (else the last position; 1e10 for the
-// last position itself, :87-97); mode 1: alpha = sigma.  s_z: depths by
-// sorted position.  Invalid positions (z < 0) get alpha 0.
-template <int E>
-__device__ __forceinline__ void ray_alpha(const float (&z)[E], const float (&sg)[E], unsigned valid, int S,
-                                          int mode, const float *s_z, float (&al)[E], float (&dl)[E]) {
-  const int lane = lane_id();
-  if (mode == 0) {
-    unsigned gtz[E];
+// Sum over the warp, pairs of neighbours first: the association of the
+// inclusive scan's last element (warp_incl_scan_f), so a total taken here
+// equals the one the adjoint's scans reach, bit for bit.
+__device__ __forceinline__ float warp_sum_scan_order(float v) {
 #pragma unroll
-    for (int e = 0; e < E; e++) gtz[e] = __ballot_sync(SG_FULL, z[e] > 0.0f);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const int i = e * 32 + lane;
-      al[e] = 0.0f;
-      dl[e] = 0.0f;
-      if ((valid >> e) & 1u) {
-        float delta;
-        if (i == S - 1) {
-          delta = 1e10f;
-        } else {
-          int m = S - 1;
-          const unsigned above = (lane == 31) ? 0u : (gtz[e] & (~0u << (lane + 1)));
-          if (above) {
-            m = e * 32 + __ffs(above) - 1;
-          } else {
-#pragma unroll
-            for (int e2 = 0; e2 < E; e2++)
-              if (e2 > e && gtz[e2] && m == S - 1) m = e2 * 32 + __ffs(gtz[e2]) - 1;
-          }
-          delta = s_z[m] - z[e];
-        }
-        dl[e] = delta;
-        al[e] = 1.0f - expf(-sg[e] * delta);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      al[e] = ((valid >> e) & 1u) ? sg[e] : 0.0f;
-      dl[e] = 0.0f;
-    }
-  }
+  for (int o = 1; o < 32; o <<= 1) v += __shfl_xor_sync(SG_FULL, v, o);
+  return v;
 }
 
-// Transmittance before each position, carried strictly sequentially over
-// positions (bit-identical to the reference's serial T *= 1 - alpha, so is
-// the early-termination decision T < t_thres, which the reference takes
-// after each valid sample).  proc: position reached; post: transmittance
-// after the position still >= t_thres.
-//
-// Every lane runs the same chain (warp-uniform), eight positions per step
-// from a shared-memory factor array; lane 0 stores the transmittance before
-// each position into a second array, which the owning lanes read back.
-// When every factor is in [0, 1] the product never increases (rounding is
-// monotonic), so one test of the step's last value finds the step where it
-// first falls below t_thres; otherwise the step's lowest value is tested.
-// The product changes only at valid positions.
-// Positions before the first valid one are padding (factor 1) and are
-// skipped.  s_f: kTransScratch<E> floats of warp-private shared scratch,
-// 16-byte aligned.
-template <int E>
-constexpr int kTransScratch = 2 * (32 * E + 8);
-
-template <int E>
-__device__ __forceinline__ void ray_transmittance(const float (&al)[E], unsigned valid, int S, float t_thres,
-                                                  float *s_f, float (&tb)[E], unsigned &proc, unsigned &post) {
+// Warp totals of 8 values: v[0] of lanes 4 k .. 4 k + 3 becomes the total of
+// value k, in the association of warp_sum.  Each exchange halves the values a
+// lane carries: 9 shuffles for 8 totals instead of 40.
+__device__ __forceinline__ void warp_sum8(float (&v)[8]) {
   const int lane = lane_id();
-  float *s_t = s_f + kTransScratch<E> / 2;
-  int m0 = 32 * E;
 #pragma unroll
-  for (int e = E - 1; e >= 0; e--) {
-    const unsigned vb = __ballot_sync(SG_FULL, (valid >> e) & 1u);
-    if (vb) m0 = e * 32 + __ffs(vb) - 1;
-  }
-  bool unit = true;  // every factor in [0, 1] (false for NaN)
+  for (int n = 4, o = 16; n >= 1; n >>= 1, o >>= 1) {
+    const bool hi = lane & o;
 #pragma unroll
-  for (int e = 0; e < E; e++) {
-    const float f = ((valid >> e) & 1u) ? (1.0f - al[e]) : 1.0f;
-    unit = unit && f >= 0.0f && f <= 1.0f;
-    s_f[e * 32 + lane] = f;
-  }
-  if (lane < 8) s_f[32 * E + lane] = 1.0f;  // the last step may read past position 32 E - 1
-  const bool mono = __all_sync(SG_FULL, unit);
-  __syncwarp();
-  int stop = 1 << 30;  // position whose update took T below t_thres
-  int end = S;
-  if (m0 < S) {
-    float T = 1.0f;
-    for (int i = m0 & ~3; i < S; i += 8) {
-      const float4 f0 = *reinterpret_cast<const float4 *>(s_f + i);
-      const float4 f1 = *reinterpret_cast<const float4 *>(s_f + i + 4);
-      float Ta[9];
-      Ta[0] = T;
-      Ta[1] = Ta[0] * f0.x;
-      Ta[2] = Ta[1] * f0.y;
-      Ta[3] = Ta[2] * f0.z;
-      Ta[4] = Ta[3] * f0.w;
-      Ta[5] = Ta[4] * f1.x;
-      Ta[6] = Ta[5] * f1.y;
-      Ta[7] = Ta[6] * f1.z;
-      Ta[8] = Ta[7] * f1.w;
-      if (lane == 0) {
-        *reinterpret_cast<float4 *>(s_t + i) = make_float4(Ta[0], Ta[1], Ta[2], Ta[3]);
-        *reinterpret_cast<float4 *>(s_t + i + 4) = make_float4(Ta[4], Ta[5], Ta[6], Ta[7]);
-      }
-      // lowest transmittance of the step: the last when the product cannot rise
-      float lo = Ta[8];
-      if (!mono)
-        lo = fminf(fminf(fminf(Ta[1], Ta[2]), fminf(Ta[3], Ta[4])), fminf(fminf(Ta[5], Ta[6]), fminf(Ta[7], Ta[8])));
-      if (lo < t_thres) {
-        // the first position q of [m0, S) in this step with T after it below
-        // t_thres (outside [m0, S) the factors are 1)
-        int k = 8;
-#pragma unroll
-        for (int q = 7; q >= 0; q--)
-          if (Ta[q + 1] < t_thres && i + q >= m0 && i + q < S) k = q;
-        if (k < 8) {
-          stop = i + k;
-          end = stop + 1;
-          break;
-        }
-      }
-      T = Ta[8];
-    }
-  } else {
-    end = 0;
-  }
-  __syncwarp();
-  proc = 0;
-  post = 0;
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int i = e * 32 + lane;
-    tb[e] = 0.0f;
-    if (i >= m0 && i < end) {
-      tb[e] = s_t[i];
-      proc |= 1u << e;
-      if (i != stop) post |= 1u << e;
+    for (int k = 0; k < n; k++) {
+      const float keep = hi ? v[k + n] : v[k], send = hi ? v[k] : v[k + n];
+      v[k] = keep + __shfl_xor_sync(SG_FULL, send, o);
     }
   }
+  v[0] += __shfl_xor_sync(SG_FULL, v[0], 2);
+  v[0] += __shfl_xor_sync(SG_FULL, v[0], 1);
+}
+
+// Transmittance through the 32 positions of a block, carried strictly in
+// order from T (the transmittance before the block): the reference's serial
+// T *= 1 - alpha, so the early-termination decision is the reference's too.
+// f: this lane's factor (1 where its position holds no sample); [lo, hi):
+// the block's positions at which termination counts.  Returns the position
+// in the block whose update took T below t_thres (32: none); tb: the
+// transmittance before this lane's position (valid up to that position).
+// Every lane runs the same chain, eight positions per step.  When every
+// factor is in [0, 1] the product cannot rise (rounding is monotonic), so
+// one test of the step's last value finds the step where it first falls
+// below t_thres; otherwise the step's lowest value is tested.
+// U: positions per unrolled stretch (8, or 32 where instructions are few).
+template <int U = 8>
+__device__ __forceinline__ int block_transmittance(float f, float &T, float t_thres, int lo, int hi, float *s_f,
+                                                   float &tb) {
+  const int lane = lane_id();
+  float *s_t = s_f + 32;
+  s_f[lane] = f;
+  const bool mono = __all_sync(SG_FULL, f >= 0.0f && f <= 1.0f);
   __syncwarp();
+  int stop = 32;
+#pragma unroll(U / 8)
+  for (int i = 0; i < 32; i += 8) {
+    const float4 f0 = *reinterpret_cast<const float4 *>(s_f + i);
+    const float4 f1 = *reinterpret_cast<const float4 *>(s_f + i + 4);
+    float Ta[9];
+    Ta[0] = T;
+    Ta[1] = Ta[0] * f0.x;
+    Ta[2] = Ta[1] * f0.y;
+    Ta[3] = Ta[2] * f0.z;
+    Ta[4] = Ta[3] * f0.w;
+    Ta[5] = Ta[4] * f1.x;
+    Ta[6] = Ta[5] * f1.y;
+    Ta[7] = Ta[6] * f1.z;
+    Ta[8] = Ta[7] * f1.w;
+    if (lane == 0) {
+      *reinterpret_cast<float4 *>(s_t + i) = make_float4(Ta[0], Ta[1], Ta[2], Ta[3]);
+      *reinterpret_cast<float4 *>(s_t + i + 4) = make_float4(Ta[4], Ta[5], Ta[6], Ta[7]);
+    }
+    float low = Ta[8];
+    if (!mono)
+      low = fminf(fminf(fminf(Ta[1], Ta[2]), fminf(Ta[3], Ta[4])), fminf(fminf(Ta[5], Ta[6]), fminf(Ta[7], Ta[8])));
+    if (low < t_thres) {
+      int k = 8;
+#pragma unroll
+      for (int q = 7; q >= 0; q--)
+        if (Ta[q + 1] < t_thres && i + q >= lo && i + q < hi) k = q;
+      if (k < 8) {
+        stop = i + k;
+        break;
+      }
+    }
+    T = Ta[8];
+  }
+  __syncwarp();
+  tb = s_t[lane];
+  return stop;
+}
+
+// Depth difference of position i (of S, depth z) in density mode: to the next
+// position holding a depth > 0 (else the last position); 1e10 for the last
+// position itself (volume_rendering.cu:87-97).  s_z: depths by position.
+__device__ __forceinline__ float depth_step(const float *s_z, int S, int i, float z) {
+  if (i == S - 1) return 1e10f;
+  float zn = s_z[i + 1];
+  if (!(zn > 0.0f)) {
+    int m = S - 1;
+    for (int q = i + 2; q < S; q++)
+      if (s_z[q] > 0.0f) {
+        m = q;
+        break;
+      }
+    zn = s_z[m];
+  }
+  return zn - z;
 }
 
 // ---------------------------------------------------------------------------

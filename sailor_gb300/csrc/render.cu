@@ -179,72 +179,6 @@ __device__ __forceinline__ RenderSmem render_smem(float *base, int mode, int cap
   return sm;
 }
 
-// Sum over the warp, pairs of neighbours first: the association of the
-// inclusive scan's last element (warp_incl_scan_f), so a total taken here
-// equals the one the adjoint's scans reach, bit for bit.
-__device__ __forceinline__ float warp_sum_scan_order(float v) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) v += __shfl_xor_sync(SG_FULL, v, o);
-  return v;
-}
-
-// Transmittance through the 32 positions of a block, carried strictly in
-// order from T (the transmittance before the block): the reference's serial
-// T *= 1 - alpha, so the early-termination decision is the reference's too.
-// f: this lane's factor (1 where its position holds no sample); [lo, hi):
-// the block's positions at which termination counts.  Returns the position
-// in the block whose update took T below t_thres (32: none); tb: the
-// transmittance before this lane's position (valid up to that position).
-// Every lane runs the same chain, eight positions per step.  When every
-// factor is in [0, 1] the product cannot rise (rounding is monotonic), so
-// one test of the step's last value finds the step where it first falls
-// below t_thres; otherwise the step's lowest value is tested.
-__device__ __forceinline__ int block_transmittance(float f, float &T, float t_thres, int lo, int hi, float *s_f,
-                                                   float &tb) {
-  const int lane = lane_id();
-  float *s_t = s_f + 32;
-  s_f[lane] = f;
-  const bool mono = __all_sync(SG_FULL, f >= 0.0f && f <= 1.0f);
-  __syncwarp();
-  int stop = 32;
-#pragma unroll 1
-  for (int i = 0; i < 32; i += 8) {
-    const float4 f0 = *reinterpret_cast<const float4 *>(s_f + i);
-    const float4 f1 = *reinterpret_cast<const float4 *>(s_f + i + 4);
-    float Ta[9];
-    Ta[0] = T;
-    Ta[1] = Ta[0] * f0.x;
-    Ta[2] = Ta[1] * f0.y;
-    Ta[3] = Ta[2] * f0.z;
-    Ta[4] = Ta[3] * f0.w;
-    Ta[5] = Ta[4] * f1.x;
-    Ta[6] = Ta[5] * f1.y;
-    Ta[7] = Ta[6] * f1.z;
-    Ta[8] = Ta[7] * f1.w;
-    if (lane == 0) {
-      *reinterpret_cast<float4 *>(s_t + i) = make_float4(Ta[0], Ta[1], Ta[2], Ta[3]);
-      *reinterpret_cast<float4 *>(s_t + i + 4) = make_float4(Ta[4], Ta[5], Ta[6], Ta[7]);
-    }
-    float low = Ta[8];
-    if (!mono)
-      low = fminf(fminf(fminf(Ta[1], Ta[2]), fminf(Ta[3], Ta[4])), fminf(fminf(Ta[5], Ta[6]), fminf(Ta[7], Ta[8])));
-    if (low < t_thres) {
-      int k = 8;
-#pragma unroll
-      for (int q = 7; q >= 0; q--)
-        if (Ta[q + 1] < t_thres && i + q >= lo && i + q < hi) k = q;
-      if (k < 8) {
-        stop = i + k;
-        break;
-      }
-    }
-    T = Ta[8];
-  }
-  __syncwarp();
-  tb = s_t[lane];
-  return stop;
-}
-
 // Geometry of a ray: what the taps of its samples need.
 struct RayGeom {
   float o[3], d[3];
@@ -486,23 +420,7 @@ __device__ __forceinline__ bool eval_block(const RenderParams &p, const RayGeom 
     }
     v.s01 = tsdf_sigmoid(t1[0], p.dk);  // kept for the adjoint
     const float sg = v.s01 * p.inv_s;
-    // the step to the next position with z > 0 (else the last position);
-    // 1e10 behind the last position (volume_rendering.cu:87-97)
-    if (i == S - 1) {
-      v.dl = 1e10f;
-    } else {
-      float zn = sm.z[i + 1];
-      if (!(zn > 0.0f)) {
-        int m = S - 1;
-        for (int q = i + 2; q < S; q++)
-          if (sm.z[q] > 0.0f) {
-            m = q;
-            break;
-          }
-        zn = sm.z[m];
-      }
-      v.dl = zn - v.z;
-    }
+    v.dl = depth_step(sm.z, S, i, v.z);
     v.al = 1.0f - expf(-sg * v.dl);
   }
   const int stop = block_transmittance(valid ? 1.0f - v.al : 1.0f, wk.T, p.t_thres, wk.m0 - e * 32, S - e * 32, sm.f,
