@@ -18,25 +18,34 @@
 // child order) below -- children of one node are a contiguous run of the
 // next level.  All counts stay on the device; no host synchronisation.
 //
-// Traversal: one thread per ray.  The reference's coarse pass writes a row
-// per ray and then runs one thread per (ray, coarse hit) that descends
-// through an 8-entry stack and appends with atomicAdd.  Here the ray's thread
-// descends each coarse node as soon as the DDA records it, with one cursor
-// per level (no stack bound: a node's children are a contiguous run), in
-// the reference's per-node order (children last to first), and writes the
-// fine row in coarse order.  The comparison that merges a descendant into an
-// entry with bit-identical depths reads the entries already in the row, and
-// only when a 64-bit filter of the coarse node's entry depths says a match
-// is possible.  Node keys decode with shifts where a level's edge is a power
-// of two, each level's node geometry is set once per ray, a node's key and
-// child run are loaded together, and each warp pads its 32 rows' tails
-// itself (16-byte stores) once its rays are done.
+// Traversal: two passes.  A thread per ray walks the start level and writes
+// the coarse row; then a warp takes four rays and lays their coarse nodes out
+// over its lanes, a descent a lane, with one cursor per level (no stack bound:
+// a node's children are a contiguous run) in the reference's per-node order
+// (children last to first).  A descent's entries wait in shared memory for the
+// warp's scan, which gives them their places in coarse order (the reference
+// runs a thread per (ray, coarse hit) with an 8-entry stack and appends with
+// atomicAdd).  The comparison that merges a descendant into an entry with
+// bit-identical depths reads the list only when a 64-bit filter of the coarse
+// node's entry depths says a match is possible.  A ray whose coarse row, list
+// or fine row is too short is walked again, its nodes descended into the row
+// one after the other: what it holds past a full row depends on that order.
+// Node keys decode with shifts where a level's edge is a power of two, and a
+// node's key and child run are loaded together.
+//
+// When a ray's own thread descended its nodes as it met them, a warp took the
+// sum of its lanes' descents (hits fall on different steps) and 7 % of the
+// warps were active.  262144 rays x (192 + 512) entries, four levels of 256^3,
+// 17 % of the rays hitting 9 nodes: 1.08 -> 0.15 (walk) + 0.34 ms; the rows
+// alone take 0.33 ms to write at the copy rate.  Rays a warp: 8 590, 4 541, 2 524,
+// 1 611 us for the call (4 keeps the lanes filled where rays hit few nodes).
 //
 // Fine sampling: one warp per ray; per chunk of 32 entries a warp scan turns
 // the per-entry sample counts into slot ranges and the chunk's samples are
 // generated slot-parallel (owner found by binary search over the chunk's
 // starts); the fill step is a warp arg-min over (node edge, midpoint,
-// position).
+// position); a ray without entries is only filled.  A CTA every few rays (64 an
+// SM at most; 16: 206 us, 64: 163 us for the call on 262144 rays x 64 samples).
 #include "common.cuh"
 #include "ray_core.cuh"
 #include "segsort.cuh"
@@ -53,23 +62,23 @@ struct OctMeta {
   const int *vol[SG_MAX_LEVELS], *key[SG_MAX_LEVELS], *child_base[SG_MAX_LEVELS], *nchild[SG_MAX_LEVELS];
 };
 
+// A thread per level.  t: a kernel parameter marked __grid_constant__ (indexed
+// in place).
 __device__ __forceinline__ void load_meta(const SgOctree &t, OctMeta &m) {
-  if (threadIdx.x == 0) {
-    m.L = t.L;
-#pragma unroll
-    for (int l = 0; l < SG_MAX_LEVELS; l++) {
-      m.dim[l] = t.dim[l];
-      m.base[l] = t.base[l];
-      m.cap[l] = t.cap[l];
-      m.vol[l] = t.vol[l];
-      m.key[l] = t.key[l];
-      m.child_base[l] = t.child_base[l];
-      m.nchild[l] = t.nchild[l];
-      m.count[l] = (l < t.L && t.counts) ? min(t.counts[l], t.cap[l]) : 0;
-      const int D = t.dim[l];
-      m.shift[l] = (D > 0 && (D & (D - 1)) == 0) ? __ffs(D) - 1 : -1;
-      m.size[l] = D > 0 ? (float)(t.dim[0] / D) : 0.0f;
-    }
+  const int l = threadIdx.x;
+  if (l == 0) m.L = t.L;
+  if (l < SG_MAX_LEVELS) {
+    m.dim[l] = t.dim[l];
+    m.base[l] = t.base[l];
+    m.cap[l] = t.cap[l];
+    m.vol[l] = t.vol[l];
+    m.key[l] = t.key[l];
+    m.child_base[l] = t.child_base[l];
+    m.nchild[l] = t.nchild[l];
+    m.count[l] = (l < t.L && t.counts) ? min(t.counts[l], t.cap[l]) : 0;
+    const int D = t.dim[l];
+    m.shift[l] = (D > 0 && (D & (D - 1)) == 0) ? __ffs(D) - 1 : -1;
+    m.size[l] = D > 0 ? (float)(t.dim[0] / D) : 0.0f;
   }
 }
 
@@ -202,7 +211,7 @@ __global__ void oct_child_emit_kernel(const int *__restrict__ n_dev, int cap, co
   }
 }
 
-__global__ void oct_nodes_kernel(SgOctree t, int n_nodes, float *out) {
+__global__ void oct_nodes_kernel(const __grid_constant__ SgOctree t, int n_nodes, float *out) {
   __shared__ OctMeta m;
   load_meta(t, m);
   __syncthreads();
@@ -251,221 +260,351 @@ __device__ __forceinline__ float level_edge(const OctMeta &m, float vs, int l) {
 }
 
 constexpr int kTravThreads = 128;
+constexpr int kTravRays = 4;  // rays a warp of the descent takes
 
 // one of 64 bits chosen by the bits of t (multiplicative hash)
 __device__ __forceinline__ unsigned long long t0_bit(float t) {
   return 1ull << ((__float_as_uint(t + 0.0f) * 0x9E3779B1u) >> 26);
 }
 
-__global__ void __launch_bounds__(kTravThreads, 8) octree_traverse_kernel(OctTravParams p) {
+struct TravRay {
+  float o[3], d[3], inv[3];
+  int b;
+  float vs;  // fine voxel edge of the ray's frame
+};
+
+__device__ __forceinline__ TravRay trav_ray(const OctTravParams &p, long r) {
+  TravRay y;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    y.o[a] = __ldg(p.ori + r * 3 + a);
+    y.d[a] = __ldg(p.dir + r * 3 + a);
+    y.inv[a] = __fdividef(1.0f, y.d[a]);
+  }
+  y.b = (int)(r / p.N);
+  y.vs = __ldg(p.t.voxel_size + y.b);
+  return y;
+}
+
+// The nodes of level s that the ray meets, in the DDA's order: hit(id, t0, t1).
+template <typename F>
+__device__ __forceinline__ void walk_level(const OctTravParams &p, const OctMeta &m, const TravRay &y, F &&hit) {
+  const int s = p.s, Ds = m.dim[s];
+  const float *bb = p.t.vol_bbox + 6 * y.b;
+  const float bmin[3] = {bb[0], bb[2], bb[4]};
+  const float xc = (bb[0] + bb[1]) / 2.0f, yc = (bb[2] + bb[3]) / 2.0f, zc = (bb[4] + bb[5]) / 2.0f;
+  const float vs = y.vs, vs_top = vs * (float)(m.dim[0] / Ds);
+  float T0, T1;
+  if (!slab(y.o, y.inv, xc, yc, zc, vs_top * (float)Ds, T0, T1) || T0 < 0.0f || T1 < 0.0f) return;
+  const LevelGeom gs = level_geom(vs, m.dim[0] / Ds);
+  const long vt = (long)Ds * Ds * Ds;
+  const int *vol_s = m.vol[s], *key_s = m.key[s];
+  int st[3];
+  float step[3], tm[3], td[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float so = __fmaf_rn(T0, y.d[a], y.o[a]) - (bmin[a] - vs / 2.0f);
+    int q = (int)(so / vs_top);
+    q = q < 0 ? 0 : q;
+    st[a] = q < Ds ? q : Ds - 1;
+    step[a] = (y.d[a] >= 0) ? 1.0f : -1.0f;
+    const float nb = (step[a] > 0) ? ((float)st[a] + step[a]) * vs_top : (float)st[a] * vs_top;
+    tm[a] = (y.d[a] != 0) ? (nb - so) / y.d[a] : 9999999.0f;
+    td[a] = (y.d[a] != 0) ? vs_top / y.d[a] * step[a] : 9999999.0f;
+  }
+  const int J = 4 * Ds;
+  bool pre_empty = false, has_valid = false;
+  int nsucc = 0, nint = 0;
+  for (int j = 0; j < J; j++) {
+    const long cell = (long)y.b * vt + ((long)st[0] * Ds + st[1]) * Ds + st[2];
+    const int v = vol_s[cell];
+    const int k0 = v - m.base[s];
+    bool node = v > -1 && k0 >= 0 && k0 < m.count[s] && key_s[k0] == (int)cell;
+    if (node) {
+      float p0, p1;
+      node = slab(y.o, y.inv, node_coord(gs, bmin[0], st[0]), node_coord(gs, bmin[1], st[1]),
+                  node_coord(gs, bmin[2], st[2]), gs.vs, p0, p1) &&
+             !(p0 < 0.0f || p1 < 0.0f);
+      if (node) hit(v, p0, p1);
+    }
+    if (p.th_early_stop > -1) {
+      if (!node) {
+        if (pre_empty && has_valid) nsucc++;
+        pre_empty = true;
+      } else {
+        nsucc = 0;
+        pre_empty = false;
+        has_valid = true;
+      }
+      if ((nsucc + 1) >= p.th_early_stop) break;
+    }
+    if (p.opt_num > -1) {
+      if (node) nint++;
+      if (nint >= p.opt_num) break;
+    }
+    const int ax = tm[0] < tm[1] ? (tm[0] < tm[2] ? 0 : 2) : (tm[1] < tm[2] ? 1 : 2);
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      if (a == ax) {
+        st[a] += (int)step[a];
+        tm[a] += td[a];
+      }
+    if (st[0] < 0 || st[0] >= Ds || st[1] < 0 || st[1] >= Ds || st[2] < 0 || st[2] >= Ds) break;
+  }
+}
+
+// Entries of a coarse node: entry e at [e * STRIDE], n of them wanted, the
+// first cap stored.
+template <int STRIDE>
+struct Entries {
+  int *id;
+  float *t0, *t1;
+  int n, cap;
+  __device__ __forceinline__ void put(int v, float a, float c) {
+    if (n < cap) {
+      id[n * STRIDE] = v;
+      t0[n * STRIDE] = a;
+      t1[n * STRIDE] = c;
+    }
+    n++;
+  }
+};
+
+// Depth-first descent of the coarse node `v` (entry depths p0, p1), children
+// last to first; a descendant whose depths equal a stored entry's takes its
+// place if it is of a finer level, and is no entry of its own.  g_vs, g_st: the
+// ray's frame's node geometry by level, GS apart.
+template <int STRIDE, int GS>
+__device__ __forceinline__ void descend(const OctMeta &m, int s, const TravRay &y, const float (&bmin)[3],
+                                        const float *g_vs, const float *g_st, int v, float p0, float p1,
+                                        Entries<STRIDE> &en) {
+  int cbs[SG_MAX_LEVELS], cur[SG_MAX_LEVELS];
+  // bit per hashed t0 of the stored entries: a depth whose bit is clear matches
+  // no entry (equal depths hash alike; + 0.0f folds -0 into +0, which compare equal)
+  unsigned long long seen = en.n < en.cap ? t0_bit(p0) : 0ull;
+  en.put(v, p0, p1);
+  int depth = -1;
+  if (s > 0) {
+    const int k0 = v - m.base[s], nc0 = m.nchild[s][k0];
+    if (nc0 > 0) {
+      depth = 0;
+      cbs[0] = m.child_base[s][k0];
+      cur[0] = nc0 - 1;
+    }
+  }
+  while (depth >= 0) {
+    if (cur[depth] < 0) {
+      depth--;
+      continue;
+    }
+    const int lv = s - 1 - depth;
+    const int kk = cbs[depth] + cur[depth];
+    cur[depth]--;
+    if (kk >= m.count[lv]) continue;  // a level past its capacity (flagged by the build)
+    // the node's key and child run, loaded together
+    const int key = m.key[lv][kk];
+    int nc = 0, cbn = 0;
+    if (lv > 0) {
+      nc = m.nchild[lv][kk];
+      cbn = m.child_base[lv][kk];
+    }
+    int cx, cy, cz;
+    decode_node(m, lv, key, cx, cy, cz);
+    const LevelGeom gl{g_vs[lv * GS], g_st[lv * GS]};
+    float c0, c1;
+    if (!slab(y.o, y.inv, node_coord(gl, bmin[0], cx), node_coord(gl, bmin[1], cy), node_coord(gl, bmin[2], cz),
+              gl.vs, c0, c1))
+      continue;
+    const int cid = m.base[lv] + kk;
+    bool found = false;
+    const unsigned long long hb = t0_bit(c0);
+    if (seen & hb) {
+      const int ne = min(en.n, en.cap);
+      for (int e = 0; e < ne; e++) {
+        if (en.t0[e * STRIDE] == c0 && en.t1[e * STRIDE] == c1) {
+          if (level_edge(m, y.vs, meta_level_of(m, en.id[e * STRIDE])) > gl.vs) en.id[e * STRIDE] = cid;
+          found = true;
+          break;
+        }
+      }
+    }
+    if (!found) {
+      if (en.n < en.cap) seen |= hb;
+      en.put(cid, c0, c1);
+    }
+    if (nc > 0) {
+      depth++;
+      cbs[depth] = cbn;
+      cur[depth] = nc - 1;
+    }
+  }
+}
+
+// First pass: a thread per ray walks the start level; coarse rows and counts.
+__global__ void __launch_bounds__(kTravThreads) octree_walk_kernel(const __grid_constant__ OctTravParams p) {
   __shared__ OctMeta m;
-  // the ray's frame's node geometry per level (edge, offset), one column
-  // per thread: set once per ray instead of once per tested node
-  __shared__ float g_vs[SG_MAX_LEVELS][kTravThreads], g_st[SG_MAX_LEVELS][kTravThreads];
   load_meta(p.t, m);
   __syncthreads();
   const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int tid = threadIdx.x;
-  const int s = p.s;
-  int cc = 0, fc = 0;
-  if (r < p.R) {
-    const SgOctree &t = p.t;
-    const int b = (int)(r / p.N);
-    const int Ds = m.dim[s];
-    const float *bb = t.vol_bbox + 6 * b;
-    const float bmin[3] = {bb[0], bb[2], bb[4]};
-    const float xc = (bb[0] + bb[1]) / 2.0f, yc = (bb[2] + bb[3]) / 2.0f, zc = (bb[4] + bb[5]) / 2.0f;
-    const float vs = t.voxel_size[b];
-    const float vs_top = vs * (float)(m.dim[0] / Ds);
-    const float bst[3] = {bb[0] - vs / 2.0f, bb[2] - vs / 2.0f, bb[4] - vs / 2.0f};
-    const float o[3] = {p.ori[r * 3 + 0], p.ori[r * 3 + 1], p.ori[r * 3 + 2]};
-    const float d[3] = {p.dir[r * 3 + 0], p.dir[r * 3 + 1], p.dir[r * 3 + 2]};
-    const float inv[3] = {__fdividef(1.0f, d[0]), __fdividef(1.0f, d[1]), __fdividef(1.0f, d[2])};
-    const LevelGeom gs = level_geom(vs, m.dim[0] / Ds);
-    for (int l = 0; l < s; l++) {
-      const LevelGeom g = level_geom(vs, m.dim[0] / m.dim[l]);
-      g_vs[l][tid] = g.vs;
-      g_st[l][tid] = g.start;
-    }
-    const long vt = (long)Ds * Ds * Ds;
-    const int *vol_s = m.vol[s], *key_s = m.key[s];
-    int *oic = p.idx_c + (size_t)r * p.Wc;
-    float *o0c = p.t0_c + (size_t)r * p.Wc, *o1c = p.t1_c + (size_t)r * p.Wc;
-    int *oif = p.idx + (size_t)r * p.Wf;
-    float *o0f = p.t0 + (size_t)r * p.Wf, *o1f = p.t1 + (size_t)r * p.Wf;
-    float vlen = 0.0f;
-    float T0, T1;
-    if (slab(o, inv, xc, yc, zc, vs_top * (float)Ds, T0, T1) && !(T0 < 0.0f || T1 < 0.0f)) {
-      float so[3];
-      int st[3];
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        float sp = __fmaf_rn(T0, d[a], o[a]);
-        so[a] = sp - bst[a];
-        int q = (int)(so[a] / vs_top);
-        q = q < 0 ? 0 : q;
-        st[a] = q < Ds ? q : Ds - 1;
-      }
-      float step[3], tm[3], td[3];
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        step[a] = (d[a] >= 0) ? 1.0f : -1.0f;
-        float nb = (step[a] > 0) ? ((float)st[a] + step[a]) * vs_top : (float)st[a] * vs_top;
-        tm[a] = (d[a] != 0) ? (nb - so[a]) / d[a] : 9999999.0f;
-        td[a] = (d[a] != 0) ? vs_top / d[a] * step[a] : 9999999.0f;
-      }
-      const int J = 4 * Ds;
-      bool pre_empty = false, has_valid = false;
-      int nsucc = 0, nint = 0;
-      int cbs[SG_MAX_LEVELS], cur[SG_MAX_LEVELS];
-      for (int j = 0; j < J; j++) {
-        int rid = -1;
-        const long cell = (long)b * vt + ((long)st[0] * Ds + st[1]) * Ds + st[2];
-        const int v = vol_s[cell];
-        const int k0 = v - m.base[s];
-        bool node = v > -1 && k0 >= 0 && k0 < m.count[s];
-        int nc0 = 0, cb0 = 0;
-        if (node) {
-          // the node's key and child run, loaded together
-          const int kv = key_s[k0];
-          if (s > 0) {
-            nc0 = m.nchild[s][k0];
-            cb0 = m.child_base[s][k0];
-          }
-          node = kv == (int)cell;
-        }
-        if (node) {
-          float p0, p1;
-          if (slab(o, inv, node_coord(gs, bmin[0], st[0]), node_coord(gs, bmin[1], st[1]),
-                   node_coord(gs, bmin[2], st[2]), gs.vs, p0, p1) &&
-              !(p0 < 0.0f || p1 < 0.0f)) {
-            rid = cc;
-            if (cc < p.Wc) {
-              oic[cc] = v;
-              o0c[cc] = p0;
-              o1c[cc] = p1;
-            }
-            cc++;
-            // descent from this coarse node
-            const int f0 = fc;
-            // bit per hashed t0 of this coarse node's stored entries: a
-            // depth whose bit is clear matches no entry (equal depths hash
-            // alike; + 0.0f folds -0 into +0, which compare equal)
-            unsigned long long seen = fc < p.Wf ? t0_bit(p0) : 0ull;
-            if (fc < p.Wf) {
-              oif[fc] = v;
-              o0f[fc] = p0;
-              o1f[fc] = p1;
-            }
-            fc++;
-            int depth = -1;
-            if (nc0 > 0) {
-              depth = 0;
-              cbs[0] = cb0;
-              cur[0] = nc0 - 1;
-            }
-            while (depth >= 0) {
-              if (cur[depth] < 0) {
-                depth--;
-                continue;
-              }
-              const int lv = s - 1 - depth;
-              const int kk = cbs[depth] + cur[depth];
-              cur[depth]--;
-              if (kk >= m.count[lv]) continue;  // a level past its capacity (flagged by the build)
-              // the node's key and child run, loaded together
-              const int key = m.key[lv][kk];
-              int nc = 0, cbn = 0;
-              if (lv > 0) {
-                nc = m.nchild[lv][kk];
-                cbn = m.child_base[lv][kk];
-              }
-              int cx, cy, cz;
-              decode_node(m, lv, key, cx, cy, cz);
-              const LevelGeom gl{g_vs[lv][tid], g_st[lv][tid]};
-              float c0, c1;
-              if (!slab(o, inv, node_coord(gl, bmin[0], cx), node_coord(gl, bmin[1], cy),
-                        node_coord(gl, bmin[2], cz), gl.vs, c0, c1))
-                continue;
-              const int cid = m.base[lv] + kk;
-              bool found = false;
-              const unsigned long long hb = t0_bit(c0);
-              if (seen & hb) {
-                const int fe = min(fc, p.Wf);
-                for (int e = f0; e < fe; e++) {
-                  if (o0f[e] == c0 && o1f[e] == c1) {
-                    const int pid = oif[e];
-                    if (level_edge(m, vs, meta_level_of(m, pid)) > gl.vs) oif[e] = cid;
-                    found = true;
-                    break;
-                  }
-                }
-              }
-              if (!found) {
-                if (fc < p.Wf) {
-                  oif[fc] = cid;
-                  o0f[fc] = c0;
-                  o1f[fc] = c1;
-                  seen |= hb;
-                }
-                fc++;
-              }
-              if (nc > 0) {
-                depth++;
-                cbs[depth] = cbn;
-                cur[depth] = nc - 1;
-              }
-            }
-            const int fe = min(fc, p.Wf);
-            for (int e = f0; e < fe; e++) {
-              const float scale = gs.vs / level_edge(m, vs, meta_level_of(m, oif[e]));
-              vlen = vlen + (o1f[e] - o0f[e]) * scale;
-            }
-          }
-        }
-        if (p.th_early_stop > -1) {
-          if (rid == -1) {
-            if (pre_empty && has_valid) nsucc++;
-            pre_empty = true;
-          } else {
-            nsucc = 0;
-            pre_empty = false;
-            has_valid = true;
-          }
-          if ((nsucc + 1) >= p.th_early_stop) break;
-        }
-        if (p.opt_num > -1) {
-          if (rid + 1 > 0) nint++;
-          if (nint >= p.opt_num) break;
-        }
-        int ax;
-        if (tm[0] < tm[1]) ax = (tm[0] < tm[2]) ? 0 : 2;
-        else ax = (tm[1] < tm[2]) ? 1 : 2;
-        st[ax] += (int)step[ax];
-        tm[ax] += td[ax];
-        if (st[0] < 0 || st[0] >= Ds || st[1] < 0 || st[1] >= Ds || st[2] < 0 || st[2] >= Ds) break;
-      }
-    }
-    p.vl[r] = vlen;
-    if (p.cnt_c) p.cnt_c[r] = cc;
-    if (p.cnt) p.cnt[r] = fc;
-    if (p.st) {
-      if (cc > 0) atomicMax(&p.st->max_coarse, cc);
-      if (fc > 0) atomicMax(&p.st->max_fine, fc);
-      if (cc > p.Wc || fc > p.Wf) atomicOr(&p.st->flags, SG_FLAG_HIT_OVERFLOW);
-    }
-  }
-  // -1 padding of the warp's 32 rows, each by the whole warp (16-byte
-  // stores; the rays' own threads would write them one element at a time)
   const int lane = lane_id();
+  int cc = 0;
+  if (r < p.R) {
+    int *oi = p.idx_c + (size_t)r * p.Wc;
+    float *o0 = p.t0_c + (size_t)r * p.Wc, *o1 = p.t1_c + (size_t)r * p.Wc;
+    walk_level(p, m, trav_ray(p, r), [&](int v, float p0, float p1) {
+      if (cc < p.Wc) {
+        oi[cc] = v;
+        o0[cc] = p0;
+        o1[cc] = p1;
+      }
+      cc++;
+    });
+    p.cnt_c[r] = cc;
+  }
+  const int most = __reduce_max_sync(SG_FULL, cc);
+  if (p.st && lane == 0 && most > 0) {
+    atomicMax(&p.st->max_coarse, most);
+    if (most > p.Wc) atomicOr(&p.st->flags, SG_FLAG_HIT_OVERFLOW);
+  }
   const long r0 = r - lane;
   for (int i = 0; i < 32; i++) {
-    const int ci = __shfl_sync(SG_FULL, cc, i), fi = __shfl_sync(SG_FULL, fc, i);
-    const long ri = r0 + i;
-    if (ri >= p.R) break;
-    pad_row_tail(p.idx_c, p.t0_c, p.t1_c, (size_t)ri * p.Wc, min(ci, p.Wc), p.Wc, lane);
-    pad_row_tail(p.idx, p.t0, p.t1, (size_t)ri * p.Wf, min(fi, p.Wf), p.Wf, lane);
+    const int ci = __shfl_sync(SG_FULL, cc, i);
+    if (r0 + i >= p.R) break;
+    pad_row_tail(p.idx_c, p.t0_c, p.t1_c, (size_t)(r0 + i) * p.Wc, min(ci, p.Wc), p.Wc, lane);
   }
+}
+
+// A ray whose coarse row, entry list or fine row is too short: walked again,
+// each coarse node descended into the row as it is met.  Returns the count.
+__device__ __noinline__ int descend_in_row(const OctTravParams &p, const OctMeta &m, long r, const float *g_vs,
+                                           const float *g_st) {
+  const TravRay y = trav_ray(p, r);
+  const float *bb = p.t.vol_bbox + 6 * y.b;
+  const float bmin[3] = {bb[0], bb[2], bb[4]};
+  int fc = 0;
+  walk_level(p, m, y, [&](int v, float p0, float p1) {
+    const int f0 = min(fc, p.Wf);
+    const size_t at = (size_t)r * p.Wf + f0;
+    Entries<1> en{p.idx + at, p.t0 + at, p.t1 + at, 0, p.Wf - f0};
+    descend<1, kTravRays>(m, p.s, y, bmin, g_vs, g_st, v, p0, p1, en);
+    fc += en.n;
+  });
+  return fc;
+}
+
+// Second pass: a warp takes four rays; their coarse nodes are laid out over
+// the lanes, a descent a lane, the entries kept in shared memory until the
+// warp's scan gives them their places in the rays' rows.
+__global__ void __launch_bounds__(kTravThreads, 6) octree_descend_kernel(const __grid_constant__ OctTravParams p, int cap) {
+  extern __shared__ int s_list[];  // [3][cap][kTravThreads]
+  __shared__ OctMeta m;
+  __shared__ float s_vs[kTravThreads / 32][SG_MAX_LEVELS * kTravRays], s_st[kTravThreads / 32][SG_MAX_LEVELS * kTravRays];
+  load_meta(p.t, m);
+  __syncthreads();
+  const int lane = lane_id(), w = threadIdx.x >> 5, s = p.s;
+  const long r0 = ((long)blockIdx.x * (kTravThreads / 32) + w) * kTravRays;
+  if (r0 >= p.R) return;
+  const int rays = (int)min((long)kTravRays, p.R - r0);
+  const int k8 = lane & (kTravRays - 1);
+  const int cc = k8 < rays ? __ldg(p.cnt_c + r0 + k8) : 0;  // lanes k, k + 4, ...: ray k
+  const int fb = (int)((r0 + min(k8, rays - 1)) / p.N);
+  int fc = 0;
+  if (__any_sync(SG_FULL, cc > 0)) {
+    const float fvs = __ldg(p.t.voxel_size + fb);
+    for (int l = lane / kTravRays; l <= s; l += 32 / kTravRays) {
+      const LevelGeom g = level_geom(fvs, m.dim[0] / m.dim[l]);
+      s_vs[w][l * kTravRays + k8] = g.vs;
+      s_st[w][l * kTravRays + k8] = g.start;
+    }
+    __syncwarp();
+    bool redo = cc > p.Wc;
+    const int n = lane < kTravRays && !redo ? cc : 0;
+    const int incl = warp_incl_scan(n), start = incl - n;
+    const int total = __shfl_sync(SG_FULL, incl, 31);
+    for (int t = 0; t < total; t += 32) {
+      const int item = t + lane;
+      int k = 0;  // the item's ray: the last whose run starts at or before it (an empty run starts where the next does)
+#pragma unroll
+      for (int q = 1; q < kTravRays; q++)
+        if (__shfl_sync(SG_FULL, start, q) <= item) k = q;
+      const int sk = __shfl_sync(SG_FULL, start, k);
+      const bool on = item < total;
+      Entries<kTravThreads> en{s_list + threadIdx.x, (float *)s_list + cap * kTravThreads + threadIdx.x,
+                               (float *)s_list + 2 * cap * kTravThreads + threadIdx.x, 0, cap};
+      if (on) {
+        const long r = r0 + k;
+        const TravRay y = trav_ray(p, r);
+        const float *bb = p.t.vol_bbox + 6 * y.b;
+        const float bmin[3] = {__ldg(bb), __ldg(bb + 2), __ldg(bb + 4)};
+        const size_t at = (size_t)r * p.Wc + (item - sk);
+        descend<kTravThreads, kTravRays>(m, s, y, bmin, s_vs[w] + k, s_st[w] + k, __ldg(p.idx_c + at), __ldg(p.t0_c + at),
+                              __ldg(p.t1_c + at), en);
+      }
+      // places: behind the ray's earlier entries
+      const int ei = warp_incl_scan(en.n), ex = ei - en.n;
+      const int at0 = __shfl_sync(SG_FULL, fc, k) + ex - __shfl_sync(SG_FULL, ex, max(sk - t, 0));
+      const unsigned over = __ballot_sync(SG_FULL, en.n > cap);
+      const int ne = min(en.n, cap);
+      for (int e = 0; e < ne; e++) {
+        const int q = at0 + e;
+        if (q < p.Wf) {
+          const size_t at = (size_t)(r0 + k) * p.Wf + q;
+          p.idx[at] = en.id[e * kTravThreads];
+          p.t0[at] = en.t0[e * kTravThreads];
+          p.t1[at] = en.t1[e * kTravThreads];
+        }
+      }
+      // lane k: ray k's items of this round are lanes [a, z)
+      const int a = max(start - t, 0), z = min(start + n - t, 32);
+      const int sa = __shfl_sync(SG_FULL, ex, a & 31), sz = __shfl_sync(SG_FULL, ei, (z - 1) & 31);
+      if (lane < kTravRays && a < z) {
+        fc += sz - sa;
+        if (over & ((z == 32 ? 0u : (1u << z)) - (1u << a))) redo = true;
+      }
+    }
+    if (lane < rays && (redo || fc > p.Wf)) fc = descend_in_row(p, m, r0 + lane, s_vs[w] + lane, s_st[w] + lane);
+    __syncwarp();
+    const int most = __reduce_max_sync(SG_FULL, lane < rays ? fc : 0);
+    if (p.st && lane == 0) {
+      if (most > 0) atomicMax(&p.st->max_fine, most);
+      if (most > p.Wf) atomicOr(&p.st->flags, SG_FLAG_HIT_OVERFLOW);
+    }
+  }
+  if (lane < rays) p.cnt[r0 + lane] = fc;
+  for (int k = 0; k < rays; k++) {
+    const int fe = min(__shfl_sync(SG_FULL, fc, k), p.Wf);
+    const size_t row = (size_t)(r0 + k) * p.Wf;
+    float vlen = 0.0f;
+    if (fe > 0) {
+      const float vs = __ldg(p.t.voxel_size + __shfl_sync(SG_FULL, fb, k)), top = s_vs[w][s * kTravRays + k];
+      for (int c = 0; c < fe; c += 32) {
+        float x = 0.0f;
+        if (c + lane < fe) {
+          const size_t at = row + c + lane;
+          x = (p.t1[at] - p.t0[at]) * (top / level_edge(m, vs, meta_level_of(m, p.idx[at])));
+        }
+        const int cn = min(32, fe - c);
+        for (int e = 0; e < cn; e++) vlen = vlen + __shfl_sync(SG_FULL, x, e);
+      }
+    }
+    if (lane == 0) p.vl[r0 + k] = vlen;
+    pad_row_tail(p.idx, p.t0, p.t1, row, fe, p.Wf, lane);
+  }
+}
+
+// Entries that a coarse node's descent is given room for: what a straight line
+// meets, at most 3 e - 2 of the e^3 cells of each level (e cells an edge), the
+// node itself, and one more where it runs along a face.
+constexpr int kMostEntries = 64;
+
+static int descent_entries(int s, int rate) {
+  long n = 2, e = 1;
+  for (int l = 0; l < s; l++) {
+    e *= rate;
+    n += 3 * e - 2;
+    if (n >= kMostEntries) return kMostEntries;
+  }
+  return (int)n;
 }
 
 // ---------------------------------------------------------------------------
@@ -483,7 +622,7 @@ struct FineParams {
 
 constexpr int kFineWarps = 4;
 
-__global__ void __launch_bounds__(kFineWarps * 32) sample_fine_kernel(FineParams p) {
+__global__ void __launch_bounds__(kFineWarps * 32) sample_fine_kernel(const __grid_constant__ FineParams p) {
   __shared__ OctMeta m;
   __shared__ int s_start[kFineWarps][33], s_id[kFineWarps][32];
   __shared__ float s_mn[kFineWarps][32], s_off[kFineWarps][32];
@@ -563,9 +702,8 @@ __global__ void __launch_bounds__(kFineWarps * 32) sample_fine_kernel(FineParams
       }
       if (bad || has >= S) break;  // with S placed the fill step never runs
     }
-    // warp arg-min of the fill candidates
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    // warp arg-min of the fill candidates (no entry, or S placed: none needed)
+    for (int o = nh > 0 && has < S ? 16 : 0; o > 0; o >>= 1) {
       const float ovs = __shfl_xor_sync(SG_FULL, bvs, o), omid = __shfl_xor_sync(SG_FULL, bmid, o);
       const float oz0 = __shfl_xor_sync(SG_FULL, bz0, o), oz1 = __shfl_xor_sync(SG_FULL, bz1, o);
       const int opos = __shfl_xor_sync(SG_FULL, bpos, o), oid = __shfl_xor_sync(SG_FULL, bid, o);
@@ -692,8 +830,14 @@ extern "C" int sg_octree_traversal(const SgOctree *tree, const float *ori, const
   const long R = (long)tree->B * N;
   OctTravParams p{*tree, ori, dir, N, tree->L - 1 - start_level, Wc, Wf, th_early_stop, opt_num,
                   idx_c, t0_c, t1_c, cnt_c, idx, t0, t1, cnt, valid_len, status, R};
-  // rows padded in the kernel
-  octree_traverse_kernel<<<ceil_div(R, kTravThreads), kTravThreads, 0, stream>>>(p);
+  octree_walk_kernel<<<ceil_div(R, kTravThreads), kTravThreads, 0, stream>>>(p);
+  const int cap = descent_entries(p.s, tree->rate);
+  const size_t smem = (size_t)3 * cap * kTravThreads * sizeof(int);
+  constexpr int kMostSmem = 3 * kMostEntries * kTravThreads * sizeof(int);
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(octree_descend_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem) != cudaSuccess)
+    return SG_ERR_CUDA;
+  octree_descend_kernel<<<ceil_div(ceil_div(R, (long)kTravRays), kTravThreads / 32), kTravThreads, smem, stream>>>(p, cap);
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
@@ -707,7 +851,7 @@ extern "C" int sg_sample_fine(const SgOctree *tree, const int *hit_idx, const fl
   const long R = (long)tree->B * N;
   FineParams p{*tree, hit_idx, hit_t0, hit_t1, valid_len, rands, N, W, S, start_level, sampled_idx, sampled_z, R};
   long g = ceil_div(R, kFineWarps);
-  if (g > (long)num_sms() * 16) g = (long)num_sms() * 16;
+  if (g > (long)num_sms() * 64) g = (long)num_sms() * 64;
   sample_fine_kernel<<<(int)g, kFineWarps * 32, 0, stream>>>(p);
   SG_LAUNCH_CHECK();
   return SG_OK;
