@@ -104,6 +104,11 @@ int sg_tune_get(int knob);
 
 /* ---- fusion ------------------------------------------------------------ */
 
+/* Colour images [n, channels >= 3, pixels] (r, g, b planes first) as the
+ * fusion's packed colours [n, pixels]: floor(b 256^2 + g 256 + r)
+ * (voxel_encoding_helper.py:213). */
+int sg_pack_colors(const float *rgb, long n, int channels, long pixels, float *out, sg_stream_t stream);
+
 /* Data-driven cubic box.  Replaces inverse_mat3x3 + obtain_origin_bbox +
  * obtain_resized_bbox as run by fusion_cuda_integrate
  * (c_lib/VoxelEncoding/src/fusion_kernel.cu:51-184, 683-708).

@@ -32,7 +32,7 @@ EXPORTS = (
     "sg_sort_pairs_scratch_bytes", "sg_sort_pairs", "sg_octree_scratch_bytes", "sg_octree_build",
     "sg_octree_nodes", "sg_octree_traversal", "sg_sample_fine", "sg_nerf_param_count", "sg_nerf_density",
     "sg_pack_fields", "sg_render_packed_fwd", "sg_render_packed_bwd", "sg_render_packed_train",
-    "sg_render_packed_train_det", "sg_channels_last",
+    "sg_render_packed_train_det", "sg_channels_last", "sg_pack_colors",
 )
 
 
@@ -119,6 +119,7 @@ def _load():
     lib.sg_composite_fwd.argtypes = [p, p, p, p, i, i, i, f, i, p, p, p, p, p]
     lib.sg_composite_bwd.argtypes = [p] * 12 + [i, i, i, f, i, i, p, p, p]
     lib.sg_sample_sorted.argtypes = [C.POINTER(SgTree), p, p, p, p, i, i, p, f, p, i, i, i, p, p, p]
+    lib.sg_pack_colors.argtypes = [p, C.c_long, i, C.c_long, p, p]
     lib.sg_grid_gather.argtypes = [p, p, p, i, i, i, p, i, i, p, p, i, f, f, p, p]
     lib.sg_grid_scatter.argtypes = [p, p, p, i, i, i, p, p, i, i, p, p, i, f, f, p, p]
     lib.sg_render_fused.argtypes = [C.POINTER(SgTree), p, p, p, p, i, i, p, f, p, i, i, i, p, p, p, i, f, f, p, i,
@@ -181,7 +182,8 @@ def ptr(t):
 
 
 def stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream (its address; no Stream object is made)."""
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def mask_words(rate):

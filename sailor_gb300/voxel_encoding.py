@@ -56,7 +56,7 @@ class _Dev:
         for t in tensors:
             if isinstance(t, torch.Tensor) and not t.is_cuda:
                 raise RuntimeError("input must be a cuda tensor")
-        self.d = torch.device("cuda", int(device)) if not isinstance(device, torch.device) else device
+        self.d = int(device) if not isinstance(device, torch.device) else device
 
     def __enter__(self):
         self.ctx = torch.cuda.device(self.d)
@@ -152,6 +152,22 @@ def integrate_in_box(occupied_vol, num_occ_voxel, cam_intr, cam_pose, color_ims,
                                    float(tsdf_th_high), N.ptr(tsdf), N.ptr(weight), N.ptr(colorv), N.ptr(occ),
                                    N.ptr(cnt), N.stream()), "fuse_tsdf")
         return tsdf, weight, colorv
+
+
+def pack_colors(colors):
+    """floor(b 256^2 + g 256 + r) of colour images [n, >= 3, h, w], [n, h, w]
+    (voxel_encoding_helper.py:213): in one pass where the images are float32
+    on the GPU, contiguous and without gradient (the seven elementwise passes
+    of the expression took 28 of a 128^3 build's 202 us of device time)."""
+    if (colors.is_cuda and colors.dtype == torch.float32 and colors.dim() == 4 and colors.shape[1] >= 3
+            and colors.is_contiguous() and colors.numel() > 0
+            and not (colors.requires_grad and torch.is_grad_enabled())):
+        n, ch, h, w = colors.shape
+        with torch.cuda.device(colors.device):
+            out = torch.empty((n, h, w), dtype=torch.float32, device=colors.device)
+            N.check(N.lib.sg_pack_colors(N.ptr(colors), n, ch, h * w, N.ptr(out), N.stream()), "pack_colors")
+        return out
+    return torch.floor(colors[:, 2] * 256.0 * 256.0 + colors[:, 1] * 256.0 + colors[:, 0])
 
 
 # --------------------------------------------------------------------------
@@ -252,9 +268,11 @@ class MultiLayerOctree:
         self.num_levels = int(num_levels)
         self.batch_size = int(batch_size)
         self.rate = int(rate)
-        self.device = torch.device("cuda", int(device))
+        self._gpu = int(device)
+        self.device = torch.device("cuda", self._gpu)
         self._tree = None
-        self._oct = None
+        self._oct = None  # multi-level tables: over two levels, made on first use
+        self._ready = False
         self._status = None  # SgStatus block, allocated by init_octree
         self._ostatus = None  # SgOctreeStatus block
         self.num_octree_nodes = 0
@@ -267,7 +285,7 @@ class MultiLayerOctree:
             raise RuntimeError(f"MultiLayerOctree: {L} levels (2 to {N.SG_MAX_LEVELS} are supported)")
         if self.rate not in (2, 4, 8):
             raise RuntimeError(f"MultiLayerOctree: rate {self.rate} (2, 4 or 8 are supported)")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             self._vols = [_inplace(v, "volume", torch.int32) for v in dense_volumes]
             self._cnts = list(num_occ_voxels_batches)
             self.num_levels = L
@@ -283,9 +301,10 @@ class MultiLayerOctree:
                     raise RuntimeError(f"volume dims {dims[l - 1]}/{dims[l]} do not match rate {self.rate}")
             dev = self.device
             i32 = dict(dtype=torch.int32, device=dev)
-            self._status = torch.zeros(4, **i32)
-            self._ostatus = torch.zeros(4, **i32)
-            self._tree = None
+            words = torch.zeros(16, **i32)  # both status blocks and the two-level counts
+            self._status, self._ostatus = words[:4], words[4:8]
+            self._tree = self._oct = None
+            self._dims = dims
             if L == 2:
                 B, Db, Dt = self.batch_size, dims[0], dims[1]
                 mw = N.mask_words(self.rate)
@@ -295,7 +314,7 @@ class MultiLayerOctree:
                     brick_mask=torch.empty(B * Dt ** 3 * mw, **i32),
                     top_key=torch.empty(cap_top, **i32), top_child_base=torch.empty(cap_top, **i32),
                     bot_key=torch.empty(cap_bot, **i32), bot_parent=torch.empty(cap_bot, **i32),
-                    counts=torch.zeros(2, **i32), brick_box=torch.empty(6 * B, **i32),
+                    counts=words[8:10], brick_box=torch.empty(6 * B, **i32),
                     scratch=torch.empty(int(N.lib.sg_tree_scratch_bytes(B, Dt)), dtype=torch.uint8, device=dev))
                 b = self._bufs
                 self._tree = N.SgTree(B, Dt, Db, self.rate, self._index[1], self._index[0], cap_top, cap_bot,
@@ -304,7 +323,16 @@ class MultiLayerOctree:
                                       b["bot_key"].data_ptr(), b["bot_parent"].data_ptr(), b["counts"].data_ptr(),
                                       self.voxel_size.data_ptr(), self.volume_bbox.data_ptr(),
                                       b["brick_box"].data_ptr())
-            # multi-level node tables: one run per level, capacity = its occupied count
+            else:
+                self._make_levels()
+            self._ready = True
+            self._oct_stale = True
+
+    def _make_levels(self):
+        """Multi-level node tables: one run per level, capacity = its occupied count."""
+        with torch.cuda.device(self._gpu):
+            L, dims, dev = self.num_levels, self._dims, self.device
+            i32 = dict(dtype=torch.int32, device=dev)
             caps = [max(c, 0) for c in self._totals]
             ob = dict(counts=torch.zeros(L, **i32))
             for name in ("key", "parent", "child_base", "nchild"):
@@ -322,12 +350,11 @@ class MultiLayerOctree:
             ob["scratch"] = torch.empty(max(int(N.lib.sg_octree_scratch_bytes(C.byref(o))), 16), dtype=torch.uint8,
                                         device=dev)
             self._oct, self._obufs = o, ob
-            self._oct_stale = True
 
     def build_octree(self):
-        if self._oct is None:
+        if not self._ready:
             raise RuntimeError("build_octree before init_octree")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             if self._tree is not None:
                 s = self._bufs["scratch"]
                 N.check(N.lib.sg_tree_build(C.byref(self._tree), N.ptr(self._vols[1]), N.ptr(self._vols[0]),
@@ -340,7 +367,7 @@ class MultiLayerOctree:
         """The multi-level node tables.  Over a two-level tree already built
         they get the same ids (the volumes hold them; occupancy is still
         value > -1) and the build writes them again."""
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             self._ostatus.zero_()
             s = self._obufs["scratch"]
             N.check(N.lib.sg_octree_build(C.byref(self._oct), N.ptr(s), s.numel(), N.ptr(self._ostatus),
@@ -348,8 +375,10 @@ class MultiLayerOctree:
         self._oct_stale = False
 
     def _levels(self):
-        if self._oct is None:
+        if not self._ready:
             raise RuntimeError("multi-level query before init_octree")
+        if self._oct is None:
+            self._make_levels()
         if getattr(self, "_oct_stale", True):
             self._build_levels()
 
@@ -364,7 +393,7 @@ class MultiLayerOctree:
         self._two_level("voxel_traversal")
         if int(start_level) != 0:
             raise RuntimeError("voxel_traversal: only start_level 0 (the top level) is supported")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             ori = _in(ray_ori, "ray_ori")
             dr = _in(ray_dir, "ray_dir")
             Nr = ori.shape[1]
@@ -385,10 +414,7 @@ class MultiLayerOctree:
     def ray_voxels_points_sampling_coarse(self, hits_idxs, min_depths, max_depths, uniform_rand_values,
                                           rays_valid_len, start_level, num_sampled):
         self._two_level("ray_voxels_points_sampling_coarse")
-        with torch.cuda.device(self.device):
-            st = self._status.tolist()  # the reference reads its max-hit counter here too
-            if st[0] & N.SG_FLAG_HIT_OVERFLOW:
-                raise RuntimeError(f"hit list overflow: a ray has {st[1]} hits, rows hold {self._last_W}")
+        with torch.cuda.device(self._gpu):
             hi = _in(hits_idxs, "hits_idxs", torch.int32)
             B, Nr, W = hi.shape
             t0 = _in(min_depths, "min_depths")
@@ -401,10 +427,15 @@ class MultiLayerOctree:
             N.check(N.lib.sg_sample_coarse(C.byref(self._tree), N.ptr(hi), N.ptr(t0), N.ptr(t1), Nr, W, N.ptr(rd),
                                            N.ptr(vl), S, self.num_levels, int(start_level), N.ptr(si), N.ptr(sz),
                                            N.stream()), "sample_coarse")
+            # the reference reads its max-hit counter here too; behind the launch, so
+            # that the GPU works while the host waits (rows are read within their width)
+            st = self._status.tolist()
+            if st[0] & N.SG_FLAG_HIT_OVERFLOW:
+                raise RuntimeError(f"hit list overflow: a ray has {st[1]} hits, rows hold {self._last_W}")
             return si, sz
 
     def sort_samplings(self, sampled_depths):
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             z = _in(sampled_depths, "sampled_depths")
             srt = torch.empty_like(z)
             idx = torch.empty(z.shape, dtype=torch.int32, device=z.device)
@@ -417,7 +448,7 @@ class MultiLayerOctree:
 
     def trilinear_aggregate_features(self, ray_ori, ray_dir, sampled_z, sampled_idx, input_feats):
         self._two_level("trilinear_aggregate_features")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             f = _in(input_feats, "input_feats")
             B, Cf, Nr, S, _ = f.shape
             out = torch.zeros((B, Cf, Nr, S), device=self.device)
@@ -430,7 +461,7 @@ class MultiLayerOctree:
     def trilinear_aggregate_features_backward(self, ray_ori, ray_dir, sampled_z, sampled_idx, input_feats,
                                               grad_output):
         self._two_level("trilinear_aggregate_features_backward")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             g = _in(grad_output, "grad_output")
             B, Cf, Nr, S = g.shape
             gin = torch.empty((B, Cf, Nr, S, 8), device=self.device)
@@ -446,11 +477,11 @@ class MultiLayerOctree:
         projected into every view: (proj_xy [B,V,N,S,9,2] or [B,V,N,S,2]
         normalised to [-1, 1], proj_z [B,V,N,S,9,1] or [B,V,N,S,1] camera z);
         -1 where the sample has no node (sampling_kernel.cu:1333-1381)."""
-        if record_corners and self._oct is None:
+        if record_corners and not self._ready:
             raise RuntimeError("project_sampled_xyz with record_corners before init_octree")
         if record_corners:
             self._two_level("project_sampled_xyz with record_corners")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             z = _in(sampled_z, "sampled_z")
             idx = _in(sampled_idx, "sampled_idx", torch.int32)
             B, Nr, S = z.shape
@@ -471,7 +502,7 @@ class MultiLayerOctree:
 
     # -- node queries -----------------------------------------------------
     def get_nodes_tensor(self):
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             out = torch.empty((self.num_octree_nodes, 6), device=self.device)
             if self._tree is not None:
                 N.check(N.lib.sg_tree_nodes(C.byref(self._tree), self.num_octree_nodes, N.ptr(out), N.stream()),
@@ -514,13 +545,13 @@ class MultiLayerOctree:
         441-643, 722-826).  Fine rows hold each coarse node's entries
         together, in descent order; the reference's atomic appends leave the
         same entries in a run-dependent order."""
-        if self._oct is None:
+        if not self._ready:
             raise RuntimeError("octree_traversal before init_octree")
         self._levels()
         start_level = int(start_level)
         if not 0 <= start_level < self.num_levels:
             raise RuntimeError(f"octree_traversal: start_level {start_level} outside [0, {self.num_levels})")
-        with torch.cuda.device(self.device):
+        with torch.cuda.device(self._gpu):
             ori = _in(ray_ori, "ray_ori")
             dr = _in(ray_dir, "ray_dir")
             Nr = ori.shape[1]
@@ -549,15 +580,10 @@ class MultiLayerOctree:
         """(sampled_idx, sampled_depths) [B,N,S] over fine rows
         (sampling_kernel.cu:911-1068, 1178-1248); unsorted, as the
         reference returns them."""
-        if self._oct is None:
+        if not self._ready:
             raise RuntimeError("ray_voxels_points_sampling before init_octree")
         self._levels()
-        with torch.cuda.device(self.device):
-            st = self._ostatus.tolist()  # the reference reads its fine max-hit counter here too
-            if st[0] & N.SG_FLAG_HIT_OVERFLOW:
-                Wc, Wf = getattr(self, "_last_fine", (0, 0))
-                raise RuntimeError(f"octree row overflow: a ray has {st[1]} coarse / {st[2]} fine entries, "
-                                   f"rows hold {Wc} / {Wf}")
+        with torch.cuda.device(self._gpu):
             hi = _in(hits_idxs, "hits_idxs", torch.int32)
             B, Nr, W = hi.shape
             t0 = _in(min_depths, "min_depths")
@@ -572,4 +598,9 @@ class MultiLayerOctree:
             N.check(N.lib.sg_sample_fine(C.byref(self._oct), N.ptr(hi), N.ptr(t0), N.ptr(t1), Nr, W, N.ptr(vl),
                                          N.ptr(rd), S, int(start_level), N.ptr(si), N.ptr(sz), N.stream()),
                     "sample_fine")
+            st = self._ostatus.tolist()  # the reference reads its fine max-hit counter here too
+            if st[0] & N.SG_FLAG_HIT_OVERFLOW:
+                Wc, Wf = getattr(self, "_last_fine", (0, 0))
+                raise RuntimeError(f"octree row overflow: a ray has {st[1]} coarse / {st[2]} fine entries, "
+                                   f"rows hold {Wc} / {Wf}")
             return si, sz

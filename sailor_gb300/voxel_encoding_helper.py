@@ -183,7 +183,7 @@ class _integrate_depths(nn.Module):
         colors, depths, masks, Ks, RTs = inputs_data
         h, w = depths.shape[-2:]
         num_views = depths.shape[0] // batch_size
-        colors = torch.floor(colors[:, 2] * 256.0 * 256.0 + colors[:, 1] * 256.0 + colors[:, 0])
+        colors = VoxelEncoding.pack_colors(colors)
         if len(depths.shape) == 4:
             depths = depths[:, 0]
         if len(masks.shape) == 4:
@@ -228,6 +228,17 @@ class _integrate_depths(nn.Module):
 integrate_depths = _integrate_depths()
 
 
+def _totals(counts):
+    """The sum of each tensor of counts, read back in one copy where they allow it."""
+    if counts and len({(c.device, c.dtype) for c in counts}) == 1 and counts[0].dtype in (torch.int32, torch.int64):
+        flat, at, out = torch.cat([c.reshape(-1) for c in counts]).tolist(), 0, []
+        for c in counts:
+            out.append(sum(flat[at:at + c.numel()]))
+            at += c.numel()
+        return out
+    return [int(torch.sum(c)) for c in counts]
+
+
 # voxel_encoding_helper.py:535-662
 class OcTreeOptions(nn.Module):
 
@@ -244,10 +255,8 @@ class OcTreeOptions(nn.Module):
     def _init_octree(self, _occupied_volumes, _num_occ_voxels, _voxel_size, _vol_bbox):
         self._vol_dim = _occupied_volumes[0].shape[-3:]
         assert len(_occupied_volumes) == self._levels and len(_num_occ_voxels) == self._levels
-        totals, index = [], []
-        for i, nv in enumerate(_num_occ_voxels):
-            totals.append(int(torch.sum(nv)))
-            index.append(sum(totals[:i]))
+        totals = _totals(_num_occ_voxels)
+        index = [sum(totals[:i]) for i in range(len(totals))]
         self._octree.init_octree(_occupied_volumes, totals, _num_occ_voxels, index, _voxel_size, _vol_bbox)
         self._octree.build_octree()
         return totals, index
