@@ -714,7 +714,7 @@ int sg_render_segments_train(const SgTree *tree, const SgRaySegments *seg,
  * begins with SG_DET_COUNTERS ints: [SG_DET_RAYS_WITH_HITS] the rays with
  * hits, [SG_DET_SLOTS_NEEDED] the record slots they need, [SG_DET_SLOTS]
  * the slots used (at most `capacity`), [SG_DET_CELLS] the distinct cells
- * summed, [SG_DET_RECORDS] the records with a cell. */
+ * summed, [SG_DET_RECORDS] the records (runs of a ray's samples in a cell). */
 #define SG_DET_COUNTERS 8
 enum { SG_DET_RAYS_WITH_HITS = 0, SG_DET_SLOTS_NEEDED = 1, SG_DET_SLOTS = 2, SG_DET_CELLS = 3, SG_DET_RECORDS = 4 };
 size_t sg_train_det_workspace_bytes(long long R, int nseg, int C, long long capacity);
@@ -723,9 +723,10 @@ size_t sg_train_det_workspace_bytes(long long R, int nseg, int C, long long capa
  * with grid gradients that are bit-identical from run to run: a segmented
  * reduction over sorted cell ids instead of float atomics.  The pass visits
  * only the rays with hits (a scan builds their list; the others get their
- * outputs directly) and writes one record per used sample -- trilinear cell,
- * cell fractions, compositing weight, ray, TSDF gradient -- plus, per ray,
- * head^T times its colour gradient; the records are sorted by cell (a
+ * outputs directly) and writes one record per run of a ray's samples in one
+ * trilinear cell -- the cell, and per corner the sum of corner weight x
+ * compositing weight (and x TSDF gradient) -- plus, per ray, head^T times its
+ * colour gradient; the records are sorted by cell (a
  * stable radix sort), and each cell's run is summed in order and added to
  * its 8 corners, one parity class of cells at a time (cells of a class
  * share no corner).  The sums are added (+=) into grad_feat [B,Df,Df,Df,C]

@@ -425,7 +425,7 @@ class BatchPipeline:
 
     def reduction_sizes(self):
         """Sizes of the last deterministic gradient reduction (synchronizes):
-        rays with hits, record slots needed and used, records with a cell,
+        rays with hits, record slots needed and used, records (runs of a ray's samples in a cell),
         distinct cells summed."""
         if self.det_ws is None:
             raise RuntimeError("the pipeline reduces gradients with atomics (deterministic=False)")

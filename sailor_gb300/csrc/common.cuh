@@ -148,6 +148,20 @@ __device__ __forceinline__ float sum3_rn(float a, float b, float c) {
   return __fadd_rn(th, v);
 }
 
+// Division by a fixed d >= 1: q = (mulhi(n, m) + n) >> s for 0 <= n < 2^31
+// (T. Granlund, P. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994).
+struct FixedDiv31 {
+  uint32_t m, s;
+  static FixedDiv31 of(uint32_t d) {
+    FixedDiv31 f{0u, 0u};
+    while ((1ull << f.s) < d) f.s++;
+    f.m = (uint32_t)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
+    return f;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
+};
+
 // ---------------------------------------------------------------------------
 // warp helpers
 // ---------------------------------------------------------------------------

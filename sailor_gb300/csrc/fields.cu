@@ -39,21 +39,14 @@
 
 namespace sg {
 
-// Division by a fixed d >= 1: q = (mulhi(n, m) + n) >> s for 0 <= n < 2^31
-// (T. Granlund, P. Montgomery, "Division by invariant integers using
-// multiplication", PLDI 1994), the plain 64-bit quotient above that.
+// Division by a fixed d >= 1, the plain 64-bit quotient where a dividend can
+// reach 2^31.
 struct FixedDiv {
-  uint32_t d, m, s;
+  FixedDiv31 q;
+  uint32_t d;
   int small;  // every dividend is below 2^31
-  static FixedDiv of(uint32_t d, long largest) {
-    FixedDiv f{d, 0u, 0u, largest < (1l << 31) ? 1 : 0};
-    while ((1ull << f.s) < d) f.s++;
-    f.m = (uint32_t)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
-    return f;
-  }
-  __device__ __forceinline__ long div(long n) const {
-    return small ? (long)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s) : n / (long)d;
-  }
+  static FixedDiv of(uint32_t d, long largest) { return FixedDiv{FixedDiv31::of(d), d, largest < (1l << 31) ? 1 : 0}; }
+  __device__ __forceinline__ long div(long n) const { return small ? (long)q.div((uint32_t)n) : n / (long)d; }
 };
 
 struct GatherParams {
@@ -82,18 +75,6 @@ struct FrameGeom {
     inv_vs = 1.0f / vs;
   }
 };
-
-// The 8 corners of a cell that lie in the grid, bit cr = (dx, dy, dz) of bits (2, 1, 0).
-__device__ __forceinline__ unsigned corners_inside(const int (&i0)[3], int D) {
-  unsigned m = 0xffu;
-  if (i0[0] < 0 || i0[0] >= D) m &= 0xf0u;
-  if (i0[0] + 1 < 0 || i0[0] + 1 >= D) m &= 0x0fu;
-  if (i0[1] < 0 || i0[1] >= D) m &= 0xccu;
-  if (i0[1] + 1 < 0 || i0[1] + 1 >= D) m &= 0x33u;
-  if (i0[2] < 0 || i0[2] >= D) m &= 0xaau;
-  if (i0[2] + 1 < 0 || i0[2] + 1 >= D) m &= 0x55u;
-  return m;
-}
 
 // VEC: grid and output are 16-byte aligned (C a multiple of 4).
 template <int C, bool VEC>

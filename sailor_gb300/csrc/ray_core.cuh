@@ -504,6 +504,18 @@ __device__ __forceinline__ void tap_cell(const float bmin[3], float vs, float in
   for (int cr = 0; cr < 8; cr++) w[cr] = corner_weight(f, cr);
 }
 
+// The 8 corners of a cell that lie in the grid, bit cr = (dx, dy, dz) of bits (2, 1, 0).
+__device__ __forceinline__ unsigned corners_inside(const int (&i0)[3], int D) {
+  unsigned m = 0xffu;
+  if (i0[0] < 0 || i0[0] >= D) m &= 0xf0u;
+  if (i0[0] + 1 < 0 || i0[0] + 1 >= D) m &= 0x0fu;
+  if (i0[1] < 0 || i0[1] >= D) m &= 0xccu;
+  if (i0[1] + 1 < 0 || i0[1] + 1 >= D) m &= 0x33u;
+  if (i0[2] < 0 || i0[2] >= D) m &= 0xaau;
+  if (i0[2] + 1 < 0 || i0[2] + 1 >= D) m &= 0x55u;
+  return m;
+}
+
 __device__ __forceinline__ bool corner_inside(const int (&i0)[3], int cr, int D, size_t &off) {
   const int ix = i0[0] + ((cr >> 2) & 1), iy = i0[1] + ((cr >> 1) & 1), iz = i0[2] + (cr & 1);
   if (ix < 0 || iy < 0 || iz < 0 || ix >= D || iy >= D || iz >= D) return false;

@@ -92,13 +92,13 @@ struct RenderParams {
   float *out_loss;
   // gradient records instead of the scatter (deterministic reduction,
   // scatter.cu): the launch's rays are hit_ray[k], k in [*k_begin, *k_end);
-  // ray k's used samples, in sorted position order, go to record slots
+  // ray k's records, in sorted position order, go to record slots
   // hit_slot[k], hit_slot[k] + 1, ... (below rec_cap), their count to
   // ray_nrec[k]
   const int *hit_ray, *hit_slot, *k_begin, *k_end;
   int *ray_nrec;
   uint32_t *rec_key;
-  GradRecord *rec;
+  GradRecord *rec, *rec_t;
   float *ray_g;  // [k][C]: head^T (colour gradient of ray k)
   long rec_cap;
   RecordKeys keys;
@@ -598,23 +598,59 @@ __device__ __forceinline__ float head_grad(const RenderParams &p, int c, const f
   return c == 0 ? gc[0] : (c == 1 ? gc[1] : (c == 2 ? gc[2] : 0.0f));
 }
 
-// Record of this lane's sample for the deterministic reduction: its cell (the
-// key), its cell fractions and compositing weight, the ray's compact index k
-// and its TSDF gradient.  The records of a ray's samples with a cell are
-// packed, in sorted position order, from slot base on (n: those written by
-// the blocks before; updated).
-__device__ __forceinline__ void emit_record(const RenderParams &p, long k, int b, long base, bool used,
-                                            const int (&i0)[3], const float (&f)[3], float w, float gt, int &n) {
+// Records of a block's samples for the deterministic reduction, one for each
+// run of samples of consecutive positions in one cell: the cell (the key) and,
+// at the run's first lane, the sums of corner weight x compositing weight (and
+// x TSDF gradient) over the run.  The records of a ray are packed, in sorted
+// position order, from slot base on (n: those written by the blocks before;
+// updated).  A record per sample made 2.1 to 2.3 times as many to write, sort
+// and sum.
+template <bool TSDF>
+__device__ __forceinline__ void emit_records(const RenderParams &p, int b, long base, bool used, const int (&i0)[3],
+                                             const float (&f)[3], float w, float gt, int &n) {
+  const int lane = lane_id();
   const uint32_t key = used ? record_key(p.keys, b, i0) : p.keys.invalid;
   const bool has = key != p.keys.invalid;
   const unsigned m = __ballot_sync(SG_FULL, has);
-  const long slot = base + n + __popc(m & ((1u << lane_id()) - 1u));
-  if (has && slot < p.rec_cap) {
-    p.rec[slot].fw = make_float4(f[0], f[1], f[2], w);
-    p.rec[slot].kt = make_int4((int)k, __float_as_int(gt), 0, 0);
+  if (m == 0u) return;
+  const uint32_t before = __shfl_up_sync(SG_FULL, key, 1);
+  const bool head = has && (lane == 0 || before != key);
+  const unsigned heads = __ballot_sync(SG_FULL, head);
+  const unsigned stops = (heads | ~m) & ~((2u << lane) - 1u);  // lanes behind this one that are not of its run
+  const int stop = stops ? __ffs(stops) - 1 : 32;
+  float a[8], t[TSDF ? 8 : 1];
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const float cw = corner_weight(f, c);
+    a[c] = has ? cw * w : 0.0f;
+    if (TSDF) t[c] = has ? cw * gt : 0.0f;
+  }
+#pragma unroll 1
+  for (int o = 1; __any_sync(SG_FULL, has && lane + o < stop); o <<= 1) {
+    const bool in = lane + o < stop;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const float x = __shfl_down_sync(SG_FULL, a[c], o);
+      if (in) a[c] += x;
+      if (TSDF) {
+        const float y = __shfl_down_sync(SG_FULL, t[c], o);
+        if (in) t[c] += y;
+      }
+    }
+  }
+  const long slot = base + n + __popc(heads & ((1u << lane) - 1u));
+  if (head && slot < p.rec_cap) {
+    float4 *r = reinterpret_cast<float4 *>(p.rec + slot);
+    r[0] = make_float4(a[0], a[1], a[2], a[3]);
+    r[1] = make_float4(a[4], a[5], a[6], a[7]);
+    if (TSDF) {
+      float4 *q = reinterpret_cast<float4 *>(p.rec_t + slot);
+      q[0] = make_float4(t[0], t[1], t[2], t[3]);
+      q[1] = make_float4(t[4], t[5], t[6], t[7]);
+    }
     p.rec_key[slot] = key;
   }
-  n += __popc(m);
+  n += __popc(heads);
 }
 
 // MODE kModeBwd: the adjoint for given upstream gradients.  The training
@@ -623,7 +659,7 @@ __device__ __forceinline__ void emit_record(const RenderParams &p, long k, int b
 // loss_scale * (rgb - target)); the outputs and per-ray loss are written, and
 // nothing is recomputed.  kModeTrain scatters with atomics; in the record
 // modes the rays are the compact list of rays with hits and the grid
-// gradients leave the kernel as per-sample records (emit_record) for the
+// gradients leave the kernel as records (emit_records) for the
 // deterministic reduction (scatter.cu).  Without the TSDF's gradient
 // (kModeRec) a record needs nothing that comes after its sample, so it is
 // written as soon as the sample's weight is known and no adjoint runs.
@@ -711,7 +747,7 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
         cw += warp_sum_scan_order(v.w);
         ca += warp_sum_scan_order(v.w * v.al);
       }
-      if (MODE == kModeRec) emit_record(p, it, b, base, v.used, v.i0, v.f, v.w, 0.0f, nrec);
+      if (MODE == kModeRec) emit_records<false>(p, b, base, v.used, v.i0, v.f, v.w, 0.0f, nrec);
     }
     float gc[3] = {0.0f, 0.0f, 0.0f}, gd = 0.0f, gws = 0.0f, ga = 0.0f;
     if (TRAIN) {
@@ -801,7 +837,7 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
           int i0[3] = {0, 0, 0};
           float f[3] = {0.0f, 0.0f, 0.0f};
           if (used) feat_cell(p, g, z, i0, f);
-          emit_record(p, it, b, base, used, i0, f, w, gt, nrec);
+          emit_records<true>(p, b, base, used, i0, f, w, gt, nrec);
         } else if (p.grad_feat || p.grad_tsdf) {
           // scatter into the grids, samples in sorted order
           int i0[3] = {0, 0, 0};
@@ -1183,6 +1219,7 @@ extern "C" int sg_render_packed_train_det(const SgTree *tree, const SgRaySegment
   p.ray_nrec = w.ray_nrec;
   p.rec_key = w.rec_key;
   p.rec = w.rec;
+  p.rec_t = w.rec_t;
   p.ray_g = w.ray_g;
   p.rec_cap = (long)capacity;
   p.keys = make_record_keys(tree->B, args->Df);
@@ -1196,7 +1233,7 @@ extern "C" int sg_render_packed_train_det(const SgTree *tree, const SgRaySegment
     rc = launch_render_c(pg, args->C, kModeRec, stream);
     if (rc != SG_OK) return rc;
   }
-  return launch_det_reduce(w, p.keys, R, (long)capacity, args->C, grad_feat, grad_tsdf, stream);
+  return launch_det_reduce(w, p.keys, *seg, args->S, R, (long)capacity, args->C, grad_feat, grad_tsdf, stream);
 }
 
 extern "C" int sg_render_segments_train_det(const SgTree *tree, const SgRaySegments *seg, const SgRenderArgs *args,

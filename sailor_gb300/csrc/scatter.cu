@@ -4,25 +4,24 @@
 // The in-kernel scatter of the render backward adds each cell run's
 // gradient into the grids with float atomics, so the summation order -- and
 // the last bits of the gradient -- change from run to run.  Here the
-// training pass (render.cu, record mode) writes one record per used sample
-// instead: the sample's trilinear cell as a 32-bit key (frame and lower
-// corner, grouped by parity class), and a 32-byte record of its cell
-// fractions, its compositing weight, its ray and its TSDF gradient; the
-// ray's colour-head factor of the feature gradient goes to a per-ray table.
+// training pass (render.cu, record mode) writes one record per run of a ray's
+// samples in one trilinear cell instead: the cell as a 32-bit key (frame and
+// lower corner, grouped by parity class), and a 32-byte record of the 8
+// corners' sums of corner weight x compositing weight (with the TSDF's gradient,
+// a second one of its sums); the ray's colour-head factor of the feature
+// gradient goes to a per-ray table.
 // The pass packs each ray's records at the front of the ray's slots and
 // writes their count.  Then
 //   1. the records are compacted (slot order kept: a scan over the rays'
 //      record counts, a warp per ray moving its keys) and their
 //      keys sorted, stably, with the record slots as values (segsort.cu):
 //      records of one cell become one run, in slot order (ray order, then
-//      sorted sample order -- fixed by the ray layout); the records are
-//      gathered into that order;
+//      sorted sample order -- fixed by the ray layout);
 //   2. run heads are flagged and scanned into the list of distinct cells;
-//   3. for each of the 8 parity classes in turn, one warp per cell sums its
-//      run in order into the 8 corners x C channels it touches (lane = corner
-//      x 4 channels) and adds the sums into the grids.  Cells of one class
-//      share no corner, so every grid value is updated by one warp per
-//      class, classes in a fixed order.
+//   3. for each of the 8 parity classes in turn, each cell's run is summed in
+//      a fixed order into the 8 corners x C channels it touches, and the sums
+//      are added into the grids.  Cells of one class share no corner, so every
+//      grid value gets one addition per class, classes in a fixed order.
 // Every grid value is therefore the same sum in the same order on every run:
 // the gradients are bit-identical across runs, launch shapes and graph
 // replays.
@@ -78,13 +77,15 @@ __global__ void det_ray_emit_kernel(long R, const int *__restrict__ hit_count, c
   }
 }
 
-// compact index of each segment's first ray; slots used (clamped to the
-// capacity) and the capacity flag
-__global__ void det_seg_kernel(SgRaySegments seg, long R, const int *__restrict__ hitb, int *__restrict__ cnt,
-                               int *__restrict__ seg_hit, long cap, SgStatus *st) {
+// compact index and slot of each segment's first ray with hits; slots used
+// (clamped to the capacity) and the capacity flag
+__global__ void det_seg_kernel(SgRaySegments seg, long R, const int *__restrict__ hitb, const int *__restrict__ slotb,
+                               int *__restrict__ cnt, int *__restrict__ seg_hit, int *__restrict__ seg_slot, long cap,
+                               SgStatus *st) {
   for (int s = threadIdx.x; s <= seg.count; s += blockDim.x) {
     const long rb = __ldg(seg.ray_begin + s);
     seg_hit[s] = rb < R ? hitb[rb] : cnt[kDetHits];
+    seg_slot[s] = rb < R ? slotb[rb] : cnt[kDetSlotsNeeded];
   }
   if (threadIdx.x == 0) {
     const int need = cnt[kDetSlotsNeeded];
@@ -123,10 +124,11 @@ __global__ void det_heads_kernel(const uint32_t *__restrict__ key, const int *__
     head[j] = (j == 0 || __ldg(key + j - 1) != __ldg(key + j)) ? 1 : 0;
 }
 
-// distinct cells: key and first sorted position; the end of the last run
+// distinct cells: key, first sorted position; the end of the last run; the
+// first cell of each parity class (bound[8]: the end of the last class)
 __global__ void det_unique_kernel(const uint32_t *__restrict__ key, const int *__restrict__ head_scan,
-                                  const int *__restrict__ cnt, uint32_t *__restrict__ ukey,
-                                  int *__restrict__ ustart) {
+                                  const int *__restrict__ cnt, uint32_t cls,
+                                  uint32_t *__restrict__ ukey, int *__restrict__ ustart, int *__restrict__ bound) {
   const long n = cnt[kDetValid];
   const int nu = cnt[kDetCells];
   for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (long)gridDim.x * blockDim.x) {
@@ -135,198 +137,195 @@ __global__ void det_unique_kernel(const uint32_t *__restrict__ key, const int *_
       const int u = head_scan[j];
       ukey[u] = k;
       ustart[u] = (int)j;
+      const int c = (int)(k / cls);
+      for (int q = j == 0 ? 0 : (int)(__ldg(key + j - 1) / cls) + 1; q <= c; q++) bound[q] = u;
     }
-    if (j + 1 == n) ustart[nu] = (int)n;
-  }
-}
-
-// the records in sorted key order (one gathered 32-byte sector per record);
-// kGatherItems records a thread per step, their loads in flight together
-constexpr int kGatherItems = 4;
-__global__ void det_gather_kernel(const uint32_t *__restrict__ sorted_slot, const int *__restrict__ cnt,
-                                  const GradRecord *__restrict__ rec, GradRecord *__restrict__ pay) {
-  const long n = cnt[kDetValid];
-  const long stride = (long)gridDim.x * blockDim.x;
-  for (long j0 = (long)blockIdx.x * blockDim.x + threadIdx.x; j0 < n; j0 += stride * kGatherItems) {
-    uint32_t slot[kGatherItems];
-    float4 fw[kGatherItems];
-    int4 kt[kGatherItems];
-#pragma unroll
-    for (int q = 0; q < kGatherItems; q++) {
-      const long j = j0 + q * stride;
-      slot[q] = j < n ? __ldg(sorted_slot + j) : 0u;
-    }
-#pragma unroll
-    for (int q = 0; q < kGatherItems; q++) {
-      if (j0 + q * stride < n) {
-        fw[q] = __ldg(&rec[slot[q]].fw);
-        kt[q] = __ldg(&rec[slot[q]].kt);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kGatherItems; q++) {
-      const long j = j0 + q * stride;
-      if (j < n) {
-        pay[j].fw = fw[q];
-        pay[j].kt = kt[q];
-      }
+    if (j + 1 == n) {
+      ustart[nu] = (int)n;
+      for (int q = (int)(k / cls) + 1; q <= 8; q++) bound[q] = nu;
     }
   }
 }
 
-__device__ __forceinline__ int lower_bound_u32(const uint32_t *a, int n, uint32_t v) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(a + mid) < v) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// Cells of parity class cls: warp per cell, its run summed in order, the
-// sums added into the 8 corner voxels of the feature grid (and TSDF grid).
-// TSDF: the TSDF gradient is reduced too (q.grad_tsdf set); without it the
-// kernel holds no TSDF staging, which leaves more of the SM's L1 to the G rows
+// Cells of parity class cls.  A warp takes a stretch of the class's sorted
+// records, cut at cell boundaries (the cells that start in the stretch), and
+// walks it 16 records at a time: lanes 2 i and 2 i + 1 hold record i's two
+// halves (its slot is loaded two steps, the record itself one step ahead), and
+// shuffles hand it to the eight lanes that sum it.  Eight lanes sum records i =
+// 0, 1, 2, 3 mod 4 each; C == 16: lane = (x corner, four channels), 4 corners x
+// 4 channels of sums in registers; C == 3: lane = corner.  At the end of a cell
+// the four partial sums meet by exchanging halves, a lane ends with one corner's
+// four channels and adds them by a reduction: a voxel gets one addition per
+// class, so their order cannot show.
+//
+// A warp per cell staged up to 32 per-sample records of its run through shared
+// memory (12 or fewer of the lanes in use at mean run lengths of 6 to 12),
+// after a pass that gathered the records into sorted order, and every CTA began
+// with a binary search for the class's cells: 26.7 M samples in 12.7 M runs,
+// 2.2 M cells of 4 x 256^3: 1.99 -> 1.01 ms for gather and classes; 2.2 M samples
+// in 0.9 M runs, 0.36 M cells: 402 -> 162 us.
 template <int C, bool TSDF>
-__global__ void __launch_bounds__(256, 4) det_class_kernel(DetReduceParams q, int cls) {
-  // per warp: the current chunk of up to 32 records of a run -- per record
-  // its 8 corner weights times its compositing weight (s_a), its 8 corner
-  // weights (s_cw, for the TSDF gradient), its TSDF gradient (s_t) and its
-  // ray's G row (s_g) -- staged by all lanes at once (lane j: record j) and
-  // read back in run order
-  __shared__ __align__(16) float4 s_g[8][32][4];
-  __shared__ __align__(16) float s_a[8][32][8];
-  __shared__ __align__(16) float s_cw[TSDF ? 8 : 1][32][8];
-  __shared__ float s_t[TSDF ? 8 : 1][32];
-  __shared__ int s_rng[2];
-  const int nu = q.cnt[kDetCells];
-  if (threadIdx.x == 0) {
-    s_rng[0] = lower_bound_u32(q.ukey, nu, (uint32_t)cls * q.keys.cls);
-    s_rng[1] = lower_bound_u32(q.ukey, nu, (uint32_t)(cls + 1) * q.keys.cls);
-  }
-  __syncthreads();
-  const int lo = s_rng[0], hi = s_rng[1];
-  const int lane = lane_id(), w8 = threadIdx.x >> 5;
-  // lane -> (corner, channels): C == 16: corner lane / 4, channels 4 (lane % 4)..+3;
-  // C == 3: lanes < 24, corner lane / 3, channel lane % 3.  TSDF: corner = lane (< 8).
-  const int cr = C == 16 ? (lane >> 2) : (lane < 24 ? lane / 3 : 0);
-  const int ch = C == 16 ? 4 * (lane & 3) : (lane < 24 ? lane % 3 : 0);
-  const bool fown = C == 16 || lane < 24;
-  const long D = q.keys.D;
-  const long wstride = ((long)gridDim.x * blockDim.x) >> 5;
-  long u = lo + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  // the cell's run bounds and key, and its first 32 records, are loaded one
-  // cell ahead: while a cell is summed, the next one's loads are in flight
-  int j0 = 0, j1 = 0;
-  uint32_t ckey = 0;
-  if (u < hi) {
-    j0 = __ldg(q.ustart + u);
-    j1 = __ldg(q.ustart + u + 1);
-    ckey = __ldg(q.ukey + u);
-  }
-  float4 pf_fw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  int4 pf_kt = make_int4(0, 0, 0, 0);
-  if (u < hi && j0 + lane < j1) {
-    pf_fw = __ldg(&q.pay[j0 + lane].fw);
-    pf_kt = __ldg(&q.pay[j0 + lane].kt);
-  }
-  for (; u < hi; u += wstride) {
-    const long un = u + wstride;
-    int nj0 = 0, nj1 = 0;
-    uint32_t nkey = 0;
-    if (un < hi) {
-      nj0 = __ldg(q.ustart + un);
-      nj1 = __ldg(q.ustart + un + 1);
-      nkey = __ldg(q.ukey + un);
+__global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, int cls) {
+  constexpr int NC = C == 16 ? 4 : 1, NV = C == 16 ? 4 : 3;  // a lane's corners, channels
+  if (q.cnt[kDetCells] == 0) return;
+  const int lo = q.bound[cls], hi = q.bound[cls + 1];
+  if (lo == hi) return;
+  const int lane = lane_id(), g = lane >> 3, l8 = lane & 7;
+  const int h = l8 >> 2, ch = C == 16 ? 4 * (l8 & 3) : 0;  // x corner, first channel
+  // the corner a lane adds at the end of a cell (C == 16), as bit and voxel offset
+  const int D = q.keys.D, cr1 = C == 16 ? 4 * h + g : l8;
+  const int at1 = ((cr1 >> 2) * D + ((cr1 >> 1) & 1)) * D + (cr1 & 1);
+  // (a stretch's position may pass 2^31, no record's does)
+  const long P0 = q.ustart[lo], P1 = q.ustart[hi];
+  const long warps = (long)gridDim.x * (blockDim.x >> 5);
+  const long Q = max((P1 - P0 + warps - 1) / warps, 32l);
+  const long pa = P0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Q;
+  if (pa >= P1) return;
+  int u = __ldg(q.heads + pa);
+  const int ub = pa + Q < P1 ? __ldg(q.heads + pa + Q) : hi;
+  if (u >= ub) return;
+  uint32_t j = __ldg(q.ustart + u);
+  const uint32_t end = __ldg(q.ustart + ub);
+  // 32 cells at a time, one a lane: lower corner's voxel, corners inside, end
+  int cvox = 0, cin = 0, cend = 0, ci = 0;
+  auto load_cells = [&]() {
+    if (u + lane < ub) {
+      const uint32_t m = __ldg(q.ukey + u + lane) - (uint32_t)cls * q.keys.cls, e = (uint32_t)D + 1;
+      cend = __ldg(q.ustart + u + lane + 1);
+      const uint32_t xy = q.by_edge.div(m), x = q.by_edge.div(xy), b = q.by_edge.div(x);
+      const int i0[3] = {(int)(x - b * e) - 1, (int)(xy - x * e) - 1, (int)(m - xy * e) - 1};
+      cvox = (((int)b * D + i0[0]) * D + i0[1]) * D + i0[2];
+      cin = (int)corners_inside(i0, D);
     }
-    // the cell's corner values are read before its run is summed, so the
-    // read of the grid overlaps the run
-    int b, i0[3];
-    record_cell(q.keys, ckey, b, i0);
-    const int vx = i0[0] + ((cr >> 2) & 1), vy = i0[1] + ((cr >> 1) & 1), vz = i0[2] + (cr & 1);
-    const bool fin = fown && vx >= 0 && vy >= 0 && vz >= 0 && vx < D && vy < D && vz < D;
-    float *gp = fin ? q.grad_feat + ((((size_t)b * D + vx) * D + vy) * D + vz) * C + ch : nullptr;
-    float4 old = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (fin) {
-      if (C == 16) old = *reinterpret_cast<const float4 *>(gp);
-      else old.x = *gp;
-    }
-    const int tx = i0[0] + ((lane >> 2) & 1), ty = i0[1] + ((lane >> 1) & 1), tz = i0[2] + (lane & 1);
-    const bool tin = TSDF && lane < 8 && tx >= 0 && ty >= 0 && tz >= 0 && tx < D && ty < D && tz < D;
-    float *tp = tin ? q.grad_tsdf + (((size_t)b * D + tx) * D + ty) * D + tz : nullptr;
-    const float told = tin ? *tp : 0.0f;
-    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float acct = 0.0f;
-    for (int c0 = j0; c0 < j1; c0 += 32) {
-      // lane jj stages the run's record c0 + jj (sorted: one coalesced load)
-      // and its ray's G row; then the samples are summed in run order
-      if (c0 + lane < j1) {
-        float4 fw;
-        int4 kt;
-        if (c0 == j0) {
-          fw = pf_fw;
-          kt = pf_kt;
-        } else {
-          fw = __ldg(&q.pay[c0 + lane].fw);
-          kt = __ldg(&q.pay[c0 + lane].kt);
-        }
-        const float *g = q.ray_g + (size_t)kt.x * C;
-        if (C == 16) {
+    ci = 0;
+  };
+  load_cells();
+  uint32_t ce = __shfl_sync(SG_FULL, cend, 0);
+  float acc[NC][NV], acct[TSDF ? NC : 1];
 #pragma unroll
-          for (int v = 0; v < 4; v++) s_g[w8][lane][v] = __ldg(reinterpret_cast<const float4 *>(g) + v);
-        } else {
-          s_g[w8][lane][0] = make_float4(__ldg(g), __ldg(g + 1), __ldg(g + 2), 0.0f);
-        }
-        const float f[3] = {fw.x, fw.y, fw.z};
-        float cw[8], a[8];
+  for (int c = 0; c < NC; c++) {
+    if (TSDF) acct[c] = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-          cw[c] = corner_weight(f, c);
-          a[c] = cw[c] * fw.w;
-        }
-        reinterpret_cast<float4 *>(s_a[w8][lane])[0] = make_float4(a[0], a[1], a[2], a[3]);
-        reinterpret_cast<float4 *>(s_a[w8][lane])[1] = make_float4(a[4], a[5], a[6], a[7]);
-        if (TSDF) {
-          reinterpret_cast<float4 *>(s_cw[w8][lane])[0] = make_float4(cw[0], cw[1], cw[2], cw[3]);
-          reinterpret_cast<float4 *>(s_cw[w8][lane])[1] = make_float4(cw[4], cw[5], cw[6], cw[7]);
-          s_t[w8][lane] = __int_as_float(kt.y);
-        }
+    for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
+  }
+  const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  auto half = [&](const GradRecord *rec, uint32_t slot) {
+    return __ldg(reinterpret_cast<const float4 *>(rec + slot) + (lane & 1));
+  };
+  const uint32_t i2 = lane >> 1;
+  float4 fa = zero4, ft = zero4;
+  uint32_t nslot = 0;
+  int k = 0, nk = 0;
+  if (j + i2 < end) {
+    const uint32_t slot = __ldg(q.slot + j + i2);
+    fa = half(q.rec, slot);
+    if (TSDF) ft = half(q.rec_t, slot);
+    k = q.rays.ray(slot);
+  }
+  if (j + 16 + i2 < end) nslot = __ldg(q.slot + j + 16 + i2);
+  for (; j < end; j += 16) {
+    float gv[4][NV];  // the rays' G rows
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const float *row = q.ray_g + (size_t)__shfl_sync(SG_FULL, k, 2 * (4 * t + g)) * C + ch;
+      if (C == 16) {
+        const float4 x = __ldg(reinterpret_cast<const float4 *>(row));
+        gv[t][0] = x.x, gv[t][1] = x.y, gv[t][2] = x.z, gv[t][NV - 1] = x.w;
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; v++) gv[t][v] = __ldg(row + v);
       }
-      if (c0 == j0 && un < hi && nj0 + lane < nj1) {
-        // the next cell's first records
-        pf_fw = __ldg(&q.pay[nj0 + lane].fw);
-        pf_kt = __ldg(&q.pay[nj0 + lane].kt);
-      }
-      __syncwarp();
-      const int m = min(32, j1 - c0);
-#pragma unroll 4
-      for (int jj = 0; jj < m; jj++) {
-        const float a = s_a[w8][jj][cr];
-        if (C == 16) {
-          const float4 g = s_g[w8][jj][lane & 3];
-          acc.x = __fmaf_rn(a, g.x, acc.x);
-          acc.y = __fmaf_rn(a, g.y, acc.y);
-          acc.z = __fmaf_rn(a, g.z, acc.z);
-          acc.w = __fmaf_rn(a, g.w, acc.w);
-        } else if (fown) {
-          const float4 g = s_g[w8][jj][0];
-          acc.x = __fmaf_rn(a, ch == 0 ? g.x : (ch == 1 ? g.y : g.z), acc.x);
-        }
-        if (TSDF && lane < 8) acct = __fmaf_rn(s_cw[w8][jj][lane], s_t[w8][jj], acct);
-      }
-      __syncwarp();
     }
-    if (fin) {
-      if (C == 16)
-        *reinterpret_cast<float4 *>(gp) = make_float4(old.x + acc.x, old.y + acc.y, old.z + acc.z, old.w + acc.w);
-      else
-        *gp = old.x + acc.x;
+    float4 nfa = zero4, nft = zero4;
+    if (j + 16 + i2 < end) {
+      nfa = half(q.rec, nslot);
+      if (TSDF) nft = half(q.rec_t, nslot);
+      nk = q.rays.ray(nslot);
     }
-    if (tin) *tp = told + acct;
-    j0 = nj0;
-    j1 = nj1;
-    ckey = nkey;
+    if (j + 32 + i2 < end) nslot = __ldg(q.slot + j + 32 + i2);
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const int src = 2 * (4 * t + g) + h;
+      float a[4] = {__shfl_sync(SG_FULL, fa.x, src), __shfl_sync(SG_FULL, fa.y, src), __shfl_sync(SG_FULL, fa.z, src),
+                    __shfl_sync(SG_FULL, fa.w, src)};
+      float at[4];
+      if (TSDF) {
+        at[0] = __shfl_sync(SG_FULL, ft.x, src), at[1] = __shfl_sync(SG_FULL, ft.y, src);
+        at[2] = __shfl_sync(SG_FULL, ft.z, src), at[3] = __shfl_sync(SG_FULL, ft.w, src);
+      }
+      if (C == 3) {  // the lane's own corner
+        a[0] = (l8 & 2) ? ((l8 & 1) ? a[3] : a[2]) : ((l8 & 1) ? a[1] : a[0]);
+        if (TSDF) at[0] = (l8 & 2) ? ((l8 & 1) ? at[3] : at[2]) : ((l8 & 1) ? at[1] : at[0]);
+      }
+      const uint32_t r = j + 4 * t + g, past = min(j + 4 * t + 4, end);
+      bool open = r < end;  // the lanes' record waits for its cell
+      while (true) {
+        if (open && r < ce) {
+          open = false;
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            if (TSDF) acct[c] += at[c];
+#pragma unroll
+            for (int v = 0; v < NV; v++) acc[c][v] = __fmaf_rn(a[c], gv[t][v], acc[c][v]);
+          }
+        }
+        if (ce > past) break;
+        // the end of a cell
+        __syncwarp();
+        const int at0 = __shfl_sync(SG_FULL, cvox, ci), in = __shfl_sync(SG_FULL, cin, ci);
+        const bool add = (in >> cr1) & 1;
+        float *gp = q.grad_feat + (long)(at0 + at1) * C + ch;
+        if constexpr (C == 16) {
+          float s2[2][4], s1[4], t2[2], t1 = 0.0f;
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+              const float keep = (g & 2) ? acc[2 + c][v] : acc[c][v], send = (g & 2) ? acc[c][v] : acc[2 + c][v];
+              s2[c][v] = keep + __shfl_xor_sync(SG_FULL, send, 16);
+            }
+            if (TSDF) {
+              const float keep = (g & 2) ? acct[2 + c] : acct[c], send = (g & 2) ? acct[c] : acct[2 + c];
+              t2[c] = keep + __shfl_xor_sync(SG_FULL, send, 16);
+            }
+          }
+#pragma unroll
+          for (int v = 0; v < 4; v++)
+            s1[v] = ((g & 1) ? s2[1][v] : s2[0][v]) + __shfl_xor_sync(SG_FULL, (g & 1) ? s2[0][v] : s2[1][v], 8);
+          if (TSDF) t1 = ((g & 1) ? t2[1] : t2[0]) + __shfl_xor_sync(SG_FULL, (g & 1) ? t2[0] : t2[1], 8);
+          if (add) {
+            red_add_f32x4(gp, s1[0], s1[1], s1[2], s1[3]);
+            if (TSDF && (l8 & 3) == 0) atomicAdd(q.grad_tsdf + (long)(at0 + at1), t1);
+          }
+        } else {
+          float v[4] = {acc[0][0], acc[0][1], acc[0][NV - 1], TSDF ? acct[0] : 0.0f};
+#pragma unroll
+          for (int k = 0; k < (TSDF ? 4 : 3); k++) {
+            v[k] += __shfl_xor_sync(SG_FULL, v[k], 16);
+            v[k] += __shfl_xor_sync(SG_FULL, v[k], 8);
+          }
+          if (add) {  // lanes of the four groups: a channel each, the TSDF gradient
+            if (g < 3) atomicAdd(gp + g, g == 0 ? v[0] : (g == 1 ? v[1] : v[2]));
+            else if (TSDF) atomicAdd(q.grad_tsdf + (long)(at0 + at1), v[3]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          if (TSDF) acct[c] = 0.0f;
+#pragma unroll
+          for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
+        }
+        if (++u == ub) {
+          ce = 0xffffffffu;  // the records are done
+          break;
+        }
+        if (++ci == 32) load_cells();
+        ce = __shfl_sync(SG_FULL, cend, ci);
+      }
+    }
+    fa = nfa;
+    ft = nft;
+    k = nk;
   }
 }
 
@@ -349,11 +348,12 @@ size_t det_layout(long R, int nseg, int C, long cap, char *base, DetWork *w) {
   d.hit_ray = (int *)take((size_t)R * 4);
   d.hit_slot = (int *)take((size_t)R * 4);
   d.seg_hit = (int *)take((size_t)(nseg + 1) * 4);
+  d.seg_slot = (int *)take((size_t)(nseg + 1) * 4);
   d.ray_nrec = (int *)take((size_t)R * 4);
   d.ray_g = (float *)take((size_t)R * C * 4);
   d.rec_key = (uint32_t *)take((size_t)cap * 4);
   d.rec = (GradRecord *)take((size_t)cap * sizeof(GradRecord));
-  d.pay = (GradRecord *)take((size_t)cap * sizeof(GradRecord));
+  d.rec_t = (GradRecord *)take((size_t)cap * sizeof(GradRecord));
   // one more than cap: after the sort, one of the pairs holds the distinct
   // cells' first positions and the end of the last run
   d.ka = (uint32_t *)take((size_t)(cap + 1) * 4);
@@ -380,14 +380,13 @@ int launch_det_prepare(const DetWork &w, const SgRaySegments &seg, int S_max, co
   launch_excl_scan(w.hitb, R, w.hitb, w.scan_scratch, w.cnt + kDetHits, stream);
   launch_excl_scan(w.slotb, R, w.slotb, w.scan_scratch, w.cnt + kDetSlotsNeeded, stream);
   det_ray_emit_kernel<<<grid_for(R), 256, 0, stream>>>(R, hit_count, w.hitb, w.slotb, w.hit_ray, w.hit_slot, o);
-  det_seg_kernel<<<1, 256, 0, stream>>>(seg, R, w.hitb, w.cnt, w.seg_hit, cap, status);
+  det_seg_kernel<<<1, 256, 0, stream>>>(seg, R, w.hitb, w.slotb, w.cnt, w.seg_hit, w.seg_slot, cap, status);
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
 
-int launch_det_reduce(const DetWork &w, const RecordKeys &keys, long R, long cap, int C, float *grad_feat,
-                      float *grad_tsdf,
-                      sg_stream_t stream) {
+int launch_det_reduce(const DetWork &w, const RecordKeys &keys, const SgRaySegments &seg, int S_max, long R, long cap,
+                      int C, float *grad_feat, float *grad_tsdf, sg_stream_t stream) {
   int key_bits = 1;
   while (key_bits < 32 && ((uint64_t)1 << key_bits) <= (uint64_t)keys.invalid) key_bits++;
   const int g = grid_for(cap, 16);
@@ -401,18 +400,18 @@ int launch_det_reduce(const DetWork &w, const RecordKeys &keys, long R, long cap
   const uint32_t *skey = (passes & 1) ? w.ka : w.kb;
   const uint32_t *sval = (passes & 1) ? w.va : w.vb;
   // the other pair is free now: head flags and their scan in one buffer,
-  // the distinct cells' first positions in the other; their keys where the
-  // unsorted keys were
+  // the distinct cells' first positions in the other
   int *heads = (int *)((passes & 1) ? w.kb : w.ka);
   int *ustart = (int *)((passes & 1) ? w.vb : w.va);
-  uint32_t *ukey = w.rec_key;
+  int *bound = (int *)w.sort_scratch;  // free behind the sort
   det_heads_kernel<<<g, 256, 0, stream>>>(skey, w.cnt, heads);
   launch_excl_scan_dev(heads, cap, w.cnt + kDetValid, heads, w.scan_scratch, w.cnt + kDetCells, stream);
-  det_unique_kernel<<<g, 256, 0, stream>>>(skey, heads, w.cnt, ukey, ustart);
-  det_gather_kernel<<<g, 256, 0, stream>>>(sval, w.cnt, w.rec, w.pay);
-  DetReduceParams q{keys, w.cnt, ukey, ustart, w.pay, w.ray_g, grad_feat, grad_tsdf};
+  det_unique_kernel<<<g, 256, 0, stream>>>(skey, heads, w.cnt, keys.cls, w.rec_key, ustart, bound);
+  DetReduceParams q{keys, FixedDiv31::of((uint32_t)keys.D + 1),
+                    SlotRays{w.seg_slot, w.seg_hit, seg.samples, seg.count, S_max},
+                    w.cnt, w.rec_key, ustart, heads, bound, sval, w.rec, w.rec_t, w.ray_g, grad_feat, grad_tsdf};
   for (int cls = 0; cls < 8; cls++) {
-    const dim3 g(num_sms() * 8), blk(256);
+    const dim3 g(num_sms() * 3), blk(256);
     if (C == 16) {
       if (grad_tsdf) det_class_kernel<16, true><<<g, blk, 0, stream>>>(q, cls);
       else det_class_kernel<16, false><<<g, blk, 0, stream>>>(q, cls);

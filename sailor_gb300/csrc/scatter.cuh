@@ -33,11 +33,31 @@ __host__ inline bool record_keys_fit(int B, int D) {
   return (double)B * (double)(D + 1) * (double)(D + 1) * (double)(D + 1) * 8.0 < 4294967295.0;
 }
 
-// One gradient record (32 bytes, one memory sector): the sample's cell
-// fractions and compositing weight, its compact ray and TSDF gradient (bits).
-struct __align__(16) GradRecord {
-  float4 fw;  // f0, f1, f2, w
-  int4 kt;    // k, gt bits, 0, 0
+// One gradient record (32 bytes, one memory sector): of a run of a ray's
+// samples in one cell, the 8 corners' sums of corner weight x compositing
+// weight.  The TSDF's records (corner weight x TSDF gradient) have the same
+// form.  The ray follows from the record's slot (SlotRays).
+struct __align__(32) GradRecord {
+  float a[8];
+};
+
+// The compact ray a slot belongs to: the rays with hits of a segment have its
+// sample count of slots each.
+struct SlotRays {
+  const int *seg_slot;  // [count]: first slot of each segment's rays
+  const int *seg_hit;   // compact index of its first ray
+  const int *samples;
+  int count, S_max;
+  __device__ __forceinline__ int ray(uint32_t slot) const {
+    int lo = 0, hi = count - 1;  // the last segment that starts at or before the slot
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if ((uint32_t)__ldg(seg_slot + mid) <= slot) lo = mid;
+      else hi = mid - 1;
+    }
+    const int S = min(__ldg(samples + lo), S_max);
+    return __ldg(seg_hit + lo) + (int)((slot - (uint32_t)__ldg(seg_slot + lo)) / (uint32_t)S);
+  }
 };
 
 __device__ __forceinline__ uint32_t record_key(const RecordKeys &k, int b, const int (&i0)[3]) {
@@ -46,18 +66,6 @@ __device__ __forceinline__ uint32_t record_key(const RecordKeys &k, int b, const
   const uint32_t x = (uint32_t)(i0[0] + 1), y = (uint32_t)(i0[1] + 1), z = (uint32_t)(i0[2] + 1);
   const uint32_t cls = ((x & 1u) << 2) | ((y & 1u) << 1) | (z & 1u);
   return cls * k.cls + (((uint32_t)b * e + x) * e + y) * e + z;
-}
-
-// Frame and lower corner of a valid key.
-__device__ __forceinline__ void record_cell(const RecordKeys &k, uint32_t key, int &b, int (&i0)[3]) {
-  const uint32_t e = (uint32_t)(k.D + 1);
-  uint32_t c = key % k.cls;
-  b = (int)(c / k.frame);
-  c -= (uint32_t)b * k.frame;
-  i0[2] = (int)(c % e) - 1;
-  c /= e;
-  i0[1] = (int)(c % e) - 1;
-  i0[0] = (int)(c / e) - 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -78,12 +86,11 @@ struct DetWork {
                             // records with a cell
   int *hitb, *slotb;        // [R]: per ray -> exclusive counts of rays with hits / record slots
   int *hit_ray, *hit_slot;  // [R]: compact list of rays with hits, first slot of each
-  int *seg_hit;             // [segments + 1]: compact index of each segment's first ray
+  int *seg_hit, *seg_slot;  // [segments + 1]: compact index and slot of each segment's first ray with hits
   int *ray_nrec;            // [R]: per compact ray, its records (then their first position)
   float *ray_g;             // [R][C]: per compact ray, head^T (colour gradient)
   uint32_t *rec_key;        // [cap] cell key per slot (later: the distinct cells' keys)
-  GradRecord *rec;          // [cap] record per slot
-  GradRecord *pay;          // [cap] the records in sorted key order
+  GradRecord *rec, *rec_t;  // [cap] record per slot; the TSDF's
   uint32_t *ka, *va, *kb, *vb;  // [cap] sort buffers
   void *sort_scratch;
   int *scan_scratch;
@@ -97,10 +104,15 @@ struct DetTrainOut {  // outputs of rays without hits (training step)
 
 struct DetReduceParams {
   RecordKeys keys;
+  FixedDiv31 by_edge;     // by D + 1
+  SlotRays rays;
   const int *cnt;
-  const uint32_t *ukey;
+  const uint32_t *ukey;   // distinct cells: key, first sorted position
   const int *ustart;
-  const GradRecord *pay;
+  const int *heads;       // per sorted position: cells that start before it
+  const int *bound;       // first cell of each parity class
+  const uint32_t *slot;   // per sorted position: the record
+  const GradRecord *rec, *rec_t;
   const float *ray_g;
   float *grad_feat, *grad_tsdf;
 };
@@ -116,8 +128,7 @@ int launch_det_prepare(const DetWork &w, const SgRaySegments &seg, int S_max, co
 
 // Sort the records, find the distinct cells and add their gradients into
 // the grids (grad_tsdf may be null).
-int launch_det_reduce(const DetWork &w, const RecordKeys &keys, long R, long cap, int C, float *grad_feat,
-                      float *grad_tsdf,
-                      sg_stream_t stream);
+int launch_det_reduce(const DetWork &w, const RecordKeys &keys, const SgRaySegments &seg, int S_max, long R, long cap,
+                      int C, float *grad_feat, float *grad_tsdf, sg_stream_t stream);
 
 }  // namespace sg
