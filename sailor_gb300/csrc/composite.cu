@@ -142,9 +142,11 @@ constexpr int kAhead = 4;     // row loads in flight a lane
 
 // V: floats a lane holds of a row (4, 2, 1), p.lanes lanes (a power of two) per
 // row; V == 0: a lane per sample, C <= 3.
-// ONE: at most 32 positions (the loops over blocks go: 16.8 M samples of three
-// channels, 32 a ray, 123 -> 98 us).
-template <int V, bool ONE>
+// OPT, V == 0: at most 32 positions (the loops over blocks go: 16.8 M samples of
+// three channels, 32 a ray, 123 -> 98 us).  OPT, V > 0: a block's rows take more
+// than kAhead steps; their sums are added in pairs and per block, so that the
+// error stays that of a sum over the lanes of a warp.
+template <int V, bool OPT>
 __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
   __shared__ float s_zall[8][kMaxPos];
   __shared__ __align__(16) float s_fall[8][64];
@@ -153,6 +155,7 @@ __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
   float *s_f = s_fall[threadIdx.x >> 5];
   const int C = p.C, S = p.S;
   constexpr int N = V ? V : 3;
+  constexpr bool ONE = V == 0 && OPT, LONG = V > 0 && OPT;
   const int L = p.lanes, c0 = V ? (lane & (L - 1)) * V : 0;  // the lane's channels
   const bool own = V && c0 < C;
   for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < p.R;
@@ -184,6 +187,9 @@ __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
         } else {
           const unsigned ub = __ballot_sync(SG_FULL, v.used);
           // up to kAhead row loads in flight
+          float prev[N], part[N];
+#pragma unroll
+          for (int c = 0; c < N; c++) part[c] = 0.0f;
           for (int it = 0; it < L; it += kAhead) {
             RowVec<N> f[kAhead];
             float w[kAhead];
@@ -196,10 +202,18 @@ __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
               if (on) f[u].load(p.feats + (rb + s) * C + c0);
               else f[u].zero(), w[u] = 0.0f;
             }
+            static_assert(kAhead == 4, "two pairs");
 #pragma unroll
-            for (int u = 0; u < kAhead; u++)
+            for (int c = 0; c < N; c++) {
+              const float x = __fmaf_rn(w[0], f[0].v[c], w[1] * f[1].v[c]) + __fmaf_rn(w[2], f[2].v[c], w[3] * f[3].v[c]);
+              if (!LONG) acc[c] += x;
+              else if (it & kAhead) part[c] += prev[c] + x;
+              else prev[c] = x;
+            }
+          }
+          if (LONG) {
 #pragma unroll
-              for (int c = 0; c < N; c++) acc[c] += w[u] * f[u].v[c];
+            for (int c = 0; c < N; c++) acc[c] += part[c];
           }
         }
       }
@@ -411,7 +425,7 @@ static int launch_comp(const CompParams &p, bool bwd, sg_stream_t stream) {
   int g = ceil_div(p.R * 32, 256);
   if (g > num_sms() * 64) g = num_sms() * 64;
   if (bwd) composite_bwd_kernel<V><<<g, 256, kBwdSmem, stream>>>(p);
-  else if (V == 0 && p.S <= 32) composite_fwd_kernel<V, V == 0><<<g, 256, 0, stream>>>(p);
+  else if (V == 0 ? p.S <= 32 : p.lanes > kAhead) composite_fwd_kernel<V, true><<<g, 256, 0, stream>>>(p);
   else composite_fwd_kernel<V, false><<<g, 256, 0, stream>>>(p);
   return SG_OK;
 }
