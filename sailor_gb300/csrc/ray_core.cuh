@@ -21,13 +21,6 @@ struct SampleParams {
   unsigned long long seed;  // rands == NULL and seed != 0: hashed jitter
 };
 
-// Warp-private shared scratch of the sampler.
-struct SampleScratch {
-  int start[32];
-  float mn[32], off[32];
-  int id[32];
-};
-
 // depth of the j-th sample (0-based) of a hit with n samples:
 // base = min + off*(j+1); z = base - off/2 + off*rand   (sampling_kernel.cu:1142-1148)
 __device__ __forceinline__ float sample_z(float mn, float off, int j, float rnd) {
@@ -41,13 +34,17 @@ __device__ __forceinline__ float sample_z(float mn, float off, int j, float rnd)
 // sample counts exactly as the reference's serial loop, a warp scan turns
 // the serial "samples left" capping into output ranges, and the chunk's
 // samples are generated position-parallel: the owner of position q is the
-// last hit whose range starts at or before q (starts are non-decreasing and
-// strictly increasing over hits that get samples).  Returns #samples.
+// last hit whose range starts at or before q.  The chunk's valid hits are its
+// leading lanes and get a sample each at least, so the owner is the number of
+// starts at or before q, less one: the starts among 32 positions are one OR
+// over the warp, and the owner's range comes by shuffles (a binary search in
+// shared memory per sample made sampling 38 % of the training pass).
+// Returns #samples.
 // b: the ray's frame; S: its sample count (<= p.S, the row stride of rands).
 // IDS: node ids are written too (si); without it si is not touched.
 template <bool IDS = true>
 __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, int b, int S, int nh,
-                                               float rand_const, float *sz, int *si, SampleScratch &sc) {
+                                               float rand_const, float *sz, int *si) {
   const int lane = lane_id();
   const int *hi = p.hit_idx + (size_t)r * p.W;
   const float *h0 = p.hit_t0 + (size_t)r * p.W, *h1 = p.hit_t1 + (size_t)r * p.W;
@@ -90,27 +87,20 @@ __device__ __forceinline__ int warp_sample_ray(const SampleParams &p, long r, in
       const int start = has + incl - n;
       int ne = S - start;
       ne = ne < 0 ? 0 : (ne < n ? ne : n);
-      sc.start[lane] = start;
-      sc.mn[lane] = mn;
-      sc.off[lane] = (mx - mn) / (float)(ne + 1);
-      if (IDS) sc.id[lane] = id;
-      __syncwarp();
+      const float off = (mx - mn) / (float)(ne + 1);
       const int end = min(has + __shfl_sync(SG_FULL, incl, 31), S);
-      // owners are among the lanes with samples; lanes past the last of
-      // them start at or after end, so the search stops there
-      const unsigned with_n = __ballot_sync(SG_FULL, n > 0);
-      const int last = with_n ? 31 - __clz(with_n) : 0;
-      for (int q = has + lane; q < end; q += 32) {
-        int lo = 0, up = last;
-        while (lo < up) {
-          const int mid = (lo + up + 1) >> 1;
-          if (sc.start[mid] <= q) lo = mid;
-          else up = mid - 1;
+      int before = 0;  // hits that start before the 32 positions
+      for (int q0 = has; q0 < end; q0 += 32) {
+        const unsigned m = __reduce_or_sync(SG_FULL, n > 0 && start >= q0 && start < q0 + 32 ? 1u << (start - q0) : 0u);
+        const int own = before + __popc(m & ((2u << lane) - 1u)) - 1, q = q0 + lane;
+        const float omn = __shfl_sync(SG_FULL, mn, own), ooff = __shfl_sync(SG_FULL, off, own);
+        const int ostart = __shfl_sync(SG_FULL, start, own), oid = IDS ? __shfl_sync(SG_FULL, id, own) : 0;
+        if (q < end) {
+          sz[q] = sample_z(omn, ooff, q - ostart, jitter(q));
+          if (IDS) si[q] = oid;
         }
-        sz[q] = sample_z(sc.mn[lo], sc.off[lo], q - sc.start[lo], jitter(q));
-        if (IDS) si[q] = sc.id[lo];
+        before += __popc(m);
       }
-      __syncwarp();
       has = end;
       nvalid += __popc(__ballot_sync(SG_FULL, ok));
     }

@@ -50,9 +50,11 @@
 // the adjoint, packed taps: 2^20 random rays of 96 samples, forward 1.46 /
 // 1.27 / 1.40 ms, adjoint 5.67 / 5.35 / 5.22 ms (at 4 the shared memory of
 // 128 positions takes 217 KB of the SM); the record pass and reduction of a
-// 4.2 M-ray step 5.60 / 5.39 / 5.39 ms.
+// 4.2 M-ray step 4.13 / 4.01 / 4.05 ms.  Unpacked forward (scalar taps, more
+// registers), 2^20 pixel rays of a 512^3 frame with their intersection, at 3 /
+// 4 / 5: 1.69 / 1.78 / 1.76 ms.
 #ifndef SG_RENDER_FWD_MINB
-#define SG_RENDER_FWD_MINB 4
+#define SG_RENDER_FWD_MINB(PACKED) ((PACKED) ? 4 : 3)
 #endif
 #ifndef SG_RENDER_REC_MINB
 #define SG_RENDER_REC_MINB 4
@@ -125,7 +127,6 @@ __device__ __forceinline__ void ray_frame(const RenderParams &p, long r, int &b,
 // 128 positions).
 //   z    [cap]     samples, then sorted depths
 //   f    [32 + 32] transmittance factors of a block and the values before them
-//   sc             sampler scratch
 //   id, pos [cap]  node ids and sorted positions (forward with out_node)
 //   keep [8][cap]  per position, for the adjoint: see Keep
 //   cw   [32][9], wg [32]  corner weights and (weight, TSDF gradient) of a
@@ -134,7 +135,6 @@ enum { kKeepW = 0, kKeepR, kKeepG, kKeepB, kKeepS01, kKeepAl, kKeepTb, kKeepDl, 
 
 struct RenderSmem {
   float *z, *f;
-  SampleScratch *sc;
   int *id, *pos;
   float *keep;
   float *cw;
@@ -151,12 +151,11 @@ __host__ __device__ constexpr bool mode_keeps(int mode) {
 __host__ __device__ constexpr bool mode_scatters(int mode) { return mode == kModeBwd || mode == kModeTrain; }
 
 __host__ __device__ constexpr int render_warp_words(int mode, int cap, bool ids) {
-  return cap + 64 + 128 + (ids ? 2 * cap : 0) + (mode_keeps(mode) ? kKeepWords * cap : 0) +
+  return cap + 64 + (ids ? 2 * cap : 0) + (mode_keeps(mode) ? kKeepWords * cap : 0) +
          (mode_scatters(mode) ? 32 * 9 + 64 : 0);
 }
 
 __device__ __forceinline__ RenderSmem render_smem(float *base, int mode, int cap, bool ids) {
-  static_assert(sizeof(SampleScratch) == 128 * 4, "sampler scratch of 128 words");
   RenderSmem sm;
   sm.cap = cap;
   float *w = base + (threadIdx.x >> 5) * render_warp_words(mode, cap, ids);
@@ -164,8 +163,6 @@ __device__ __forceinline__ RenderSmem render_smem(float *base, int mode, int cap
   w += cap;
   sm.f = w;
   w += 64;
-  sm.sc = reinterpret_cast<SampleScratch *>(w);
-  w += 128;
   sm.id = sm.pos = nullptr;
   if (ids) {
     sm.id = reinterpret_cast<int *>(w);
@@ -390,7 +387,9 @@ struct RayWalk {
 // Block e: density taps, alpha, transmittance, and the colour of the samples
 // that count -- positions past the early termination are never tapped.
 // Returns false when the block holds no sample.
-template <int C, bool PACKED>
+// U: positions per unrolled stretch of the transmittance chain (the record
+// pass is the faster for 32, by 0.7 %; forward and adjoint for 8, by 2 to 6 %).
+template <int C, bool PACKED, int U = 8>
 __device__ __forceinline__ bool eval_block(const RenderParams &p, const RayGeom &g, int S, int e,
                                            const RenderSmem &sm, const float *s_head, RayWalk &wk, BlockEval &v) {
   const int lane = lane_id(), i = e * 32 + lane;
@@ -423,7 +422,7 @@ __device__ __forceinline__ bool eval_block(const RenderParams &p, const RayGeom 
     v.dl = depth_step(sm.z, S, i, v.z);
     v.al = 1.0f - expf(-sg * v.dl);
   }
-  const int stop = block_transmittance(valid ? 1.0f - v.al : 1.0f, wk.T, p.t_thres, wk.m0 - e * 32, S - e * 32, sm.f,
+  const int stop = block_transmittance<U>(valid ? 1.0f - v.al : 1.0f, wk.T, p.t_thres, wk.m0 - e * 32, S - e * 32, sm.f,
                                        v.tb);
   if (stop < 32) wk.end = e * 32 + stop + 1;
   v.used = valid && i < wk.end;
@@ -444,7 +443,7 @@ __device__ __forceinline__ bool eval_block(const RenderParams &p, const RayGeom 
 template <bool IDS>
 __device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, int b, int S, const RenderSmem &sm) {
   const int nh = p.hit_count ? min(__ldg(p.hit_count + r), p.sp.W) : p.sp.W;
-  const int done = warp_sample_ray<IDS>(p.sp, r, b, S, nh, p.rand_const, sm.z, sm.id, *sm.sc);
+  const int done = warp_sample_ray<IDS>(p.sp, r, b, S, nh, p.rand_const, sm.z, sm.id);
   if (done > 0) warp_sort_samples<4, IDS>(sm.z, sm.pos, S, done);
   return done;
 }
@@ -452,7 +451,7 @@ __device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, in
 extern __shared__ __align__(16) float s_render[];
 
 template <int C, bool IDS, bool PACKED>
-__global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB) render_fwd_kernel(RenderParams p) {
+__global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB(PACKED)) render_fwd_kernel(RenderParams p) {
   __shared__ __align__(16) float s_head[3 * C];
   load_head<C>(p.head, s_head);
   const RenderSmem sm = render_smem(s_render, kModeFwd, p.cap, IDS);
@@ -717,7 +716,7 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
 #pragma unroll 1
     for (; e1 * 32 < wk.end; e1++) {
       BlockEval v;
-      const bool any = eval_block<C, PACKED>(p, g, S, e1, sm, s_head, wk, v);
+      const bool any = eval_block<C, PACKED, MODE == kModeRec ? 32 : 8>(p, g, S, e1, sm, s_head, wk, v);
       if (mode_keeps(MODE)) {
         const int i = e1 * 32 + lane;
         sm.k(kKeepW, i) = any ? v.w : 0.0f;

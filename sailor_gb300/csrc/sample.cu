@@ -22,12 +22,11 @@ template <int E>
 __global__ void __launch_bounds__(256) sample_coarse_kernel(SampleParams p) {
   __shared__ float s_z[8][32 * E];
   __shared__ int s_i[8][32 * E];
-  __shared__ SampleScratch s_sc[8];
   const int lane = lane_id(), w8 = threadIdx.x >> 5;
   const long R = (long)p.t.B * p.N;
   for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < R;
        r += ((long)gridDim.x * blockDim.x) >> 5) {
-    warp_sample_ray(p, r, (int)(r / p.N), p.S, p.W, 0.5f, s_z[w8], s_i[w8], s_sc[w8]);
+    warp_sample_ray(p, r, (int)(r / p.N), p.S, p.W, 0.5f, s_z[w8], s_i[w8]);
     for (int q = lane; q < p.S; q += 32) {
       p.sampled_z[(size_t)r * p.S + q] = s_z[w8][q];
       p.sampled_idx[(size_t)r * p.S + q] = s_i[w8][q];
@@ -119,14 +118,13 @@ __global__ void __launch_bounds__(256) sample_sorted_kernel(SampleParams p, cons
   __shared__ __align__(16) float s_z[8][32 * E];
   __shared__ int s_i[8][32 * E];
   __shared__ int s_p[8][32 * E];
-  __shared__ SampleScratch s_sc[8];
   const int lane = lane_id(), w8 = threadIdx.x >> 5;
   const long R = (long)p.t.B * p.N;
   const int S = p.S;
   for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < R;
        r += ((long)gridDim.x * blockDim.x) >> 5) {
     const int nh = hit_count ? min(hit_count[r], p.W) : p.W;
-    const int done = warp_sample_ray(p, r, (int)(r / p.N), S, nh, rand_const, s_z[w8], s_i[w8], s_sc[w8]);
+    const int done = warp_sample_ray(p, r, (int)(r / p.N), S, nh, rand_const, s_z[w8], s_i[w8]);
     warp_sort_samples<E, true>(s_z[w8], s_p[w8], S, done);
     for (int i = lane; i < S; i += 32) {
       out_z[(size_t)r * S + i] = s_z[w8][i];
