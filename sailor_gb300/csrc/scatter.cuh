@@ -84,7 +84,7 @@ enum {
 struct DetWork {
   int *cnt;                 // counters: rays with hits, slots needed, slots used, distinct cells,
                             // records with a cell
-  int *hitb, *slotb;        // [R]: per ray -> exclusive counts of rays with hits / record slots
+  int *hitb;                // [R]: per ray -> exclusive count of rays with hits
   int *hit_ray, *hit_slot;  // [R]: compact list of rays with hits, first slot of each
   int *seg_hit, *seg_slot;  // [segments + 1]: compact index and slot of each segment's first ray with hits
   int *ray_nrec;            // [R]: per compact ray, its records (then their first position)

@@ -22,39 +22,12 @@
 
 namespace sg {
 
-constexpr int kScanBlock = 1024;  // ints per scan block
 constexpr int kSortTile = 4096;   // items per sort tile (256 threads x 16)
 constexpr int kDigits = 256;
 
 // ---------------------------------------------------------------------------
 // exclusive scan
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int block_excl_scan_256(int v, int *s_warp, int &total) {
-  // exclusive scan of one int per thread over a 256-thread block
-  const int lane = lane_id(), w = threadIdx.x >> 5;
-  const int incl = warp_incl_scan(v);
-  if (lane == 31) s_warp[w] = incl;
-  __syncthreads();
-  if (w == 0) {
-    const int x = lane < 8 ? s_warp[lane] : 0;
-    const int xi = warp_incl_scan(x);
-    if (lane < 8) s_warp[8 + lane] = xi - x;
-    if (lane == 7) s_warp[16] = xi;
-  }
-  __syncthreads();
-  const int out = s_warp[8 + w] + incl - v;
-  total = s_warp[16];
-  __syncthreads();
-  return out;
-}
-
-// n_dev (may be null): the live count in device memory, at most n
-__device__ __forceinline__ long live_count(long n, const int *n_dev) {
-  if (!n_dev) return n;
-  const long m = *n_dev;
-  return m < n ? m : n;
-}
-
 // Blocks of kScanBlock elements up to the live count; a fixed grid strides
 // over them, so a capacity far above the live count costs no launches.
 __global__ void __launch_bounds__(256) scan_block_sums_kernel(const int *__restrict__ in, long n,
@@ -125,6 +98,10 @@ __global__ void __launch_bounds__(256) scan_apply_kernel(const int *__restrict__
       run += v[k];
     }
   }
+}
+
+void launch_scan_sums(int *sums, long n, const int *n_dev, int *total, sg_stream_t stream) {
+  scan_sums_kernel<<<1, 1024, 0, stream>>>(sums, n, n_dev, total);
 }
 
 size_t scan_scratch_ints(long n) { return (size_t)ceil_div(n, kScanBlock) + 1; }

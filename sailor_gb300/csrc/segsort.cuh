@@ -7,6 +7,38 @@
 
 namespace sg {
 
+// The scan's parts, for kernels that form its input or use its output in place:
+// blocks of kScanBlock elements (256 threads x 4), their sums in sums[block];
+// launch_scan_sums turns those of the first min(*n_dev, n) elements into offsets.
+constexpr int kScanBlock = 1024;
+void launch_scan_sums(int *sums, long n, const int *n_dev, int *total, sg_stream_t stream);
+
+__device__ __forceinline__ int block_excl_scan_256(int v, int *s_warp, int &total) {
+  // exclusive scan of one int per thread over a 256-thread block
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  const int incl = warp_incl_scan(v);
+  if (lane == 31) s_warp[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    const int x = lane < 8 ? s_warp[lane] : 0;
+    const int xi = warp_incl_scan(x);
+    if (lane < 8) s_warp[8 + lane] = xi - x;
+    if (lane == 7) s_warp[16] = xi;
+  }
+  __syncthreads();
+  const int out = s_warp[8 + w] + incl - v;
+  total = s_warp[16];
+  __syncthreads();
+  return out;
+}
+
+// n_dev (may be null): the live count in device memory, at most n
+__device__ __forceinline__ long live_count(long n, const int *n_dev) {
+  if (!n_dev) return n;
+  const long m = *n_dev;
+  return m < n ? m : n;
+}
+
 // ints of scratch an exclusive scan of n elements needs
 size_t scan_scratch_ints(long n);
 
