@@ -129,8 +129,8 @@ __device__ __forceinline__ void ray_frame(const RenderParams &p, long r, int &b,
 //   f    [32 + 32] transmittance factors of a block and the values before them
 //   id, pos [cap]  node ids and sorted positions (forward with out_node)
 //   keep [8][cap]  per position, for the adjoint: see Keep
-//   cw   [32][9], wg [32]  corner weights and (weight, TSDF gradient) of a
-//                  block's samples (in-kernel scatter)
+//   cw   [32][9], wg [32]  corner sums and (voxel, corners inside) of a block's
+//                  runs (in-kernel scatter)
 enum { kKeepW = 0, kKeepR, kKeepG, kKeepB, kKeepS01, kKeepAl, kKeepTb, kKeepDl, kKeepWords };
 
 struct RenderSmem {
@@ -138,7 +138,7 @@ struct RenderSmem {
   int *id, *pos;
   float *keep;
   float *cw;
-  float2 *wg;
+  unsigned long long *wg;
   int cap;
   __device__ __forceinline__ float &k(int which, int i) const { return keep[which * cap + i]; }
 };
@@ -172,7 +172,7 @@ __device__ __forceinline__ RenderSmem render_smem(float *base, int mode, int cap
   sm.keep = w;
   if (mode_keeps(mode)) w += kKeepWords * cap;
   sm.cw = w;
-  sm.wg = reinterpret_cast<float2 *>(w + 32 * 9);
+  sm.wg = reinterpret_cast<unsigned long long *>(w + 32 * 9);
   return sm;
 }
 
@@ -450,6 +450,27 @@ __device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, in
 
 extern __shared__ __align__(16) float s_render[];
 
+// The rays of a CTA: eight consecutive ones, and the same a grid apart.  SHARE:
+// its warps take them one by one, so that a ray that misses or ends early
+// leaves its warp free for the next; otherwise warp w takes the w-th of each
+// eight.  2^20 random rays, a third of them hitting, shared / fixed: forward
+// 1.19 / 1.27 ms, adjoint 4.34 / 4.94; rays that all hit (record pass) 3.91 / 3.86
+// with the reduction, pixel rays of an unpacked frame 1.70 / 1.68 (with their
+// intersection): fixed there.
+template <bool SHARE>
+__device__ __forceinline__ long next_ray(int &next, long first, long &own) {
+  if constexpr (SHARE) {
+    int i = 0;
+    if (lane_id() == 0) i = atomicAdd(&next, 1);
+    i = __shfl_sync(SG_FULL, i, 0);
+    return first + ((long)(i >> 3) * gridDim.x + blockIdx.x) * 8 + (i & 7);
+  } else {
+    const long r = own;
+    own += ((long)gridDim.x * blockDim.x) >> 5;
+    return r;
+  }
+}
+
 template <int C, bool IDS, bool PACKED>
 __global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB(PACKED)) render_fwd_kernel(RenderParams p) {
   __shared__ __align__(16) float s_head[3 * C];
@@ -460,8 +481,13 @@ __global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB(PACKED)) render_fwd_ke
   // a segment table covers rays [ray_begin[0], total): a sub-table of
   // consecutive segments is a group of targets
   const long r0 = p.nseg > 0 ? (long)__ldg(p.seg_begin) : 0;
-  for (long r = r0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < p.R;
-       r += ((long)gridDim.x * blockDim.x) >> 5) {
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  long own = r0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  while (true) {
+    const long r = next_ray<PACKED>(s_next, r0, own);
+    if (r >= p.R) break;
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
     const int done = sample_and_sort<IDS>(p, r, b, S, sm);
@@ -512,78 +538,101 @@ __global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB(PACKED)) render_fwd_ke
 // ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
-// A trilinear cell (lower corner i0, each axis in [-1, D-1] when any corner
-// is inside the grid) packed into one non-negative key of 21 bits per axis;
-// -1 when no corner is inside (the sample contributes nothing).
-__device__ __forceinline__ long long cell_key(const int (&i0)[3], int D) {
-  if (i0[0] < -1 || i0[1] < -1 || i0[2] < -1 || i0[0] >= D || i0[1] >= D || i0[2] >= D) return -1;
-  return ((long long)(i0[0] + 1) << 42) | ((long long)(i0[1] + 1) << 21) | (long long)(i0[2] + 1);
-}
-
-// Scatter of the in-kernel backward.  The colour head is linear, so the
-// feature gradient of the sample at sorted position i is w_i G with
-// G = head^T g_c (g_c: the gradient of the ray's colour, w_i its compositing
-// weight): per cell run only the 8 sums of corner weight x w_i are carried,
-// and G multiplies them when the run ends.  C == 16: lane l owns corner
-// l / 4, channels 4 (l % 4) .. 4 (l % 4) + 3 (one vector reduction), and its
-// corner's TSDF gradient (written by channel group 0).  C == 3: lane l < 24
-// owns corner l / 3, channel l % 3; lane l >= 24 the TSDF gradient of corner
-// l - 24.
-struct Scatter {
-  long long cur;  // cell of the current run, -1: none
-  float a, t;     // corner weight x compositing weight, x TSDF gradient
-};
-
-template <int C, bool FEAT, bool TSDF>
-__device__ __forceinline__ void scatter_flush(const RenderParams &p, int b, const float (&G)[4], Scatter &s) {
+// Sums over the runs of lanes that share a cell, at each run's first lane:
+// 8 corner weights x the compositing weight (A) and x the TSDF gradient (T).
+// stop: the first lane behind this one that is not of its run.
+template <bool A, bool T>
+__device__ __forceinline__ void run_sums(bool has, int stop, const float (&f)[3], float w, float gt, float (&a)[8],
+                                         float (&t)[8]) {
   const int lane = lane_id();
-  const int cell[3] = {(int)(s.cur >> 42) - 1, (int)((s.cur >> 21) & 0x1fffff) - 1, (int)(s.cur & 0x1fffff) - 1};
-  size_t off;
-  if constexpr (C == 16) {
-    if (FEAT && s.a != 0.0f && corner_inside(cell, lane >> 2, p.Df, off))
-      red_add_f32x4(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + 4 * (lane & 3), s.a * G[0], s.a * G[1],
-                    s.a * G[2], s.a * G[3]);
-    if (TSDF && (lane & 3) == 0 && s.t != 0.0f && corner_inside(cell, lane >> 2, p.D, off))
-      atomicAdd(p.grad_tsdf + (size_t)b * p.D * p.D * p.D + off, s.t);
-  } else {
-    if (FEAT && lane < 24 && s.a != 0.0f && corner_inside(cell, lane / 3, p.Df, off))
-      atomicAdd(p.grad_feat + ((size_t)b * p.Df * p.Df * p.Df + off) * C + lane % 3, s.a * G[0]);
-    if (TSDF && lane >= 24 && s.t != 0.0f && corner_inside(cell, lane - 24, p.D, off))
-      atomicAdd(p.grad_tsdf + (size_t)b * p.D * p.D * p.D + off, s.t);
-  }
-  s.a = s.t = 0.0f;
-}
-
-// One block's samples into the run sums: key (-1: none), corner weights from
-// f, the sample's weight and TSDF gradient.
-template <int C, bool FEAT, bool TSDF>
-__device__ __forceinline__ void scatter_block(const RenderParams &p, int b, const RenderSmem &sm, long long key,
-                                              const float (&f)[3], float w, float gt, const float (&G)[4],
-                                              Scatter &s) {
-  const int lane = lane_id();
-  const unsigned m = __ballot_sync(SG_FULL, key >= 0);
-  if (m == 0u) return;
-  if (key >= 0) {
 #pragma unroll
-    for (int cr = 0; cr < 8; cr++) sm.cw[lane * 9 + cr] = corner_weight(f, cr);
-    sm.wg[lane] = make_float2(w, gt);
+  for (int c = 0; c < 8; c++) {
+    const float cw = corner_weight(f, c);
+    if (A) a[c] = has ? cw * w : 0.0f;
+    if (T) t[c] = has ? cw * gt : 0.0f;
   }
-  // run heads: samples whose cell differs from the one before
-  const unsigned before = m & ((1u << lane) - 1u);
-  const long long pk = __shfl_sync(SG_FULL, key, before ? 31 - __clz(before) : 0);
-  const unsigned heads = __ballot_sync(SG_FULL, key >= 0 && key != (before ? pk : s.cur));
+#pragma unroll 1
+  for (int o = 1; __any_sync(SG_FULL, has && lane + o < stop); o <<= 1) {
+    const bool in = lane + o < stop;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      if (A) {
+        const float x = __shfl_down_sync(SG_FULL, a[c], o);
+        if (in) a[c] += x;
+      }
+      if (T) {
+        const float y = __shfl_down_sync(SG_FULL, t[c], o);
+        if (in) t[c] += y;
+      }
+    }
+  }
+}
+
+// A block's samples added into the grids.  The colour head is linear, so the
+// feature gradient of the sample at sorted position i is w_i G with G = head^T
+// g_c (g_c: the gradient of the ray's colour, w_i its compositing weight): each
+// run of samples in one cell is summed first (run_sums), its first lane leaves
+// the 8 sums, the cell's voxel and the corners inside the grid in shared memory,
+// and the warp adds run after run.  C == 16: lane l owns corner l / 4, channels
+// 4 (l % 4) .. + 3 (one vector reduction), and its corner's TSDF gradient
+// (channel group 0).  C == 3: lane l < 24 owns corner l / 3, channel l % 3; lane
+// l >= 24 the TSDF gradient of corner l - 24.
+//
+// keep: the block's 8 x 32 words of the positions' values (all read by now),
+// which take the TSDF sums, corner c of lane l at word (l + 4 c) % 32 of row c.
+// Sample by sample with a flush at each change of cell, 2^20 random rays of 96
+// samples and 16 channels took 5.24 ms, now 4.94 (adjoint; 4.3 with the
+// rays shared among a CTA's warps).
+template <int C, bool FEAT, bool TSDF>
+__device__ __forceinline__ void scatter_block(const RenderParams &p, int b, const RenderSmem &sm, int block, bool used,
+                                              const int (&i0)[3], const float (&f)[3], float w, float gt,
+                                              const float (&G)[4]) {
+  const int lane = lane_id(), D = FEAT ? p.Df : p.D;
+  const unsigned in = used ? corners_inside(i0, D) : 0u;
+  const unsigned m = __ballot_sync(SG_FULL, in != 0u);
+  if (m == 0u) return;
+  const int px = __shfl_up_sync(SG_FULL, i0[0], 1), py = __shfl_up_sync(SG_FULL, i0[1], 1),
+            pz = __shfl_up_sync(SG_FULL, i0[2], 1);
+  const bool head = in != 0u && (lane == 0 || !((m >> (lane - 1)) & 1u) || px != i0[0] || py != i0[1] || pz != i0[2]);
+  const unsigned heads = __ballot_sync(SG_FULL, head);
+  const unsigned stops = (heads | ~m) & ~((2u << lane) - 1u);
+  float a[8], t[8];
+  run_sums<FEAT, TSDF>(in != 0u, stops ? __ffs(stops) - 1 : 32, f, w, gt, a, t);
+  float *keep = sm.keep + block * 32;
+  unsigned long long *cell = sm.wg;
+  __syncwarp();
+  if (head) {
+    // lower corner's voxel (frame included; two's complement) and the corners inside
+    const long at = (((long)b * D + i0[0]) * D + i0[1]) * D + i0[2];
+    cell[lane] = ((unsigned long long)at << 8) | in;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      if (FEAT) sm.cw[lane * 9 + c] = a[c];
+      if (TSDF) keep[c * sm.cap + ((lane + 4 * c) & 31)] = t[c];
+    }
+  }
   __syncwarp();
   const int cr = C == 16 ? lane >> 2 : (lane < 24 ? lane / 3 : lane - 24);
-  for (unsigned q = m; q; q &= q - 1) {
+  const int ch = C == 16 ? 4 * (lane & 3) : lane % 3;
+  const long at1 = ((long)(cr >> 2) * D + ((cr >> 1) & 1)) * D + (cr & 1);
+  const bool fown = FEAT && (C == 16 || lane < 24), town = TSDF && (C == 16 ? (lane & 3) == 0 : lane >= 24);
+  for (unsigned q = heads; q; q &= q - 1) {
     const int j = __ffs(q) - 1;
-    if ((heads >> j) & 1u) {
-      if (s.cur >= 0) scatter_flush<C, FEAT, TSDF>(p, b, G, s);
-      s.cur = __shfl_sync(SG_FULL, key, j);
+    const unsigned long long x = cell[j];
+    if (!((x >> cr) & 1u)) continue;
+    const long v = ((long)x >> 8) + at1;
+    if (fown) {
+      const float k = sm.cw[j * 9 + cr];
+      if (k != 0.0f) {
+        float *g = p.grad_feat + v * C + ch;
+        if (C == 16) red_add_f32x4(g, k * G[0], k * G[1], k * G[2], k * G[3]);
+        else atomicAdd(g, k * G[0]);
+      }
     }
-    const float c = sm.cw[j * 9 + cr];
-    const float2 x = sm.wg[j];
-    if (FEAT) s.a = __fmaf_rn(c, x.x, s.a);
-    if (TSDF) s.t = __fmaf_rn(c, x.y, s.t);
+    if (town) {
+      const float k = keep[cr * sm.cap + ((j + 4 * cr) & 31)];
+      if (k != 0.0f) atomicAdd(p.grad_tsdf + v, k);
+    }
   }
   __syncwarp();
 }
@@ -617,26 +666,8 @@ __device__ __forceinline__ void emit_records(const RenderParams &p, int b, long 
   const unsigned heads = __ballot_sync(SG_FULL, head);
   const unsigned stops = (heads | ~m) & ~((2u << lane) - 1u);  // lanes behind this one that are not of its run
   const int stop = stops ? __ffs(stops) - 1 : 32;
-  float a[8], t[TSDF ? 8 : 1];
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const float cw = corner_weight(f, c);
-    a[c] = has ? cw * w : 0.0f;
-    if (TSDF) t[c] = has ? cw * gt : 0.0f;
-  }
-#pragma unroll 1
-  for (int o = 1; __any_sync(SG_FULL, has && lane + o < stop); o <<= 1) {
-    const bool in = lane + o < stop;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const float x = __shfl_down_sync(SG_FULL, a[c], o);
-      if (in) a[c] += x;
-      if (TSDF) {
-        const float y = __shfl_down_sync(SG_FULL, t[c], o);
-        if (in) t[c] += y;
-      }
-    }
-  }
+  float a[8], t[8];
+  run_sums<true, TSDF>(has, stop, f, w, gt, a, t);
   const long slot = base + n + __popc(heads & ((1u << lane) - 1u));
   if (head && slot < p.rec_cap) {
     float4 *r = reinterpret_cast<float4 *>(p.rec + slot);
@@ -676,8 +707,13 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
   // consecutive segments is a group of targets
   const long it0 = REC ? (long)__ldg(p.k_begin) : (p.nseg > 0 ? (long)__ldg(p.seg_begin) : 0);
   const long it1 = REC ? (long)__ldg(p.k_end) : p.R;
-  for (long it = it0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < it1;
-       it += ((long)gridDim.x * blockDim.x) >> 5) {
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  long own = it0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  while (true) {
+    const long it = next_ray<!REC>(s_next, it0, own);
+    if (it >= it1) break;
     const long r = REC ? (long)__ldg(p.hit_ray + it) : it;
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
@@ -796,7 +832,6 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
           if (lane < 24) G[0] = head_grad<C>(p, lane % 3, gc);
         }
       }
-      Scatter sf{-1, 0.0f, 0.0f}, st{-1, 0.0f, 0.0f};
 #pragma unroll 1
       for (int e = e0; e < e1; e++) {
         const int i = e * 32 + lane;
@@ -842,31 +877,22 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
           int i0[3] = {0, 0, 0};
           float f[3] = {0.0f, 0.0f, 0.0f};
           if (used) feat_cell(p, g, z, i0, f);
-          const long long kf = used ? cell_key(i0, p.Df) : -1;
           if (p.shared) {
-            if (p.grad_feat && p.grad_tsdf) scatter_block<C, true, true>(p, b, sm, kf, f, w, gt, G, sf);
-            else if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, kf, f, w, gt, G, sf);
-            else scatter_block<C, false, true>(p, b, sm, kf, f, w, gt, G, sf);
+            if (p.grad_feat && p.grad_tsdf) scatter_block<C, true, true>(p, b, sm, e, used, i0, f, w, gt, G);
+            else if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, e, used, i0, f, w, gt, G);
+            else scatter_block<C, false, true>(p, b, sm, e, used, i0, f, w, gt, G);
           } else {
-            if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, kf, f, w, gt, G, sf);
+            if (p.grad_feat) scatter_block<C, true, false>(p, b, sm, e, used, i0, f, w, gt, G);
             if (p.grad_tsdf) {
               if (used) {
                 float pt[3];
                 ray_point(g, z, pt);
                 tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
               }
-              scatter_block<C, false, true>(p, b, sm, used ? cell_key(i0, p.D) : -1, f, w, gt, G, st);
+              scatter_block<C, false, true>(p, b, sm, e, used, i0, f, w, gt, G);
             }
           }
         }
-      }
-      if (mode_scatters(MODE)) {
-        if (sf.cur >= 0) {
-          if (p.shared && p.grad_feat && p.grad_tsdf) scatter_flush<C, true, true>(p, b, G, sf);
-          else if (p.grad_feat) scatter_flush<C, true, false>(p, b, G, sf);
-          else scatter_flush<C, false, true>(p, b, G, sf);
-        }
-        if (st.cur >= 0) scatter_flush<C, false, true>(p, b, G, st);
       }
       if (MODE == kModeBwd && p.grad_sigma) {
         // positions of blocks that were not evaluated: no gradient
