@@ -450,25 +450,18 @@ __device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, in
 
 extern __shared__ __align__(16) float s_render[];
 
-// The rays of a CTA: eight consecutive ones, and the same a grid apart.  SHARE:
-// its warps take them one by one, so that a ray that misses or ends early
-// leaves its warp free for the next; otherwise warp w takes the w-th of each
-// eight.  2^20 random rays, a third of them hitting, shared / fixed: forward
-// 1.19 / 1.27 ms, adjoint 4.34 / 4.94; rays that all hit (record pass) 3.91 / 3.86
-// with the reduction, pixel rays of an unpacked frame 1.70 / 1.68 (with their
-// intersection): fixed there.
-template <bool SHARE>
-__device__ __forceinline__ long next_ray(int &next, long first, long &own) {
-  if constexpr (SHARE) {
-    int i = 0;
-    if (lane_id() == 0) i = atomicAdd(&next, 1);
-    i = __shfl_sync(SG_FULL, i, 0);
-    return first + ((long)(i >> 3) * gridDim.x + blockIdx.x) * 8 + (i & 7);
-  } else {
-    const long r = own;
-    own += ((long)gridDim.x * blockDim.x) >> 5;
-    return r;
-  }
+// The rays of a CTA are eight consecutive ones, and the same a grid apart: warp
+// w takes the w-th of each eight, or, where rays may miss, the warps take them
+// one by one (take_ray), so that a ray that misses or ends early leaves its warp
+// free for the next.  2^20 random rays, a third of them hitting, one by one /
+// fixed: forward 1.19 / 1.27 ms, adjoint 4.30 / 4.94; rays that all hit (record
+// pass) 3.91 / 3.85 with the reduction, pixel rays of an unpacked frame 1.70 /
+// 1.68 (with their intersection): fixed there.
+__device__ __forceinline__ long take_ray(int &taken, long first) {
+  int i = 0;
+  if (lane_id() == 0) i = atomicAdd(&taken, 1);
+  i = __shfl_sync(SG_FULL, i, 0);
+  return first + ((long)(i >> 3) * gridDim.x + blockIdx.x) * 8 + (i & 7);
 }
 
 template <int C, bool IDS, bool PACKED>
@@ -481,13 +474,13 @@ __global__ void __launch_bounds__(256, SG_RENDER_FWD_MINB(PACKED)) render_fwd_ke
   // a segment table covers rays [ray_begin[0], total): a sub-table of
   // consecutive segments is a group of targets
   const long r0 = p.nseg > 0 ? (long)__ldg(p.seg_begin) : 0;
-  __shared__ int s_next;
-  if (threadIdx.x == 0) s_next = 0;
-  __syncthreads();
-  long own = r0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  while (true) {
-    const long r = next_ray<PACKED>(s_next, r0, own);
-    if (r >= p.R) break;
+  __shared__ int s_taken;
+  if (PACKED) {
+    if (threadIdx.x == 0) s_taken = 0;
+    __syncthreads();
+  }
+  for (long r = PACKED ? take_ray(s_taken, r0) : r0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < p.R;
+       r = PACKED ? take_ray(s_taken, r0) : r + (((long)gridDim.x * blockDim.x) >> 5)) {
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
     const int done = sample_and_sort<IDS>(p, r, b, S, sm);
@@ -707,13 +700,13 @@ __global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(R
   // consecutive segments is a group of targets
   const long it0 = REC ? (long)__ldg(p.k_begin) : (p.nseg > 0 ? (long)__ldg(p.seg_begin) : 0);
   const long it1 = REC ? (long)__ldg(p.k_end) : p.R;
-  __shared__ int s_next;
-  if (threadIdx.x == 0) s_next = 0;
-  __syncthreads();
-  long own = it0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  while (true) {
-    const long it = next_ray<!REC>(s_next, it0, own);
-    if (it >= it1) break;
+  __shared__ int s_taken;
+  if (!REC) {
+    if (threadIdx.x == 0) s_taken = 0;
+    __syncthreads();
+  }
+  for (long it = REC ? it0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : take_ray(s_taken, it0); it < it1;
+       it = REC ? it + (((long)gridDim.x * blockDim.x) >> 5) : take_ray(s_taken, it0)) {
     const long r = REC ? (long)__ldg(p.hit_ray + it) : it;
     int b, S, sgm;
     ray_frame(p, r, b, S, sgm);
