@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) det_cells_kernel(const uint32_t *__restri
 // memory (12 or fewer of the lanes in use at mean run lengths of 6 to 12),
 // after a pass that gathered the records into sorted order, and every CTA began
 // with a binary search for the class's cells: 26.7 M samples in 12.7 M runs,
-// 2.2 M cells of 4 x 256^3: 1.99 -> 1.01 ms for gather and classes; 2.2 M samples
+// 2.2 M cells of 4 x 256^3: 1.99 -> 0.89 ms for gather and classes; 2.2 M samples
 // in 0.9 M runs, 0.36 M cells: 402 -> 162 us.
 template <int C, bool TSDF>
 __global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, int cls) {
@@ -231,155 +231,160 @@ __global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, in
   const int at1 = ((cr1 >> 2) * D + ((cr1 >> 1) & 1)) * D + (cr1 & 1);
   // (a stretch's position may pass 2^31, no record's does)
   const long P0 = q.ustart[lo], P1 = q.ustart[hi];
-  const long warps = (long)gridDim.x * (blockDim.x >> 5);
-  const long Q = max((P1 - P0 + warps - 1) / warps, 32l);
-  const long pa = P0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Q;
-  if (pa >= P1) return;
-  int u = __ldg(q.heads + pa);
-  const int ub = pa + Q < P1 ? __ldg(q.heads + pa + Q) : hi;
-  if (u >= ub) return;
-  uint32_t j = __ldg(q.ustart + u);
-  const uint32_t end = __ldg(q.ustart + ub);
-  // 32 cells at a time, one a lane: lower corner's voxel, corners inside, end
-  int cvox = 0, cin = 0, cend = 0, ci = 0;
-  auto load_cells = [&]() {
-    if (u + lane < ub) {
-      const uint32_t m = __ldg(q.ukey + u + lane) - (uint32_t)cls * q.keys.cls, e = (uint32_t)D + 1;
-      cend = __ldg(q.ustart + u + lane + 1);
-      const uint32_t xy = q.by_edge.div(m), x = q.by_edge.div(xy), b = q.by_edge.div(x);
-      const int i0[3] = {(int)(x - b * e) - 1, (int)(xy - x * e) - 1, (int)(m - xy * e) - 1};
-      cvox = (((int)b * D + i0[0]) * D + i0[1]) * D + i0[2];
-      cin = (int)corners_inside(i0, D);
-    }
-    ci = 0;
-  };
-  load_cells();
-  uint32_t ce = __shfl_sync(SG_FULL, cend, 0);
-  float acc[NC][NV], acct[TSDF ? NC : 1];
-#pragma unroll
-  for (int c = 0; c < NC; c++) {
-    if (TSDF) acct[c] = 0.0f;
-#pragma unroll
-    for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
-  }
-  const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  auto half = [&](const GradRecord *rec, uint32_t slot) {
-    return __ldg(reinterpret_cast<const float4 *>(rec + slot) + (lane & 1));
-  };
-  const uint32_t i2 = lane >> 1;
-  float4 fa = zero4, ft = zero4;
-  uint32_t nslot = 0;
-  int k = 0, nk = 0;
-  if (j + i2 < end) {
-    const uint32_t slot = __ldg(q.slot + j + i2);
-    fa = half(q.rec, slot);
-    if (TSDF) ft = half(q.rec_t, slot);
-    k = q.rays.ray(slot);
-  }
-  if (j + 16 + i2 < end) nslot = __ldg(q.slot + j + 16 + i2);
-  for (; j < end; j += 16) {
-    float gv[4][NV];  // the rays' G rows
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const float *row = q.ray_g + (size_t)__shfl_sync(SG_FULL, k, 2 * (4 * t + g)) * C + ch;
-      if (C == 16) {
-        const float4 x = __ldg(reinterpret_cast<const float4 *>(row));
-        gv[t][0] = x.x, gv[t][1] = x.y, gv[t][2] = x.z, gv[t][NV - 1] = x.w;
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; v++) gv[t][v] = __ldg(row + v);
+  // one stretch a warp, or, where they are long, eight shorter ones a grid
+  // apart: they take the warps unequal times (27 M samples 3.85 -> 3.73 ms a pass
+  // and reduction; starting more CTAs instead cost 3 us a class on 2 M)
+  const long warps = (long)gridDim.x * (blockDim.x >> 5), even = (P1 - P0 + warps - 1) / warps;
+  const long Q = max(even > 256 ? (even + 7) / 8 : even, 32l);
+  long pa = P0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Q;
+#pragma unroll 1
+  for (; pa < P1; pa += warps * Q) {
+    int u = __ldg(q.heads + pa);
+    const int ub = pa + Q < P1 ? __ldg(q.heads + pa + Q) : hi;
+    if (u >= ub) continue;
+    uint32_t j = __ldg(q.ustart + u);
+    const uint32_t end = __ldg(q.ustart + ub);
+    // 32 cells at a time, one a lane: lower corner's voxel, corners inside, end
+    int cvox = 0, cin = 0, cend = 0, ci = 0;
+    auto load_cells = [&]() {
+      if (u + lane < ub) {
+        const uint32_t m = __ldg(q.ukey + u + lane) - (uint32_t)cls * q.keys.cls, e = (uint32_t)D + 1;
+        cend = __ldg(q.ustart + u + lane + 1);
+        const uint32_t xy = q.by_edge.div(m), x = q.by_edge.div(xy), b = q.by_edge.div(x);
+        const int i0[3] = {(int)(x - b * e) - 1, (int)(xy - x * e) - 1, (int)(m - xy * e) - 1};
+        cvox = (((int)b * D + i0[0]) * D + i0[1]) * D + i0[2];
+        cin = (int)corners_inside(i0, D);
       }
-    }
-    float4 nfa = zero4, nft = zero4;
-    if (j + 16 + i2 < end) {
-      nfa = half(q.rec, nslot);
-      if (TSDF) nft = half(q.rec_t, nslot);
-      nk = q.rays.ray(nslot);
-    }
-    if (j + 32 + i2 < end) nslot = __ldg(q.slot + j + 32 + i2);
+      ci = 0;
+    };
+    load_cells();
+    uint32_t ce = __shfl_sync(SG_FULL, cend, 0);
+    float acc[NC][NV], acct[TSDF ? NC : 1];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const int src = 2 * (4 * t + g) + h;
-      float a[4] = {__shfl_sync(SG_FULL, fa.x, src), __shfl_sync(SG_FULL, fa.y, src), __shfl_sync(SG_FULL, fa.z, src),
-                    __shfl_sync(SG_FULL, fa.w, src)};
-      float at[4];
-      if (TSDF) {
-        at[0] = __shfl_sync(SG_FULL, ft.x, src), at[1] = __shfl_sync(SG_FULL, ft.y, src);
-        at[2] = __shfl_sync(SG_FULL, ft.z, src), at[3] = __shfl_sync(SG_FULL, ft.w, src);
+    for (int c = 0; c < NC; c++) {
+      if (TSDF) acct[c] = 0.0f;
+#pragma unroll
+      for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
+    }
+    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto half = [&](const GradRecord *rec, uint32_t slot) {
+      return __ldg(reinterpret_cast<const float4 *>(rec + slot) + (lane & 1));
+    };
+    const uint32_t i2 = lane >> 1;
+    float4 fa = zero4, ft = zero4;
+    uint32_t nslot = 0;
+    int k = 0, nk = 0;
+    if (j + i2 < end) {
+      const uint32_t slot = __ldg(q.slot + j + i2);
+      fa = half(q.rec, slot);
+      if (TSDF) ft = half(q.rec_t, slot);
+      k = q.rays.ray(slot);
+    }
+    if (j + 16 + i2 < end) nslot = __ldg(q.slot + j + 16 + i2);
+    for (; j < end; j += 16) {
+      float gv[4][NV];  // the rays' G rows
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const float *row = q.ray_g + (size_t)__shfl_sync(SG_FULL, k, 2 * (4 * t + g)) * C + ch;
+        if (C == 16) {
+          const float4 x = __ldg(reinterpret_cast<const float4 *>(row));
+          gv[t][0] = x.x, gv[t][1] = x.y, gv[t][2] = x.z, gv[t][NV - 1] = x.w;
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; v++) gv[t][v] = __ldg(row + v);
+        }
       }
-      if (C == 3) {  // the lane's own corner
-        a[0] = (l8 & 2) ? ((l8 & 1) ? a[3] : a[2]) : ((l8 & 1) ? a[1] : a[0]);
-        if (TSDF) at[0] = (l8 & 2) ? ((l8 & 1) ? at[3] : at[2]) : ((l8 & 1) ? at[1] : at[0]);
+      float4 nfa = zero4, nft = zero4;
+      if (j + 16 + i2 < end) {
+        nfa = half(q.rec, nslot);
+        if (TSDF) nft = half(q.rec_t, nslot);
+        nk = q.rays.ray(nslot);
       }
-      const uint32_t r = j + 4 * t + g, past = min(j + 4 * t + 4, end);
-      bool open = r < end;  // the lanes' record waits for its cell
-      while (true) {
-        if (open && r < ce) {
-          open = false;
+      if (j + 32 + i2 < end) nslot = __ldg(q.slot + j + 32 + i2);
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int src = 2 * (4 * t + g) + h;
+        float a[4] = {__shfl_sync(SG_FULL, fa.x, src), __shfl_sync(SG_FULL, fa.y, src), __shfl_sync(SG_FULL, fa.z, src),
+                      __shfl_sync(SG_FULL, fa.w, src)};
+        float at[4];
+        if (TSDF) {
+          at[0] = __shfl_sync(SG_FULL, ft.x, src), at[1] = __shfl_sync(SG_FULL, ft.y, src);
+          at[2] = __shfl_sync(SG_FULL, ft.z, src), at[3] = __shfl_sync(SG_FULL, ft.w, src);
+        }
+        if (C == 3) {  // the lane's own corner
+          a[0] = (l8 & 2) ? ((l8 & 1) ? a[3] : a[2]) : ((l8 & 1) ? a[1] : a[0]);
+          if (TSDF) at[0] = (l8 & 2) ? ((l8 & 1) ? at[3] : at[2]) : ((l8 & 1) ? at[1] : at[0]);
+        }
+        const uint32_t r = j + 4 * t + g, past = min(j + 4 * t + 4, end);
+        bool open = r < end;  // the lanes' record waits for its cell
+        while (true) {
+          if (open && r < ce) {
+            open = false;
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+              if (TSDF) acct[c] += at[c];
+#pragma unroll
+              for (int v = 0; v < NV; v++) acc[c][v] = __fmaf_rn(a[c], gv[t][v], acc[c][v]);
+            }
+          }
+          if (ce > past) break;
+          // the end of a cell
+          __syncwarp();
+          const int at0 = __shfl_sync(SG_FULL, cvox, ci), in = __shfl_sync(SG_FULL, cin, ci);
+          const bool add = (in >> cr1) & 1;
+          float *gp = q.grad_feat + (long)(at0 + at1) * C + ch;
+          if constexpr (C == 16) {
+            float s2[2][4], s1[4], t2[2], t1 = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+#pragma unroll
+              for (int v = 0; v < 4; v++) {
+                const float keep = (g & 2) ? acc[2 + c][v] : acc[c][v], send = (g & 2) ? acc[c][v] : acc[2 + c][v];
+                s2[c][v] = keep + __shfl_xor_sync(SG_FULL, send, 16);
+              }
+              if (TSDF) {
+                const float keep = (g & 2) ? acct[2 + c] : acct[c], send = (g & 2) ? acct[c] : acct[2 + c];
+                t2[c] = keep + __shfl_xor_sync(SG_FULL, send, 16);
+              }
+            }
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+              s1[v] = ((g & 1) ? s2[1][v] : s2[0][v]) + __shfl_xor_sync(SG_FULL, (g & 1) ? s2[0][v] : s2[1][v], 8);
+            if (TSDF) t1 = ((g & 1) ? t2[1] : t2[0]) + __shfl_xor_sync(SG_FULL, (g & 1) ? t2[0] : t2[1], 8);
+            if (add) {
+              red_add_f32x4(gp, s1[0], s1[1], s1[2], s1[3]);
+              if (TSDF && (l8 & 3) == 0) atomicAdd(q.grad_tsdf + (long)(at0 + at1), t1);
+            }
+          } else {
+            float v[4] = {acc[0][0], acc[0][1], acc[0][NV - 1], TSDF ? acct[0] : 0.0f};
+#pragma unroll
+            for (int k = 0; k < (TSDF ? 4 : 3); k++) {
+              v[k] += __shfl_xor_sync(SG_FULL, v[k], 16);
+              v[k] += __shfl_xor_sync(SG_FULL, v[k], 8);
+            }
+            if (add) {  // lanes of the four groups: a channel each, the TSDF gradient
+              if (g < 3) atomicAdd(gp + g, g == 0 ? v[0] : (g == 1 ? v[1] : v[2]));
+              else if (TSDF) atomicAdd(q.grad_tsdf + (long)(at0 + at1), v[3]);
+            }
+          }
 #pragma unroll
           for (int c = 0; c < NC; c++) {
-            if (TSDF) acct[c] += at[c];
+            if (TSDF) acct[c] = 0.0f;
 #pragma unroll
-            for (int v = 0; v < NV; v++) acc[c][v] = __fmaf_rn(a[c], gv[t][v], acc[c][v]);
+            for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
           }
+          if (++u == ub) {
+            ce = 0xffffffffu;  // the records are done
+            break;
+          }
+          if (++ci == 32) load_cells();
+          ce = __shfl_sync(SG_FULL, cend, ci);
         }
-        if (ce > past) break;
-        // the end of a cell
-        __syncwarp();
-        const int at0 = __shfl_sync(SG_FULL, cvox, ci), in = __shfl_sync(SG_FULL, cin, ci);
-        const bool add = (in >> cr1) & 1;
-        float *gp = q.grad_feat + (long)(at0 + at1) * C + ch;
-        if constexpr (C == 16) {
-          float s2[2][4], s1[4], t2[2], t1 = 0.0f;
-#pragma unroll
-          for (int c = 0; c < 2; c++) {
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-              const float keep = (g & 2) ? acc[2 + c][v] : acc[c][v], send = (g & 2) ? acc[c][v] : acc[2 + c][v];
-              s2[c][v] = keep + __shfl_xor_sync(SG_FULL, send, 16);
-            }
-            if (TSDF) {
-              const float keep = (g & 2) ? acct[2 + c] : acct[c], send = (g & 2) ? acct[c] : acct[2 + c];
-              t2[c] = keep + __shfl_xor_sync(SG_FULL, send, 16);
-            }
-          }
-#pragma unroll
-          for (int v = 0; v < 4; v++)
-            s1[v] = ((g & 1) ? s2[1][v] : s2[0][v]) + __shfl_xor_sync(SG_FULL, (g & 1) ? s2[0][v] : s2[1][v], 8);
-          if (TSDF) t1 = ((g & 1) ? t2[1] : t2[0]) + __shfl_xor_sync(SG_FULL, (g & 1) ? t2[0] : t2[1], 8);
-          if (add) {
-            red_add_f32x4(gp, s1[0], s1[1], s1[2], s1[3]);
-            if (TSDF && (l8 & 3) == 0) atomicAdd(q.grad_tsdf + (long)(at0 + at1), t1);
-          }
-        } else {
-          float v[4] = {acc[0][0], acc[0][1], acc[0][NV - 1], TSDF ? acct[0] : 0.0f};
-#pragma unroll
-          for (int k = 0; k < (TSDF ? 4 : 3); k++) {
-            v[k] += __shfl_xor_sync(SG_FULL, v[k], 16);
-            v[k] += __shfl_xor_sync(SG_FULL, v[k], 8);
-          }
-          if (add) {  // lanes of the four groups: a channel each, the TSDF gradient
-            if (g < 3) atomicAdd(gp + g, g == 0 ? v[0] : (g == 1 ? v[1] : v[2]));
-            else if (TSDF) atomicAdd(q.grad_tsdf + (long)(at0 + at1), v[3]);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          if (TSDF) acct[c] = 0.0f;
-#pragma unroll
-          for (int v = 0; v < NV; v++) acc[c][v] = 0.0f;
-        }
-        if (++u == ub) {
-          ce = 0xffffffffu;  // the records are done
-          break;
-        }
-        if (++ci == 32) load_cells();
-        ce = __shfl_sync(SG_FULL, cend, ci);
       }
+      fa = nfa;
+      ft = nft;
+      k = nk;
     }
-    fa = nfa;
-    ft = nft;
-    k = nk;
   }
 }
 
