@@ -156,12 +156,14 @@ def integrate_in_box(occupied_vol, num_occ_voxel, cam_intr, cam_pose, color_ims,
 
 def pack_colors(colors):
     """floor(b 256^2 + g 256 + r) of colour images [n, >= 3, h, w], [n, h, w]
-    (voxel_encoding_helper.py:213): in one pass where the images are float32
-    on the GPU, contiguous and without gradient (the seven elementwise passes
-    of the expression took 28 of a 128^3 build's 202 us of device time)."""
-    if (colors.is_cuda and colors.dtype == torch.float32 and colors.dim() == 4 and colors.shape[1] >= 3
-            and colors.is_contiguous() and colors.numel() > 0
-            and not (colors.requires_grad and torch.is_grad_enabled())):
+    (voxel_encoding_helper.py:213): in one pass where the images are plain
+    contiguous float32 tensors on the GPU and neither gradients nor a trace or
+    function transform are recorded (the seven elementwise passes of the
+    expression took 28 of a 128^3 build's 202 us of device time)."""
+    if (type(colors) is torch.Tensor and colors.is_cuda and colors.dtype == torch.float32 and colors.dim() == 4
+            and colors.shape[1] >= 3 and colors.is_contiguous() and colors.numel() > 0
+            and not torch.is_grad_enabled() and not torch.jit.is_tracing()
+            and torch._C._functorch.peek_interpreter_stack() is None):
         n, ch, h, w = colors.shape
         with torch.cuda.device(colors.device):
             out = torch.empty((n, h, w), dtype=torch.float32, device=colors.device)

@@ -20,7 +20,13 @@ def test_pack_colors(shape, shift):
     c = buf[shift:shift + n].view(shape)
     ref = torch.floor(c[:, 2] * 256.0 * 256.0 + c[:, 1] * 256.0 + c[:, 0])
     for x in (c, c.transpose(2, 3).contiguous().transpose(2, 3)):  # as given, and by the expression
-        assert torch.equal(VE.pack_colors(x).nan_to_num(-1.0, -2.0, -3.0), ref.nan_to_num(-1.0, -2.0, -3.0))
+        with torch.no_grad():
+            assert torch.equal(VE.pack_colors(x).nan_to_num(-1.0, -2.0, -3.0), ref.nan_to_num(-1.0, -2.0, -3.0))
+    leaf = c.clone().requires_grad_()
+    assert VE.pack_colors(leaf).requires_grad
+    with torch.no_grad():
+        many = torch.vmap(VE.pack_colors)(torch.stack([c, c]))
+    assert torch.equal(many[1].nan_to_num(-1.0, -2.0, -3.0), ref.nan_to_num(-1.0, -2.0, -3.0))
     assert torch.equal(VE.pack_colors(c.double()).float().nan_to_num(), torch.floor(
         c.double()[:, 2] * 256.0 * 256.0 + c.double()[:, 1] * 256.0 + c.double()[:, 0]).float().nan_to_num())
 
