@@ -15,7 +15,7 @@
 // per sample wrote its 16 channels 64 bytes apart from its neighbours': the
 // L1 data path was 73 % busy).  Sample -> ray -> frame by multiplication (two
 // 64-bit divisions a sample were a third of the 1- and 3-channel gathers).
-// 12.6 M samples x 16 channels of 256^3: 1.02 -> 0.74 ms; 16.8 M samples x 3
+// 12.6 M samples x 16 channels of 256^3: 1.02 -> 0.57 ms; 16.8 M samples x 3
 // channels 122 -> 121 us, x 1 90 -> 78 us.
 //
 // grid_scatter_kernel (the adjoint): 8 lanes per ray walk the ray's samples in
@@ -27,7 +27,12 @@
 // depth-sorted and cluster in the few hit voxels, so a flush carries many
 // samples.  A warp per ray, its lanes over the 8 C slots, took 88 warp
 // instructions a sample at C = 16 (staging through shared memory): 12.6 M
-// samples 1.16 -> 0.96 ms, at C = 1 0.69 -> 0.34 ms; now bound by the atomics.
+// samples 1.16 -> 0.68 ms, at C = 1 0.69 -> 0.34 ms; now bound by the atomics.
+//
+// Registers (both wait on memory most of the time): 16 channels, gather at 5 /
+// 6 / 8 CTAs an SM 0.74 / 0.57 / 0.58 ms, adjoint at 2 / 4 / 5 0.96 / 0.68 / 0.83;
+// one and three channels are best without a bound (gather 78 and 121 us against
+// 86 and 125 at 6, adjoint 344 against 352 at 4): 0 leaves the choice to the compiler.
 //
 // mode 1 turns a gathered normalised TSDF t (C == 1) into a density
 // sigma = sigmoid(-t * scale / s) / s  (scale = truncation margin in metres,
@@ -78,7 +83,7 @@ struct FrameGeom {
 
 // VEC: grid and output are 16-byte aligned (C a multiple of 4).
 template <int C, bool VEC>
-__global__ void __launch_bounds__(256) grid_gather_kernel(GatherParams p) {
+__global__ void __launch_bounds__(256, VEC && C >= 8 ? 6 : 0) grid_gather_kernel(GatherParams p) {
   constexpr int L = VEC ? C / 4 : 1;  // lanes of a sample
   const long n = p.R * p.S;
   const int lane = lane_id();
@@ -196,7 +201,7 @@ __device__ __forceinline__ void scatter_flush(const ScatterParams &p, long cell,
 }
 
 template <int C, bool VEC>
-__global__ void __launch_bounds__(256) grid_scatter_kernel(ScatterParams p) {
+__global__ void __launch_bounds__(256, C >= 8 ? 4 : 0) grid_scatter_kernel(ScatterParams p) {
   const int cr = lane_id() & 7;  // corner, and sample of a step of 8
   FrameGeom g;
   const long nw = ((long)gridDim.x * blockDim.x) >> 5;
