@@ -255,8 +255,10 @@ struct CompKeep {
   int idx[kMaxPos];  // sample, with bit 30: counts, bit 31: its gradient is written
 };
 
+// CTAs an SM 4 / 5 / 6 (131072 rays x 96): 3 channels 174 / 156 / 158 us, 5 channels
+// 334 / 315 / 315, 16 channels 270 / 264 / 283.
 template <int V>
-__global__ void __launch_bounds__(256) composite_bwd_kernel(CompParams p) {
+__global__ void __launch_bounds__(256, 5) composite_bwd_kernel(CompParams p) {
   extern __shared__ __align__(16) unsigned char s_comp[];
   const int lane = lane_id(), w8 = threadIdx.x >> 5;
   float *s_z = reinterpret_cast<float *>(s_comp) + w8 * (kMaxPos + 64);
