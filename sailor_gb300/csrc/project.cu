@@ -639,8 +639,12 @@ extern "C" int sg_project_gather(const SgProjGather *a, sg_stream_t stream) {
       };
       g.rows = fits(4) ? 4 : (fits(2) ? 2 : 1);
     }
+    // 32-bit offsets hold every step of a map: images, channels (one channel
+    // is never stepped over), rows and columns with one beyond the edges
     auto mag = [](long long v) { return (double)(v < 0 ? -v : v); };
-    if (mag(m.stride[0]) * a->n_images + mag(m.stride[2]) * (m.H + 1.0) + mag(m.stride[3]) * (m.W + 1.0) + m.C >= 2147483647.0)
+    if (mag(m.stride[0]) * a->n_images + (m.C > 1 ? mag(m.stride[1]) * m.C : 0.0) + mag(m.stride[2]) * (m.H + 1.0) +
+            mag(m.stride[3]) * (m.W + 1.0) >=
+        2147483647.0)
       small = false;
   }
   p.psdf_map = a->psdf_map;
