@@ -470,7 +470,10 @@ __global__ void __launch_bounds__(256, 4) project_gather_kernel(ProjGatherParams
       const GatherMap &m = p.maps[mi];
       if (m.H != fh || m.W != fw) {
         f = footprint(m.H, m.W, gx, gy);
-        if (!live) f.mask = 0;
+        // past the last item: no corner, and texel (0, 0), which the lane groups
+        // read beside their last item's (the footprint of (-2, -2) has a corner
+        // in an image of two or three pixels an edge, from texel (-1, -1) on)
+        if (!live) f.mask = f.x0 = f.y0 = 0;
         fh = m.H;
         fw = m.W;
         staged = false;
