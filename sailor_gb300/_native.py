@@ -12,6 +12,7 @@ import torch
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsailor_gb300.so")
 
+SG_ERR_UNSUPPORTED = 4
 SG_FLAG_HIT_OVERFLOW = 1
 SG_FLAG_TREE_CAPACITY = 2
 SG_FLAG_RECORD_CAPACITY = 4

@@ -49,32 +49,53 @@ def _cams(K, R, T, n_images):
 CHANNELS_LAST_FROM = 0.25
 
 
-def _map(a, img, N_pts):
-    """SgFeatureMap of a [n_images, C, H, W] map, its [n_images, N, C] output,
-    and what has to live until the launch."""
-    if img.dim() != 4:
-        raise RuntimeError("feature maps must be [n_images, C, H, W]")
-    _f32(img, "feature map")
+def _channels_last(img):
+    """A copy of a [n, C, H, W] map in channels-last order ([n, H, W, C]
+    contiguous), or None where the kernel does not take the size or the memory
+    has no room for one (the map is then gathered through its strides)."""
     n, Cm, H, W = img.shape
-    out = torch.empty((n, N_pts, Cm), device=img.device)
-    m = N.SgFeatureMap()
-    src, strides = img, img.stride()
-    # A thread per item walks the channels of an NCHW map through scattered
-    # 4-byte loads; rows of a channels-last one are read whole.  Measured on 4
-    # images of 512^2 pixels and 68 channels, direct against rewritten: 104 and
-    # 203 us at 0.11 points per pixel, 232 and 222 at 0.25, 803 and 292 at 1,
-    # 2369 and 486 at 3.
-    if Cm > 4 and img.stride(1) != 1 and N_pts >= CHANNELS_LAST_FROM * H * W:
-        src = torch.empty((n, H, W, Cm), device=img.device)
-        N.check(N.lib.sg_channels_last(N.ptr(img), (C.c_longlong * 4)(*img.stride()), n, Cm, H, W, N.ptr(src),
-                                       N.stream()), "channels_last")
-        strides = (H * W * Cm, 1, W * Cm, Cm)
-    m.data = src.data_ptr()
-    for k in range(4):
-        m.stride[k] = strides[k]
-    m.C, m.H, m.W = Cm, H, W
-    m.out = out.data_ptr()
-    return m, out, src
+    try:
+        out = torch.empty((n, H, W, Cm), device=img.device)
+    except torch.OutOfMemoryError:
+        return None
+    rc = N.lib.sg_channels_last(N.ptr(img), (C.c_longlong * 4)(*img.stride()), n, Cm, H, W, N.ptr(out), N.stream())
+    if rc == N.SG_ERR_UNSUPPORTED:
+        return None
+    N.check(rc, "channels_last")
+    return out
+
+
+def _maps(a, imgs, N_pts):
+    """The [n_images, C, H, W] maps and their [n_images, N, C] outputs into the
+    arguments; returns the outputs, and what has to live until the launch."""
+    for img in imgs:
+        if img.dim() != 4:
+            raise RuntimeError("feature maps must be [n_images, C, H, W]")
+        _f32(img, "feature map")
+    # before any copy of a map, which can be done without
+    outs = [torch.empty((img.shape[0], N_pts, img.shape[1]), device=img.device) for img in imgs]
+    keep = []
+    for i, img in enumerate(imgs):
+        n, Cm, H, W = img.shape
+        src, strides = img, img.stride()
+        # A thread per item walks the channels of an NCHW map through scattered
+        # 4-byte loads; rows of a channels-last one are read whole.  Measured on 4
+        # images of 512^2 pixels and 68 channels, direct against rewritten: 104 and
+        # 203 us at 0.11 points per pixel, 232 and 222 at 0.25, 803 and 292 at 1,
+        # 2369 and 486 at 3.
+        if Cm > 4 and img.stride(1) != 1 and N_pts >= CHANNELS_LAST_FROM * H * W:
+            rows = _channels_last(img)
+            if rows is not None:
+                src, strides = rows, (H * W * Cm, 1, W * Cm, Cm)
+        m = a.maps[i]
+        m.data = src.data_ptr()
+        for k in range(4):
+            m.stride[k] = strides[k]
+        m.C, m.H, m.W = Cm, H, W
+        m.out = outs[i].data_ptr()
+        keep.append(src)
+    a.n_maps = len(imgs)
+    return outs, keep + list(imgs)
 
 
 def _launch(a, keep):
@@ -146,16 +167,10 @@ def forward_sample_feature(feats_geo, depths, feats_rgb, rgbs_n, xy, z):
     a = N.SgProjGather()
     a.grids_in, a.depth_in = g.data_ptr(), zz.data_ptr()
     a.n_images, a.num_points = n, Np
-    outs, keep = [], [g, zz]
-    for i, img in enumerate((feats_geo, depths, feats_rgb, rgbs_n)):
-        m, o, src = _map(a, img, Np)
-        a.maps[i] = m
-        outs.append(o)
-        keep += [img, src]
-    a.n_maps = 4
     psdf = torch.empty((n, Np, 1), device=g.device)
     a.psdf_map, a.psdf_clip, a.psdf_scale, a.psdf = 1, PSDF_CLIP, 1.0 / PSDF_CLIP, psdf.data_ptr()
-    _launch(a, keep)
+    outs, maps = _maps(a, (feats_geo, depths, feats_rgb, rgbs_n), Np)
+    _launch(a, [g, zz] + maps)
     return outs[0], outs[2], psdf, outs[3]
 
 
@@ -175,15 +190,9 @@ def project_sample_features(points, K, R, T, p_depths, n_views, feats_geo, depth
     if want_grids:
         grids = torch.empty((n, 2, Np), device=dev)
         a.grids = grids.data_ptr()
-    outs = []
-    for i, img in enumerate((feats_geo, depths, feats_rgb, rgbs_n)):
-        m, o, src = _map(a, img, Np)
-        a.maps[i] = m
-        outs.append(o)
-        keep += [img, src]
-    a.n_maps = 4
     psdf = torch.empty((n, Np, 1), device=dev)
     a.psdf_map, a.psdf_clip, a.psdf_scale, a.psdf = 1, PSDF_CLIP, 1.0 / PSDF_CLIP, psdf.data_ptr()
-    _launch(a, keep)
+    outs, maps = _maps(a, (feats_geo, depths, feats_rgb, rgbs_n), Np)
+    _launch(a, keep + maps)
     res_ = (depth, outs[0], outs[2], psdf, outs[3])
     return res_ + (grids,) if want_grids else res_

@@ -1,0 +1,48 @@
+"""GPU checks of the feature gather where channel-first maps are rewritten
+channels-last first: more images and channels than a grid dimension holds, and
+no memory left for a copy.  Same bits as the gather through the strides."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _args(n, C, H, W, n_pts, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    maps = [torch.rand((n, c, H, W), generator=g, device="cuda") for c in (C, 1, 1, 3)]
+    xy = torch.rand((n, n_pts, 1, 2), generator=g, device="cuda") * 2.2 - 1.1
+    return maps + [xy, torch.rand((n, 1, n_pts), generator=g, device="cuda")]
+
+
+def _direct(views, monkeypatch, args):
+    with monkeypatch.context() as mp:
+        mp.setattr(views, "CHANNELS_LAST_FROM", float("inf"))
+        return views.forward_sample_feature(*args)
+
+
+@pytest.mark.parametrize("n,C,H,W", [(70000, 32, 4, 4), (65535, 9, 3, 2), (1, 32 * 65535 + 40, 2, 2), (3, 33, 9, 8)])
+def test_any_number_of_images_and_channels(n, C, H, W, monkeypatch):
+    from sailor_gb300 import views
+    args = _args(n, C, H, W, H * W, C)
+    monkeypatch.setattr(views, "CHANNELS_LAST_FROM", 0.0)
+    rows = views._channels_last(args[0])
+    assert torch.equal(rows, args[0].permute(0, 2, 3, 1))
+    for a, b in zip(views.forward_sample_feature(*args), _direct(views, monkeypatch, args)):
+        assert torch.equal(a, b)
+
+
+def test_no_room_for_a_copy(monkeypatch):
+    from sailor_gb300 import views
+    args = _args(2, 64, 1536, 1536, 600000, 1)  # a map of 1.2 GB, 0.3 GB of output
+    ref = _direct(views, monkeypatch, args)
+    got = None
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 8e8) / total)
+    try:
+        assert views._channels_last(args[0]) is None
+        got = views.forward_sample_feature(*args)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)
