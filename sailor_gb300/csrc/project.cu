@@ -520,14 +520,12 @@ __global__ void __launch_bounds__(256, 4) project_gather_kernel(ProjGatherParams
 // cold (3.1 TB/s in and out; latency of the strided reads).
 constexpr int kClPix = 64, kClChan = 32;
 
-// n0, cb: the launch's first image and channel block.
 __global__ void __launch_bounds__(256) channels_last_kernel(const float *__restrict__ src, long sn, long sc, long sy,
-                                                            long sx, int n0, int cb, int C, int H, int W,
-                                                            float *__restrict__ dst) {
+                                                            long sx, int C, int H, int W, float *__restrict__ dst) {
   __shared__ float s[kClChan][kClPix + 1];
   const int HW = H * W;
-  const int p0 = blockIdx.x * kClPix, c0 = (cb + (int)blockIdx.y) * kClChan;
-  const long n = n0 + (long)blockIdx.z;
+  const int p0 = blockIdx.x * kClPix, c0 = blockIdx.y * kClChan;
+  const long n = blockIdx.z;
   const bool lin = sy == (long)W * sx;
 #pragma unroll
   for (int i = 0; i < kClPix * kClChan / 256; i++) {
@@ -673,16 +671,15 @@ extern "C" int sg_channels_last(const float *src, const long long *stride, int n
   if (n == 0) return SG_OK;
   if (!src || !stride || !dst) return SG_ERR_INVALID_ARG;
   const long hw = (long)H * W;
-  if (hw > INT_MAX - kClPix || C > INT_MAX - kClChan) return SG_ERR_UNSUPPORTED;
-  const int blocks = (C + kClChan - 1) / kClChan;
-  // a grid holds 65535 images and as many channel blocks
-  constexpr int kMost = 65535;
-  for (int n0 = 0; n0 < n; n0 += n - n0 < kMost ? n - n0 : kMost) {
-    for (int cb = 0; cb < blocks; cb += kMost) {
-      const dim3 g((unsigned)((hw + kClPix - 1) / kClPix), (unsigned)(blocks - cb < kMost ? blocks - cb : kMost),
-                   (unsigned)(n - n0 < kMost ? n - n0 : kMost));
-      channels_last_kernel<<<g, 256, 0, stream>>>(src, stride[0], stride[1], stride[2], stride[3], n0, cb, C, H, W, dst);
-    }
+  const long blocks = ((long)C + kClChan - 1) / kClChan;
+  constexpr int kMost = 65535;  // images and channel blocks of a grid
+  if (hw > INT_MAX - kClPix || blocks > kMost) return SG_ERR_UNSUPPORTED;
+  for (int n0 = 0; n0 < n;) {
+    const int k = n - n0 < kMost ? n - n0 : kMost;
+    const dim3 g((unsigned)((hw + kClPix - 1) / kClPix), (unsigned)blocks, (unsigned)k);
+    channels_last_kernel<<<g, 256, 0, stream>>>(src + n0 * stride[0], stride[0], stride[1], stride[2], stride[3], C, H, W,
+                                                dst + n0 * hw * C);
+    n0 += k;
   }
   SG_LAUNCH_CHECK();
   return SG_OK;

@@ -26,7 +26,10 @@ def test_any_number_of_images_and_channels(n, C, H, W, monkeypatch):
     args = _args(n, C, H, W, H * W, C)
     monkeypatch.setattr(views, "CHANNELS_LAST_FROM", 0.0)
     rows = views._channels_last(args[0])
-    assert torch.equal(rows, args[0].permute(0, 2, 3, 1))
+    if C <= 32 * 65535:
+        assert torch.equal(rows, args[0].permute(0, 2, 3, 1))
+    else:
+        assert rows is None  # gathered through its strides
     for a, b in zip(views.forward_sample_feature(*args), _direct(views, monkeypatch, args)):
         assert torch.equal(a, b)
 
