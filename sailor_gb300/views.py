@@ -44,9 +44,29 @@ def _cams(K, R, T, n_images):
     return K, R, T
 
 
-# Points per image, as a share of its pixels, from which a map that is not
-# channels-last is rewritten before the gather
-CHANNELS_LAST_FROM = 0.25
+# A thread per item walks the channels of a map that is not channels-last
+# through scattered 4-byte loads, near points sharing them; rows of a
+# channels-last map are read whole.  Rewriting costs a pass over the map and
+# about 10 us of calls, so it is done where the points outnumber
+# CHANNELS_LAST_FROM of the pixels by more the fewer channels there are
+# (C > 5 only), and the output is large enough to hide the calls.  Measured,
+# direct against rewritten, on samples along rays / on a raster of neighbouring
+# pixels, 4 images of 512^2:
+#   C   8: 1 point a pixel 160 and 160 /  66 and  87 us;  2: 309 and 214 / -
+#   C  16: 0.5             178 and 172 /  63 and  95;     1: 329 and 207 / 105 and 117
+#   C  32: 0.25            235 and 221 /  79 and 128;   0.5: 426 and 245 / 148 and 143
+#   C  68: 0.25            419 and 532 / 187 and 290;   0.5: 788 and 588 / 323 and 318
+#   C   5: 5 points a pixel 439 and 469; C 6: 2: 213 and 237, 3: 316 and 304
+# and, where the calls count, one image of 512^2, C 16: 0.5 (2^21 values) 50 and
+# 66 us, 1 (2^22) 87 and 65.  (Samples along rays: two such maps a call.)
+CHANNELS_LAST_FROM = 0.5
+CHANNELS_LAST_WORK = 1 << 22
+
+
+def _rewrites(n, Cm, pixels, N_pts):
+    """Whether n maps of Cm channels, not channels-last, are rewritten for N_pts points each."""
+    return (Cm > 5 and N_pts >= CHANNELS_LAST_FROM * pixels * max(1.0, 32.0 / Cm)
+            and n * N_pts * Cm >= CHANNELS_LAST_WORK)
 
 
 def _channels_last(img):
@@ -78,12 +98,7 @@ def _maps(a, imgs, N_pts):
     for i, img in enumerate(imgs):
         n, Cm, H, W = img.shape
         src, strides = img, img.stride()
-        # A thread per item walks the channels of an NCHW map through scattered
-        # 4-byte loads; rows of a channels-last one are read whole.  Measured on 4
-        # images of 512^2 pixels and 68 channels, direct against rewritten: 104 and
-        # 203 us at 0.11 points per pixel, 232 and 222 at 0.25, 803 and 292 at 1,
-        # 2369 and 486 at 3.
-        if Cm > 4 and img.stride(1) != 1 and N_pts >= CHANNELS_LAST_FROM * H * W:
+        if img.stride(1) != 1 and _rewrites(n, Cm, H * W, N_pts):
             rows = _channels_last(img)
             if rows is not None:
                 src, strides = rows, (H * W * Cm, 1, W * Cm, Cm)

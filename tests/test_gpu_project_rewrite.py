@@ -25,6 +25,7 @@ def test_any_number_of_images_and_channels(n, C, H, W, monkeypatch):
     from sailor_gb300 import views
     args = _args(n, C, H, W, H * W, C)
     monkeypatch.setattr(views, "CHANNELS_LAST_FROM", 0.0)
+    monkeypatch.setattr(views, "CHANNELS_LAST_WORK", 0)
     rows = views._channels_last(args[0])
     if C <= 32 * 65535:
         assert torch.equal(rows, args[0].permute(0, 2, 3, 1))
