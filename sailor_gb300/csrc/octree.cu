@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(kTravThreads, 6) octree_descend_kernel(const _
         if (over & ((z == 32 ? 0u : (1u << z)) - (1u << a))) redo = true;
       }
     }
+    __syncwarp();  // the lanes' entries are in the rows before a lane rewrites one and reads it back
     if (lane < rays && (redo || fc > p.Wf)) fc = descend_in_row(p, m, r0 + lane, s_vs[w] + lane, s_st[w] + lane);
     __syncwarp();
     const int most = __reduce_max_sync(SG_FULL, lane < rays ? fc : 0);
