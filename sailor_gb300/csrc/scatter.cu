@@ -201,6 +201,28 @@ __global__ void __launch_bounds__(256) det_cells_kernel(const uint32_t *__restri
   }
 }
 
+// The one addition a class makes to grid values.  A global float reduction
+// takes operands and results below 2^-126 as 0; where the terms are 2^-101 and
+// more that cannot show (a subnormal grid value is less than half a unit in
+// their last place, and two such values that cancel leave 2^-125 or 0).  Smaller
+// terms are added by load and store: no other lane adds to the value in this
+// launch.
+constexpr float kReduceFrom = 3.9443045e-31f;  // 2^-101
+__device__ __forceinline__ void add_once(float *g, float a) {
+  if (fabsf(a) >= kReduceFrom) atomicAdd(g, a);
+  else if (a != 0.0f) *g += a;
+}
+__device__ __forceinline__ void add_once4(float *g, const float (&a)[4]) {
+  const float lo = fminf(fminf(fabsf(a[0]), fabsf(a[1])), fminf(fabsf(a[2]), fabsf(a[3])));
+  if (lo >= kReduceFrom) {
+    red_add_f32x4(g, a[0], a[1], a[2], a[3]);
+  } else {
+    float4 *q = reinterpret_cast<float4 *>(g);
+    const float4 v = *q;
+    *q = make_float4(v.x + a[0], v.y + a[1], v.z + a[2], v.w + a[3]);
+  }
+}
+
 // Cells of parity class cls.  A warp takes a stretch of the class's sorted
 // records, cut at cell boundaries (the cells that start in the stretch), and
 // walks it 16 records at a time: lanes 2 i and 2 i + 1 hold record i's two
@@ -352,8 +374,8 @@ __global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, in
               s1[v] = ((g & 1) ? s2[1][v] : s2[0][v]) + __shfl_xor_sync(SG_FULL, (g & 1) ? s2[0][v] : s2[1][v], 8);
             if (TSDF) t1 = ((g & 1) ? t2[1] : t2[0]) + __shfl_xor_sync(SG_FULL, (g & 1) ? t2[0] : t2[1], 8);
             if (add) {
-              red_add_f32x4(gp, s1[0], s1[1], s1[2], s1[3]);
-              if (TSDF && (l8 & 3) == 0) atomicAdd(q.grad_tsdf + (long)(at0 + at1), t1);
+              add_once4(gp, s1);
+              if (TSDF && (l8 & 3) == 0) add_once(q.grad_tsdf + (long)(at0 + at1), t1);
             }
           } else {
             float v[4] = {acc[0][0], acc[0][1], acc[0][NV - 1], TSDF ? acct[0] : 0.0f};
@@ -363,8 +385,8 @@ __global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, in
               v[k] += __shfl_xor_sync(SG_FULL, v[k], 8);
             }
             if (add) {  // lanes of the four groups: a channel each, the TSDF gradient
-              if (g < 3) atomicAdd(gp + g, g == 0 ? v[0] : (g == 1 ? v[1] : v[2]));
-              else if (TSDF) atomicAdd(q.grad_tsdf + (long)(at0 + at1), v[3]);
+              if (g < 3) add_once(gp + g, g == 0 ? v[0] : (g == 1 ? v[1] : v[2]));
+              else if (TSDF) add_once(q.grad_tsdf + (long)(at0 + at1), v[3]);
             }
           }
 #pragma unroll
