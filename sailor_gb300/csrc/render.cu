@@ -616,10 +616,14 @@ __device__ __forceinline__ void scatter_block(const RenderParams &p, int b, cons
     const long v = ((long)x >> 8) + at1;
     if (fown) {
       const float k = sm.cw[j * 9 + cr];
-      if (k != 0.0f) {
-        float *g = p.grad_feat + v * C + ch;
-        if (C == 16) red_add_f32x4(g, k * G[0], k * G[1], k * G[2], k * G[3]);
-        else atomicAdd(g, k * G[0]);
+      float *g = p.grad_feat + v * C + ch;
+      // terms of 0 are left out; 0 x NaN and 0 x infinity are not 0
+      if constexpr (C == 16) {
+        const float t0 = k * G[0], t1 = k * G[1], t2 = k * G[2], t3 = k * G[3];
+        if (t0 != 0.0f || t1 != 0.0f || t2 != 0.0f || t3 != 0.0f) red_add_f32x4(g, t0, t1, t2, t3);
+      } else {
+        const float t0 = k * G[0];
+        if (t0 != 0.0f) atomicAdd(g, t0);
       }
     }
     if (town) {
