@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256, VEC && C >= 8 ? 6 : 0) grid_gather_kernel
       tap_frac(g.bmin, g.vs, g.inv_vs, pt, i0, f);
       in = corners_inside(i0, p.D);
       off = (((long)g.b * p.D + i0[0]) * p.D + i0[1]) * p.D + i0[2];
+      if (in == 0u) f[0] = f[1] = f[2] = 0.0f;  // they may be NaN, and weigh zeros below
     }
     if constexpr (L == 1) {
       float acc[C];
