@@ -69,6 +69,29 @@ def capacity_layout(targets):
     return order, rb, ray_slices, groups
 
 
+def pack_pays(samples, frames, Dt, rate, C):
+    """Whether packing the fields near the tree's nodes (sg_pack_fields) before
+    a render of so many samples (rays x S, of all targets) is faster than
+    reading the grids: for (forward, backward, train_step).
+
+    A pack reads the voxels of the nodes' bricks and one around them; scenes of
+    closed surfaces have about 1.25 Dt^2 nodes a frame, whence V below (17 us
+    per million voxels at 16 channels, 10 at 3, 8 us at least).  What it gives
+    back per million samples of camera rays: forward 7 us (3 channels: 3),
+    adjoint 14 (7).  train_step packs beside the intersection.  Grids / packed
+    with the pack, us:
+      forward, C = 16: 1 frame of 256^3, 16384 rays x 96 (1.6 M samples) 36 / 46,
+        2^18 x 64 (16.8 M) 312 / 187; 4 frames 1.6 M 33 / 108, 12.6 M 185 / 176;
+        C = 3, 4 frames 12.6 M 126 / 139, 16.8 M 187 / 191
+      backward, C = 16: 1 frame 1.6 M 78 / 73; 4 frames 4.2 M 179 / 203, 12.6 M
+        408 / 316
+      train_step, C = 16 (graph): 1 frame 0.4 M 642 / 634; 4 frames 1.6 M 1102 /
+        1129, 4.2 M 1207 / 1206, 12.6 M 1325 / 1263
+    Without a rule 256 rays over 4 such frames took 105 us for 10."""
+    V = frames * Dt ** 2 * (rate + 2) ** 3
+    return (samples >= (3 if C == 16 else 4) * V + (1 << 20), samples >= 1.5 * V + (1 << 18), samples >= V)
+
+
 class BatchPipeline:
     def __init__(self, view_hw, targets, D=256, rate=8, C=16, W_hits=64, train_tsdf=False, target_widths=None,
                  device="cuda", deterministic=True, record_capacity=None):
@@ -186,13 +209,18 @@ class BatchPipeline:
         self.grad_feat = torch.zeros((B, D, D, D, C), **f32)
         self.grad_tsdf = torch.zeros((B, D, D, D), **f32)
         # (colour, TSDF) of the voxels near the tree's nodes, packed from the
-        # grids at the start of every render (sg_pack_fields): 18-25 us for a
-        # frame or three, which the render gains back from about 4000 rays of
-        # 96 samples on (forward 40 us with it, 37 without; their adjoint 237,
-        # 254; at 16000 rays 59, 104 and 311, 449)
+        # grids at the start of a render where that pays (pack_pays): 16 bytes a
+        # voxel, or None -- no render of this size is packed, or there is no
+        # room; set to None (before a capture) it is freed, and the renders
+        # read the grids: the same bits
+        self._packs = dict(zip(("forward", "backward", "train"),
+                               pack_pays(sum(n * s_ for _, n, s_ in self.targets), B, self.Dt, rate, C)))
         self.packed = None
-        if C in (3, 16) and rate & (rate - 1) == 0:
-            self.packed = torch.empty((B, D, D, D, 4), **f32)
+        if C in (3, 16) and rate & (rate - 1) == 0 and any(self._packs.values()):
+            try:
+                self.packed = torch.empty((B, D, D, D, 4), **f32)
+            except torch.OutOfMemoryError:
+                pass
         # brick map of the tree the gradients were last accumulated over (-1:
         # none): outside its nodes' bricks and their neighbours the gradient
         # grids are 0, so train_step clears only those (sg_zero_near_nodes)
@@ -340,17 +368,20 @@ class BatchPipeline:
                                             N.ptr(self.status), N.stream()), "intersect_segments")
         self._mark("intersect")
 
-    def _pack(self):
+    def _pack(self, use):
         """The fields near the tree's nodes into self.packed, for the render
-        that follows (the grids may have changed since the last one)."""
-        if self.packed is not None:
-            N.check(N.lib.sg_pack_fields(C.byref(self.tree), C.byref(self.seg), C.byref(self.args),
-                                         N.ptr(self.packed), N.stream()), "pack_fields")
+        that follows (the grids may have changed since the last one); None
+        where that render reads the grids."""
+        if self.packed is None or not self._packs[use]:
+            return None
+        N.check(N.lib.sg_pack_fields(C.byref(self.tree), C.byref(self.seg), C.byref(self.args),
+                                     N.ptr(self.packed), N.stream()), "pack_fields")
+        return self.packed
 
     def forward(self, out_z=None, out_node=None):
-        self._pack()
+        packed = self._pack("forward")
         N.check(N.lib.sg_render_packed_fwd(C.byref(self.tree), C.byref(self.seg), C.byref(self.args),
-                                           N.ptr(self.packed), N.ptr(self.out_rgb), N.ptr(self.out_depth),
+                                           N.ptr(packed), N.ptr(self.out_rgb), N.ptr(self.out_depth),
                                            N.ptr(self.out_ws), N.ptr(self.out_alpha), N.ptr(out_z),
                                            N.ptr(out_node), N.stream()), "render_fwd")
         self._mark("forward")
@@ -362,9 +393,9 @@ class BatchPipeline:
             self.grad_feat.zero_()
             self.grad_tsdf.zero_()  # both, so one brick map describes both grids
         self._mark("grad_prep")
-        self._pack()
+        packed = self._pack("backward")
         N.check(N.lib.sg_render_packed_bwd(C.byref(self.tree), C.byref(self.seg), C.byref(self.args),
-                                           N.ptr(self.packed), N.ptr(g_rgb), N.ptr(g_depth), N.ptr(g_ws),
+                                           N.ptr(packed), N.ptr(g_rgb), N.ptr(g_depth), N.ptr(g_ws),
                                            N.ptr(g_alpha), N.ptr(self.grad_feat),
                                            N.ptr(self.grad_tsdf) if tsdf_grad else None, N.ptr(grad_sigma),
                                            N.ptr(grad_rgb), N.stream()), "render_bwd")
@@ -397,17 +428,20 @@ class BatchPipeline:
                 self.side_events = (z0, self._side_event())
         self.build(before_tree=lambda: main.wait_stream(self.side))
         # the fields are packed beside the intersection, which reads neither
-        self.side.wait_stream(main)
-        with torch.cuda.stream(self.side):
-            self._pack()
+        packed = None
+        if self.packed is not None and self._packs["train"]:
+            self.side.wait_stream(main)
+            with torch.cuda.stream(self.side):
+                packed = self._pack("train")
         self.intersect()
-        main.wait_stream(self.side)
+        if packed is not None:
+            main.wait_stream(self.side)
         self._mark("grad_prep")
         loss_scale = 2.0 / (3.0 * self.R)
         tsdf = N.ptr(self.grad_tsdf) if self.train_tsdf else None
         if self.deterministic:
             N.check(N.lib.sg_render_packed_train_det(
-                C.byref(self.tree), C.byref(self.seg), C.byref(self.args), N.ptr(self.packed), len(self._groups),
+                C.byref(self.tree), C.byref(self.seg), C.byref(self.args), N.ptr(packed), len(self._groups),
                 self._det_groups,
                 self._det_group_S, N.ptr(self.target_rgb), loss_scale, N.ptr(self.out_rgb), N.ptr(self.out_depth),
                 N.ptr(self.out_ws), N.ptr(self.out_alpha), N.ptr(self.out_loss), N.ptr(self.grad_feat), tsdf,
@@ -416,7 +450,7 @@ class BatchPipeline:
         else:
             for seg, args in self._group_launch:
                 N.check(N.lib.sg_render_packed_train(
-                    C.byref(self.tree), C.byref(seg), C.byref(args), N.ptr(self.packed), N.ptr(self.target_rgb),
+                    C.byref(self.tree), C.byref(seg), C.byref(args), N.ptr(packed), N.ptr(self.target_rgb),
                     loss_scale,
                     N.ptr(self.out_rgb), N.ptr(self.out_depth), N.ptr(self.out_ws), N.ptr(self.out_alpha),
                     N.ptr(self.out_loss), N.ptr(self.grad_feat), tsdf, N.stream()), "render_train")
