@@ -52,17 +52,20 @@
 // 128 positions takes 217 KB of the SM); the record pass and reduction of a
 // 4.2 M-ray step 4.13 / 4.01 / 4.05 ms.  Unpacked forward (scalar taps, more
 // registers), 2^20 pixel rays of a 512^3 frame with their intersection, at 3 /
-// 4 / 5: 1.69 / 1.78 / 1.76 ms.
+// 4 / 5: 1.69 / 1.78 / 1.76 ms.  Unpacked adjoint of 16 channels (at 4 it
+// spilled), at 2 / 3 / 4, camera rays over 256^3: 1024 x 48 samples 27 / 31 / 39
+// us, 9216 x 96 44 / 58 / 74, 65536 x 64 171 / 159 / 169, 2^18 x 96 772 / 804 / 858;
+// training steps by records 2 % slower at 2 and 4 than at 3.
 #ifndef SG_RENDER_FWD_MINB
 #define SG_RENDER_FWD_MINB(PACKED) ((PACKED) ? 4 : 3)
 #endif
 #ifndef SG_RENDER_REC_MINB
-#define SG_RENDER_REC_MINB 4
+#define SG_RENDER_REC_MINB(PACKED) ((PACKED) ? 4 : 3)
 #endif
 #ifndef SG_RENDER_ADJ_MINB
-#define SG_RENDER_ADJ_MINB 4
+#define SG_RENDER_ADJ_MINB(PACKED) ((PACKED) ? 4 : 3)
 #endif
-#define SG_RENDER_MINB(MODE) ((MODE) == kModeRec ? SG_RENDER_REC_MINB : SG_RENDER_ADJ_MINB)
+#define SG_RENDER_MINB(MODE, PACKED) ((MODE) == kModeRec ? SG_RENDER_REC_MINB(PACKED) : SG_RENDER_ADJ_MINB(PACKED))
 
 namespace sg {
 
@@ -691,7 +694,7 @@ __device__ __forceinline__ void emit_records(const RenderParams &p, int b, long 
 // (kModeRec) a record needs nothing that comes after its sample, so it is
 // written as soon as the sample's weight is known and no adjoint runs.
 template <int C, int MODE, bool PACKED>
-__global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE)) render_bwd_kernel(RenderParams p) {
+__global__ void __launch_bounds__(256, SG_RENDER_MINB(MODE, PACKED)) render_bwd_kernel(RenderParams p) {
   static_assert(C == 3 || C == 16, "feature grids of 3 or 16 channels");
   constexpr bool REC = MODE == kModeRec || MODE == kModeRecTsdf;
   constexpr bool TRAIN = MODE != kModeBwd;
