@@ -257,7 +257,11 @@ __global__ void __launch_bounds__(256, 3) det_class_kernel(DetReduceParams q, in
   // apart: they take the warps unequal times (27 M samples 3.85 -> 3.73 ms a pass
   // and reduction; starting more CTAs instead cost 3 us a class on 2 M)
   const long warps = (long)gridDim.x * (blockDim.x >> 5), even = (P1 - P0 + warps - 1) / warps;
-  const long Q = max(even > 256 ? (even + 7) / 8 : even, 32l);
+  // few records: still four a warp, as a stretch is one chain of loads and sums
+  // (steps of 256 / 4096 / 9216 rays with the TSDF, at least 32 / 8 / 4 / 1: 339
+  // / 280 / 270 / 261, 402 / 324 / 314 / 310, 414 / 338 / 331 / 329 us; at 65536
+  // rays 465 / 420 / 420 / 420)
+  const long Q = max(even > 256 ? (even + 7) / 8 : even, 4l);
   long pa = P0 + (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Q;
 #pragma unroll 1
   for (; pa < P1; pa += warps * Q) {
