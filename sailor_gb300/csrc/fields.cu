@@ -179,6 +179,7 @@ struct ScatterParams {
   int mode;
   float scale, s;
   float *ggrid;        // [B, D, D, D, C], accumulated
+  int parts, part;     // a ray's samples in so many parts of so many (a multiple of 8)
 };
 
 // VEC: gradients and grid are 16-byte aligned (C a multiple of 4).
@@ -201,14 +202,24 @@ __device__ __forceinline__ void scatter_flush(const ScatterParams &p, long cell,
   for (int c = 0; c < C; c++) acc[c] = 0.0f;
 }
 
-template <int C, bool VEC>
+// PARTS: a ray's samples are walked in p.parts parts of p.part, each by lanes of
+// its own: with fewer rays than kScatterFill an SM the eight lanes' chain
+// through all samples is what the call takes.  One ray a lane group / in parts,
+// 96 samples of 16 channels: 1 ray 33 / 6 us, 500 43 / 10, 4000 45 / 28, 16384 96 / 99;
+// of one channel 500 rays 21 / 6, 16384 45 / 38.
+constexpr int kScatterFill = 128;
+
+template <int C, bool VEC, bool PARTS>
 __global__ void __launch_bounds__(256, C >= 8 ? 4 : 0) grid_scatter_kernel(ScatterParams p) {
   const int cr = lane_id() & 7;  // corner, and sample of a step of 8
   FrameGeom g;
   const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-  for (long r0 = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; r0 < p.R; r0 += nw * 4) {
-    const long r = r0 + (lane_id() >> 3);
-    const bool live = r < p.R;
+  const long n = PARTS ? p.R * p.parts : p.R;
+  for (long r0 = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; r0 < n; r0 += nw * 4) {
+    const long v = r0 + (lane_id() >> 3);
+    const bool live = v < n;
+    const long r = PARTS ? v / p.parts : v;
+    const int first = PARTS ? (int)(v - r * p.parts) * p.part : 0;  // the part's first sample
     float o[3] = {0.0f, 0.0f, 0.0f}, d[3] = {0.0f, 0.0f, 0.0f};
     if (live) {
       g.load(p.vol_bbox, p.voxel_size, (int)(r / p.N));
@@ -223,7 +234,7 @@ __global__ void __launch_bounds__(256, C >= 8 ? 4 : 0) grid_scatter_kernel(Scatt
     for (int c = 0; c < C; c++) acc[c] = 0.0f;
     long cur = 0;        // lower corner's voxel of the current run
     unsigned cur_in = 0u;
-    for (int c0 = 0; c0 < p.S; c0 += 8) {
+    for (int c0 = first; c0 < (PARTS ? first + p.part : p.S); c0 += 8) {
       // a lane per sample: cell, fractions (as the forward tap forms them) and,
       // at one channel, the gradient
       const int i = c0 + cr;
@@ -290,6 +301,28 @@ __global__ void __launch_bounds__(256, C >= 8 ? 4 : 0) grid_scatter_kernel(Scatt
       }
     }
     if (cur_in) scatter_flush<C, VEC>(p, cur, cr, cur_in, acc);
+  }
+}
+
+template <bool PARTS>
+static void launch_scatter(const ScatterParams &p, int C, sg_stream_t stream) {
+  int g = ceil_div(p.R * p.parts * 8, 256);
+  if (g > num_sms() * 32) g = num_sms() * 32;
+  const bool vec = (((uintptr_t)p.gout) | ((uintptr_t)p.ggrid)) % 16 == 0;
+  switch (C) {
+    case 1: grid_scatter_kernel<1, false, PARTS><<<g, 256, 0, stream>>>(p); break;
+    case 3: grid_scatter_kernel<3, false, PARTS><<<g, 256, 0, stream>>>(p); break;
+    case 4:
+      if (vec) grid_scatter_kernel<4, true, PARTS><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<4, false, PARTS><<<g, 256, 0, stream>>>(p);
+      break;
+    case 8:
+      if (vec) grid_scatter_kernel<8, true, PARTS><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<8, false, PARTS><<<g, 256, 0, stream>>>(p);
+      break;
+    default:
+      if (vec) grid_scatter_kernel<16, true, PARTS><<<g, 256, 0, stream>>>(p);
+      else grid_scatter_kernel<16, false, PARTS><<<g, 256, 0, stream>>>(p);
   }
 }
 
@@ -382,29 +415,17 @@ extern "C" int sg_grid_scatter(const float *ori, const float *dir, const float *
   if (B <= 0 || N <= 0 || S <= 0 || D <= 0 || C <= 0 || C > 16) return SG_ERR_INVALID_ARG;
   if (mode == 1 && (C != 1 || s == 0.0f || !grid)) return SG_ERR_INVALID_ARG;
   if (mode != 0 && mode != 1) return SG_ERR_INVALID_ARG;
+  if (C != 1 && C != 3 && C != 4 && C != 8 && C != 16) return SG_ERR_UNSUPPORTED;
   ScatterParams p{ori, dir, z, (long)B * N, N, S, grad_out, grid, D, vol_bbox, voxel_size, mode, scale, s,
-                  grad_grid};
-  long R = (long)B * N;
-  int g = ceil_div(R * 8, 256);
-  if (g > num_sms() * 32) g = num_sms() * 32;
-  const bool vec = (((uintptr_t)grad_out) | ((uintptr_t)grad_grid)) % 16 == 0;
-  switch (C) {
-    case 1: grid_scatter_kernel<1, false><<<g, 256, 0, stream>>>(p); break;
-    case 3: grid_scatter_kernel<3, false><<<g, 256, 0, stream>>>(p); break;
-    case 4:
-      if (vec) grid_scatter_kernel<4, true><<<g, 256, 0, stream>>>(p);
-      else grid_scatter_kernel<4, false><<<g, 256, 0, stream>>>(p);
-      break;
-    case 8:
-      if (vec) grid_scatter_kernel<8, true><<<g, 256, 0, stream>>>(p);
-      else grid_scatter_kernel<8, false><<<g, 256, 0, stream>>>(p);
-      break;
-    case 16:
-      if (vec) grid_scatter_kernel<16, true><<<g, 256, 0, stream>>>(p);
-      else grid_scatter_kernel<16, false><<<g, 256, 0, stream>>>(p);
-      break;
-    default: return SG_ERR_UNSUPPORTED;
+                  grad_grid, 1, 0};
+  const long R = (long)B * N, fill = (long)num_sms() * kScatterFill;
+  if (R < fill && S > 8) {
+    const int steps = (S - 1) / 8 + 1, want = (int)((fill + R - 1) / R);  // steps of 8 samples
+    p.part = ((steps - 1) / want + 1) * 8;
+    p.parts = (S - 1) / p.part + 1;
   }
+  if (p.parts > 1) launch_scatter<true>(p, C, stream);
+  else launch_scatter<false>(p, C, stream);
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
