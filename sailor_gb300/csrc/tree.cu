@@ -31,14 +31,52 @@ namespace sg {
 // ---------------------------------------------------------------------------
 // coarse occupancy
 // ---------------------------------------------------------------------------
-// A CTA per row of bricks (X, Y): a thread takes four voxels along z and walks
-// the rate^2 rows, four loads in flight; where rows are shorter than 64 such
-// threads, `groups` of them share the rows (2 x 128^3 at rate 8 33 -> 10 us,
-// 128^3 at rate 4 10.5 -> 6).  Longer rows keep one group: 4 x 256^3 45 us (6.0
-// TB/s); with four groups of threads 53 (their rows lie apart in memory).
+// A CTA per row of bricks (X, Y), a thread per four voxels along z.
+//
+// Rows of 64 such threads and more: each walks the rate^2 rows of its voxels and
+// leaves a flag a voxel (4 x 256^3 at rate 8 47 us, 5.7 TB/s; the kernel below 51,
+// and 53 with four groups: their rows lie apart in memory).
 __global__ void __launch_bounds__(256) brick_occupancy_kernel(const int *__restrict__ fine, int Df, int rate,
-                                                              int groups, FixedDiv31 by_rate, int *coarse,
-                                                              int *count) {
+                                                              int *coarse, int *count) {
+  extern __shared__ unsigned char s_any[];  // [Df]
+  const int Dc = Df / rate;
+  const int b = blockIdx.z, X = blockIdx.y, Y = blockIdx.x;
+  const size_t vf = (size_t)Df * Df * Df;
+  const int n4 = Df / 4;
+  for (int t = threadIdx.x; t < n4; t += blockDim.x) {
+    int any = 0;
+    for (int a = 0; a < rate; a++) {
+      for (int c = 0; c < rate; c++) {
+        const int4 *row =
+            reinterpret_cast<const int4 *>(fine + (size_t)b * vf + ((size_t)(X * rate + a) * Df + (Y * rate + c)) * Df);
+        const int4 q = __ldg(row + t);
+        any |= (q.x > -1) | ((q.y > -1) << 1) | ((q.z > -1) << 2) | ((q.w > -1) << 3);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++) s_any[4 * t + c] = (any >> c) & 1;
+  }
+  __syncthreads();
+  const size_t vc = (size_t)Dc * Dc * Dc;
+  int cnt = 0;
+  for (int Z = threadIdx.x; Z < Dc; Z += blockDim.x) {
+    int any = 0;
+    for (int e = 0; e < rate; e++) any |= s_any[Z * rate + e];
+    const int local = (X * Dc + Y) * Dc + Z;
+    coarse[(size_t)b * vc + local] = any ? local : -1;
+    cnt += any;
+  }
+  cnt = warp_sum(cnt);
+  if (lane_id() == 0 && cnt) atomicAdd(count + b, cnt);
+}
+
+// Shorter rows: groups of threads share the rate^2 rows, four loads in flight
+// (2 x 128^3 at rate 8 33 -> 10 us, 128^3 at rate 4 10.5 -> 6); no more groups than
+// get four rows each, but where the CTAs are few (8 x 128^3 at rate 2, eight groups
+// 63 us, one 29; 32^3 at rate 4, all 16 groups 7 us cold, four 9).
+__global__ void __launch_bounds__(256) brick_occupancy_rows_kernel(const int *__restrict__ fine, int Df, int rate,
+                                                                   int groups, FixedDiv31 by_rate, int *coarse,
+                                                                   int *count) {
   extern __shared__ unsigned char s_any[];  // [Dc]
   const int Dc = Df / rate;
   const int b = blockIdx.z, X = blockIdx.y, Y = blockIdx.x;
@@ -47,30 +85,28 @@ __global__ void __launch_bounds__(256) brick_occupancy_kernel(const int *__restr
   for (int Z = threadIdx.x; Z < Dc; Z += blockDim.x) s_any[Z] = 0;
   __syncthreads();
   const int4 *base = reinterpret_cast<const int4 *>(fine + (size_t)b * vf + ((size_t)X * rate * Df + (size_t)Y * rate) * Df);
-  const int grp = groups > 1 ? (int)threadIdx.x / n4 : 0;
+  const int grp = (int)threadIdx.x / n4, z4 = (int)threadIdx.x - grp * n4;
   if (grp < groups) {
-    for (int z4 = (int)threadIdx.x - grp * n4; z4 < n4; z4 += groups > 1 ? n4 : (int)blockDim.x) {
-      int any = 0;
-      for (int r0 = grp; r0 < rows; r0 += 4 * groups) {
-        int4 q[4];
+    int any = 0;
+    for (int r0 = grp; r0 < rows; r0 += 4 * groups) {
+      int4 q[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const int row = r0 + k * groups;
-          q[k] = make_int4(-1, -1, -1, -1);
-          if (row < rows) {
-            const int a = (int)by_rate.div((uint32_t)row);
-            q[k] = __ldg(base + ((size_t)a * Df + (row - a * rate)) * n4 + z4);
-          }
+      for (int k = 0; k < 4; k++) {
+        const int row = r0 + k * groups;
+        q[k] = make_int4(-1, -1, -1, -1);
+        if (row < rows) {
+          const int a = (int)by_rate.div((uint32_t)row);
+          q[k] = __ldg(base + ((size_t)a * Df + (row - a * rate)) * n4 + z4);
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-          any |= (q[k].x > -1) | ((q[k].y > -1) << 1) | ((q[k].z > -1) << 2) | ((q[k].w > -1) << 3);
       }
-      if (any) {  // the same value whoever stores it
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-          if ((any >> c) & 1) s_any[by_rate.div((uint32_t)(4 * z4 + c))] = 1;
-      }
+      for (int k = 0; k < 4; k++)
+        any |= (q[k].x > -1) | ((q[k].y > -1) << 1) | ((q[k].z > -1) << 2) | ((q[k].w > -1) << 3);
+    }
+    if (any) {  // the same value whoever stores it
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        if ((any >> c) & 1) s_any[by_rate.div((uint32_t)(4 * z4 + c))] = 1;
     }
   }
   __syncthreads();
@@ -381,10 +417,18 @@ extern "C" int sg_brick_occupancy(const int *occ_fine, int B, int Df, int rate, 
   if (B <= 0 || rate <= 0 || Df <= 0 || Df % rate != 0 || Df % 4 != 0) return SG_ERR_INVALID_ARG;
   if (((uintptr_t)occ_fine) % 16 != 0) return SG_ERR_INVALID_ARG;
   int Dc = Df / rate;
-  const int n4 = Df / 4, groups = n4 < 64 ? 256 / n4 : 1;
-  const int threads = groups > 1 ? 256 : (n4 < 256 ? (n4 + 31) / 32 * 32 : 256);
-  brick_occupancy_kernel<<<dim3(Dc, Dc, B), threads, Dc, stream>>>(occ_fine, Df, rate, groups,
-                                                                   FixedDiv31::of((uint32_t)rate), occ_coarse, count);
+  const int n4 = Df / 4, rows = rate * rate;
+  if (n4 >= 64) {
+    const int threads = n4 < 256 ? (n4 + 31) / 32 * 32 : 256;
+    brick_occupancy_kernel<<<dim3(Dc, Dc, B), threads, Df, stream>>>(occ_fine, Df, rate, occ_coarse, count);
+  } else {
+    const int each = (long)Dc * Dc * B > 2l * num_sms() ? 4 : 1;  // rows a group at least
+    int groups = 256 / n4;
+    if (groups > (rows + each - 1) / each) groups = (rows + each - 1) / each;
+    const int threads = (groups * n4 + 31) / 32 * 32;
+    brick_occupancy_rows_kernel<<<dim3(Dc, Dc, B), threads, Dc, stream>>>(occ_fine, Df, rate, groups,
+                                                                         FixedDiv31::of((uint32_t)rate), occ_coarse, count);
+  }
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
