@@ -328,23 +328,26 @@ static void launch_scatter(const ScatterParams &p, int C, sg_stream_t stream) {
 
 // Zero of the part of a gradient grid [B, Db, Db, Db, C] (the tree's fine
 // geometry) that a training pass over the tree's nodes can write: a CTA takes
-// 16 top bricks, a thread each tests its brick's 26-neighbourhood for a node,
-// and all threads clear the bricks found, rate^3 voxels each (rate^2 z-runs of
-// rate * C floats).  Few bricks are near a node, so a CTA per brick was bound by
-// starting CTAs: 4 x 32^3 bricks of 8^3 voxels of 16 channels 182 -> 83 us,
-// 2 x 16^3 bricks 30 -> 22 us.
+// BRICKS top bricks, a thread each tests its brick's 26-neighbourhood
+// for a node, and all threads clear the bricks found, rate^3 voxels each (rate^2
+// z-runs of rate * C floats).  Few bricks are near a node, so a CTA per brick was
+// bound by starting CTAs: 4 x 32^3 bricks of 8^3 voxels of 16 channels 182 -> 83
+// us, 2 x 16^3 bricks 30 -> 22 us (16).  One brick a CTA where 16 would leave SMs
+// without one (8^3 bricks, a quarter of them near nodes: 16 14 us, one 8).  A
+// compile-time count: as an argument it took 1.2 to 1.9 times as long.
 constexpr int kZeroBricks = 16;
 
+template <int BRICKS>
 __global__ void __launch_bounds__(256) zero_near_nodes_kernel(SgTree t, float *grid, int C, int vec4, FixedDiv31 by_brick,
                                                               FixedDiv31 by_run, FixedDiv31 by_rate) {
-  __shared__ int2 s_near[kZeroBricks];
+  __shared__ int2 s_near[BRICKS];
   __shared__ int s_n;
   const int b = blockIdx.y, Dt = t.Dt;
   const int vt = Dt * Dt * Dt;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
-  const int own = (int)blockIdx.x * kZeroBricks + (int)threadIdx.x;
-  if (threadIdx.x < kZeroBricks && own < vt) {
+  const int own = (int)blockIdx.x * BRICKS + (int)threadIdx.x;
+  if (threadIdx.x < BRICKS && own < vt) {
     const int Z = own % Dt, xy = own / Dt, Y = xy % Dt, X = xy / Dt;
     const int *node = t.brick_node + (long)b * vt;
     bool near = false;
@@ -438,9 +441,14 @@ extern "C" int sg_zero_near_nodes(const SgTree *tree, float *grid, int C, sg_str
   if (vt > INT_MAX || tree->B > 65535) return SG_ERR_UNSUPPORTED;
   const int vec4 = ((tree->rate * C) % 4 == 0 && ((uintptr_t)grid) % 16 == 0) ? 1 : 0;
   const int per_run = vec4 ? tree->rate * C / 4 : tree->rate * C;
-  zero_near_nodes_kernel<<<dim3((unsigned)ceil_div(vt, kZeroBricks), tree->B), 256, 0, stream>>>(
-      *tree, grid, C, vec4, FixedDiv31::of((uint32_t)(tree->rate * tree->rate * per_run)), FixedDiv31::of((uint32_t)per_run),
-      FixedDiv31::of((uint32_t)tree->rate));
+  const FixedDiv31 by_brick = FixedDiv31::of((uint32_t)(tree->rate * tree->rate * per_run)),
+                   by_run = FixedDiv31::of((uint32_t)per_run), by_rate = FixedDiv31::of((uint32_t)tree->rate);
+  if (vt * tree->B >= (long)num_sms() * kZeroBricks)
+    zero_near_nodes_kernel<kZeroBricks><<<dim3((unsigned)ceil_div(vt, kZeroBricks), tree->B), 256, 0, stream>>>(
+        *tree, grid, C, vec4, by_brick, by_run, by_rate);
+  else
+    zero_near_nodes_kernel<1><<<dim3((unsigned)vt, tree->B), 256, 0, stream>>>(*tree, grid, C, vec4, by_brick, by_run,
+                                                                               by_rate);
   SG_LAUNCH_CHECK();
   return SG_OK;
 }
