@@ -455,6 +455,12 @@ __global__ void __launch_bounds__(512) intersect_padded_kernel(IsectParams p) {
   intersect_rays<RATE, true>(p);
 }
 
+// Rays from which the walking warps pad their rows themselves: the few warps of
+// fewer rays would write them one row after another, where a second kernel has a
+// warp a row (64 rows of 1024: 18 us by the walking warps, 12 by two kernels; 200
+// rows 20 and 18; 256 and more the walking warps).
+constexpr long kPadInWalk = 256;
+
 template <bool PAD>
 static void launch_intersect(const IsectParams &p, sg_stream_t stream) {
   const int blk = tune(SG_TUNE_ISECT_BLOCK);
@@ -725,10 +731,11 @@ extern "C" int sg_intersect(const SgTree *tree, const float *ori, const float *d
   if (tune(SG_TUNE_ISECT_WARP)) {
     intersect_warp_kernel<<<ceil_div(R, 256), 256, 0, stream>>>(p);
     if (padded) launch_pad_rows(R, W, hit_count, hit_idx, hit_t0, hit_t1, stream);
-  } else if (padded) {
+  } else if (padded && R >= kPadInWalk) {
     launch_intersect<true>(p, stream);
   } else {
     launch_intersect<false>(p, stream);
+    if (padded) launch_pad_rows(R, W, hit_count, hit_idx, hit_t0, hit_t1, stream);
   }
   SG_LAUNCH_CHECK();
   return SG_OK;
