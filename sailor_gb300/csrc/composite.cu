@@ -66,21 +66,25 @@ struct CompWalk {
 
 // Depths of the sorted positions into shared memory; false for an invalid ray.
 template <bool ONE>
-__device__ __forceinline__ bool comp_load(const CompParams &p, size_t rb, float *s_z) {
+__device__ __forceinline__ bool comp_load(const CompParams &p, size_t rb, float *s_z, int *s_i) {
   const int lane = lane_id(), S = p.S;
   const int last = p.sort_idx ? __ldg(p.sort_idx + rb + S - 1) : S - 1;
   if (__ldg(p.z + rb + last) < 0) return false;
   if (ONE) {
     if (lane < S) s_z[lane] = __ldg(p.z + rb + (p.sort_idx ? __ldg(p.sort_idx + rb + lane) : lane));
   } else {
-    for (int i = lane; i < S; i += 32) s_z[i] = __ldg(p.z + rb + (p.sort_idx ? __ldg(p.sort_idx + rb + i) : i));
+    for (int i = lane; i < S; i += 32) {
+      const int s = p.sort_idx ? __ldg(p.sort_idx + rb + i) : i;
+      s_i[i] = s;
+      s_z[i] = __ldg(p.z + rb + s);
+    }
   }
   __syncwarp();
   return true;
 }
 
 template <bool ONE>
-__device__ __forceinline__ bool comp_block(const CompParams &p, size_t rb, int e, const float *s_z, float *s_f,
+__device__ __forceinline__ bool comp_block(const CompParams &p, size_t rb, int e, const float *s_z, const int *s_i, float *s_f,
                                            CompWalk &wk, CompBlock &v) {
   const int lane = lane_id(), i = e * 32 + lane, S = p.S;
   v.z = i < S ? s_z[i] : -1.0f;
@@ -89,7 +93,7 @@ __device__ __forceinline__ bool comp_block(const CompParams &p, size_t rb, int e
   v.used = v.post = false;
   const bool valid = v.z >= 0.0f;
   const unsigned vb = __ballot_sync(SG_FULL, valid);
-  if (i < S) v.s = p.sort_idx ? __ldg(p.sort_idx + rb + i) : i;
+  if (i < S) v.s = ONE ? (p.sort_idx ? __ldg(p.sort_idx + rb + i) : i) : s_i[i];
   if (vb == 0u) return false;
   if (wk.m0 < 0) wk.m0 = e * 32 + __ffs(vb) - 1;
   if (valid) {
@@ -149,10 +153,12 @@ constexpr int kAhead = 4;     // row loads in flight a lane
 template <int V, bool OPT>
 __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
   __shared__ float s_zall[8][kMaxPos];
+  __shared__ int s_iall[8][V == 0 && OPT ? 1 : kMaxPos];
   __shared__ __align__(16) float s_fall[8][64];
   const int lane = lane_id();
   float *s_z = s_zall[threadIdx.x >> 5];
   float *s_f = s_fall[threadIdx.x >> 5];
+  int *s_i = s_iall[threadIdx.x >> 5];
   const int C = p.C, S = p.S;
   constexpr int N = V ? V : 3;
   constexpr bool ONE = V == 0 && OPT, LONG = V > 0 && OPT;
@@ -165,13 +171,13 @@ __global__ void __launch_bounds__(256, 6) composite_fwd_kernel(CompParams p) {
 #pragma unroll
     for (int c = 0; c < N; c++) acc[c] = 0.0f;
     float d = 0.0f, ws = 0.0f, aa = 0.0f;
-    const bool ok = comp_load<ONE>(p, rb, s_z);
+    const bool ok = comp_load<ONE>(p, rb, s_z, s_i);
     if (ok) {
       CompWalk wk{1.0f, -1, S};
 #pragma unroll 1
       for (int e = 0; ONE ? e < 1 : e * 32 < wk.end; e++) {
         CompBlock v;
-        if (!comp_block<ONE>(p, rb, e, s_z, s_f, wk, v)) continue;
+        if (!comp_block<ONE>(p, rb, e, s_z, s_i, s_f, wk, v)) continue;
         if (v.used) {
           d += v.w * v.z;
           ws += v.w;
@@ -278,7 +284,7 @@ __global__ void __launch_bounds__(256, 5) composite_bwd_kernel(CompParams p) {
 #pragma unroll
     for (int c = 0; c < N; c++) gc[c] = (V ? own : c < C) ? __ldg(p.g_feat + (size_t)r * C + c0 + c) : 0.0f;
     const float gws = __ldg(p.g_ws + r), gd = __ldg(p.g_depth + r), ga = __ldg(p.g_alpha + r);
-    const bool ok = comp_load<false>(p, rb, s_z);  // an invalid ray has no gradient (the reference leaves its zero fill)
+    const bool ok = comp_load<false>(p, rb, s_z, kp.idx);  // an invalid ray has no gradient (the reference leaves its zero fill)
     // totals over the samples: w s, w z, w, w alpha
     float Fs = 0.0f, Fd = 0.0f, Fw = 0.0f, Fa = 0.0f;
     if (ok) {
@@ -287,7 +293,7 @@ __global__ void __launch_bounds__(256, 5) composite_bwd_kernel(CompParams p) {
       for (; e1 * 32 < wk.end; e1++) {
         CompBlock v;
         const int i = e1 * 32 + lane;
-        const bool any = comp_block<false>(p, rb, e1, s_z, s_f, wk, v);
+        const bool any = comp_block<false>(p, rb, e1, s_z, kp.idx, s_f, wk, v);
         float sv = 0.0f;  // g . features of the lane's sample
         if (any) {
           if constexpr (V == 0) {
