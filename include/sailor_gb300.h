@@ -499,7 +499,9 @@ int sg_project_gather(const SgProjGather *args, sg_stream_t stream);
 
 /* A map [n,C,H,W] read through its element strides (4, host) into dst
  * [n,H,W,C]: sg_project_gather reads channels-last maps in whole texel rows,
- * which pays from about a quarter as many points per image as pixels. */
+ * which pays from max(1/2, 16 / C) points per pixel on, C > 5.  2^31 pixels or
+ * more than 32 * 65535 channels: SG_ERR_UNSUPPORTED (sg_project_gather reads such
+ * maps through their strides). */
 int sg_channels_last(const float *src, const long long *stride, int n, int C, int H,
                      int W, float *dst, sg_stream_t stream);
 
@@ -727,9 +729,10 @@ size_t sg_train_det_workspace_bytes(long long R, int nseg, int C, long long capa
  * trilinear cell -- the cell, and per corner the sum of corner weight x
  * compositing weight (and x TSDF gradient) -- plus, per ray, head^T times its
  * colour gradient; the records are sorted by cell (a
- * stable radix sort), and each cell's run is summed in order and added to
- * its 8 corners, one parity class of cells at a time (cells of a class
- * share no corner).  The sums are added (+=) into grad_feat [B,Df,Df,Df,C]
+ * stable radix sort), and each cell's run is summed in a fixed order (four
+ * sums of every fourth record in ray order, added in pairs: the cell's own
+ * records alone decide its bits) and added to its 8 corners, one parity class of
+ * cells at a time (cells of a class share no corner).  The sums are added (+=) into grad_feat [B,Df,Df,Df,C]
  * and grad_tsdf [B,D,D,D] (may be NULL; needs the feature grid on the TSDF
  * grid's geometry).  groups: ngroups + 1 host ints, the segment index where
  * each group of the table starts (one launch of the pass per group, sized

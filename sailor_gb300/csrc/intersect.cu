@@ -14,8 +14,9 @@
 // the ray's own thread the occupied children the ray can reach; the
 // warp-cooperative variant (intersect_warp_kernel, tune knob
 // SG_TUNE_ISECT_WARP) tests every occupied child of a hit brick with the
-// whole warp, one brick at a time -- the same rows, but measured about 8x
-// slower at 8^3 bricks, where the reach test leaves ~1/5 of the children.  Hits
+// whole warp, one brick at a time -- the same rows, but measured 17x slower
+// (28 against 1.6 ms, the bench's 7.4 M rays), where the reach test leaves ~1/5
+// of the children: the tests' second opinion.  Hits
 // are appended to the ray's row; the reference's -1 padding of the row tail
 // is written by the same warps with bulk copies out of shared memory once
 // their rays are done (by a second kernel under the other variant).

@@ -49,7 +49,7 @@
 // Measured at 3 / 4 / 5 for the forward and the record pass and 2 / 3 / 4 for
 // the adjoint, packed taps: 2^20 random rays of 96 samples, forward 1.46 /
 // 1.27 / 1.40 ms, adjoint 5.67 / 5.35 / 5.22 ms (at 4 the shared memory of
-// 128 positions takes 217 KB of the SM); the record pass and reduction of a
+// 128 positions takes 196 KB of the SM); the record pass and reduction of a
 // 4.2 M-ray step 4.13 / 4.01 / 4.05 ms.  Unpacked forward (scalar taps, more
 // registers), 2^20 pixel rays of a 512^3 frame with their intersection, at 3 /
 // 4 / 5: 1.69 / 1.78 / 1.76 ms.  Unpacked adjoint of 16 channels (at 4 it
@@ -454,12 +454,13 @@ __device__ __forceinline__ int sample_and_sort(const RenderParams &p, long r, in
 extern __shared__ __align__(16) float s_render[];
 
 // The rays of a CTA are eight consecutive ones, and the same a grid apart: warp
-// w takes the w-th of each eight, or, where rays may miss, the warps take them
-// one by one (take_ray), so that a ray that misses or ends early leaves its warp
-// free for the next.  2^20 random rays, a third of them hitting, one by one /
-// fixed: forward 1.19 / 1.27 ms, adjoint 4.30 / 4.94; rays that all hit (record
-// pass) 3.91 / 3.85 with the reduction, pixel rays of an unpacked frame 1.70 /
-// 1.68 (with their intersection): fixed there.
+// w takes the w-th of each eight, or the warps take them one by one (take_ray), so
+// that a ray that misses or ends early leaves its warp free for the next.  One by
+// one in the packed forward and in the adjoints: 2^20 random rays, a third of them
+// hitting, one by one / fixed, forward 1.19 / 1.27 ms, adjoint 4.30 / 4.94.  Fixed
+// in the record pass, whose rays all hit (3.91 / 3.85 with the reduction), and in
+// the unpacked forward (pixel rays of a frame, with their intersection, 1.70 /
+// 1.68: no gain).
 __device__ __forceinline__ long take_ray(int &taken, long first) {
   int i = 0;
   if (lane_id() == 0) i = atomicAdd(&taken, 1);

@@ -19,8 +19,10 @@
 //      sorted sample order -- fixed by the ray layout);
 //   2. run heads are flagged and scanned into the list of distinct cells;
 //   3. for each of the 8 parity classes in turn, each cell's run is summed in
-//      a fixed order into the 8 corners x C channels it touches, and the sums
-//      are added into the grids.  Cells of one class share no corner, so every
+//      a fixed order into the 8 corners x C channels it touches (four sums of
+//      every fourth record, added in pairs: which of the four takes a record
+//      depends on its place in the warp's stretch, the four sets and the pairs do
+//      not), and the sums are added into the grids.  Cells of one class share no corner, so every
 //      grid value gets one addition per class, classes in a fixed order.
 // Every grid value is therefore the same sum in the same order on every run:
 // the gradients are bit-identical across runs, launch shapes and graph
