@@ -499,7 +499,7 @@ int sg_project_gather(const SgProjGather *args, sg_stream_t stream);
 
 /* A map [n,C,H,W] read through its element strides (4, host) into dst
  * [n,H,W,C]: sg_project_gather reads channels-last maps in whole texel rows,
- * which pays from max(1/2, 16 / C) points per pixel on, C > 5.  2^31 pixels or
+ * which pays from about max(0.4, 8 / C) points per pixel on.  2^31 pixels or
  * more than 32 * 65535 channels: SG_ERR_UNSUPPORTED (sg_project_gather reads such
  * maps through their strides). */
 int sg_channels_last(const float *src, const long long *stride, int n, int C, int H,

@@ -47,26 +47,28 @@ def _cams(K, R, T, n_images):
 # A thread per item walks the channels of a map that is not channels-last
 # through scattered 4-byte loads, near points sharing them; rows of a
 # channels-last map are read whole.  Rewriting costs a pass over the map and
-# about 10 us of calls, so it is done where the points outnumber
-# CHANNELS_LAST_FROM of the pixels by more the fewer channels there are
-# (C > 5 only), and the output is large enough to hide the calls.  Measured,
-# direct against rewritten, on samples along rays / on a raster of neighbouring
-# pixels, 4 images of 512^2:
-#   C   8: 1 point a pixel 160 and 160 /  66 and  87 us;  2: 309 and 214 / -
+# about 10 us of calls, so it is done from CHANNELS_LAST_FROM points a pixel on,
+# more with few channels (8 / C; 3 below 8, never below 6), and where the output
+# is large enough to hide the calls.  Measured, direct against rewritten, on
+# samples along rays (two maps a call) / on a raster of neighbouring pixels, 4
+# images of 512^2, us:
+#   C   8: 1 point a pixel 160 and 160 /  66 and  87;  2: 309 and 214 / -
 #   C  16: 0.5             178 and 172 /  63 and  95;     1: 329 and 207 / 105 and 117
 #   C  32: 0.25            235 and 221 /  79 and 128;   0.5: 426 and 245 / 148 and 143
 #   C  68: 0.25            419 and 532 / 187 and 290;   0.5: 788 and 588 / 323 and 318
 #   C   5: 5 points a pixel 439 and 469; C 6: 2: 213 and 237, 3: 316 and 304
-# and, where the calls count, one image of 512^2, C 16: 0.5 (2^21 values) 50 and
-# 66 us, 1 (2^22) 87 and 65.  (Samples along rays: two such maps a call.)
-CHANNELS_LAST_FROM = 0.5
+# (the raster of few channels is what rewriting loses on, by less than the direct
+# walk has gained there) and, where the calls count, one image of 512^2, C 16: 0.5
+# (2^21 values) 50 and 66, 1 (2^22) 87 and 65.
+CHANNELS_LAST_FROM = 0.4
 CHANNELS_LAST_WORK = 1 << 22
 
 
 def _rewrites(n, Cm, pixels, N_pts):
     """Whether n maps of Cm channels, not channels-last, are rewritten for N_pts points each."""
-    return (Cm > 5 and N_pts >= CHANNELS_LAST_FROM * pixels * max(1.0, 32.0 / Cm)
-            and n * N_pts * Cm >= CHANNELS_LAST_WORK)
+    if Cm < 6 or n * N_pts * Cm < CHANNELS_LAST_WORK:
+        return False
+    return N_pts >= CHANNELS_LAST_FROM * pixels * (max(1.0, 20.0 / Cm) if Cm >= 8 else 7.5)
 
 
 def _channels_last(img):
