@@ -94,13 +94,20 @@ def _maps(a, imgs, N_pts):
         if img.dim() != 4:
             raise RuntimeError("feature maps must be [n_images, C, H, W]")
         _f32(img, "feature map")
-    # before any copy of a map, which can be done without
-    outs = [torch.empty((img.shape[0], N_pts, img.shape[1]), device=img.device) for img in imgs]
-    keep = []
+    try:
+        return _fill_maps(a, imgs, N_pts, True)
+    except torch.OutOfMemoryError:
+        pass
+    return _fill_maps(a, imgs, N_pts, False)  # the copies of maps before an output that had no room are gone
+
+
+def _fill_maps(a, imgs, N_pts, rewrite):
+    outs, keep = [], []
     for i, img in enumerate(imgs):
         n, Cm, H, W = img.shape
+        out = torch.empty((n, N_pts, Cm), device=img.device)
         src, strides = img, img.stride()
-        if img.stride(1) != 1 and _rewrites(n, Cm, H * W, N_pts):
+        if rewrite and img.stride(1) != 1 and _rewrites(n, Cm, H * W, N_pts):
             rows = _channels_last(img)
             if rows is not None:
                 src, strides = rows, (H * W * Cm, 1, W * Cm, Cm)
@@ -109,10 +116,11 @@ def _maps(a, imgs, N_pts):
         for k in range(4):
             m.stride[k] = strides[k]
         m.C, m.H, m.W = Cm, H, W
-        m.out = outs[i].data_ptr()
-        keep.append(src)
+        m.out = out.data_ptr()
+        outs.append(out)
+        keep += [img, src]
     a.n_maps = len(imgs)
-    return outs, keep + list(imgs)
+    return outs, keep
 
 
 def _launch(a, keep):

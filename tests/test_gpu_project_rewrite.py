@@ -53,3 +53,27 @@ def test_no_room_for_a_copy(monkeypatch):
         got = views.forward_sample_feature(*args)
     for a, b in zip(got, ref):
         assert torch.equal(a, b)
+
+
+def test_no_room_for_an_output_beside_the_copies(monkeypatch):
+    """The third map's output has no room while the first map's copy is held."""
+    from sailor_gb300 import views
+    n, C, H, W = 2, 64, 48, 40
+    args = _args(n, C, H, W, H * W, 1)
+    monkeypatch.setattr(views, "CHANNELS_LAST_FROM", 0.0)
+    monkeypatch.setattr(views, "CHANNELS_LAST_WORK", 0)
+    ref, real, copies = views.forward_sample_feature(*args), torch.empty, []
+
+    def full(shape, *a, **k):
+        if shape == (n, H, W, C):
+            copies.append(shape)
+        if shape == (n, H * W, 3) and len(copies) == 1:
+            copies.append("refused")
+            raise torch.OutOfMemoryError("no room")
+        return real(shape, *a, **k)
+    with monkeypatch.context() as mp:
+        mp.setattr(torch, "empty", full)
+        got = views.forward_sample_feature(*args)
+    assert copies == [(n, H, W, C), "refused"]  # and no copy the second time
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)
