@@ -18,8 +18,11 @@
 
 namespace sg {
 
+// Both wait on the hits and the jitter, so registers for six CTAs an SM: left to the
+// compiler (61 registers, four CTAs) 131072 rays x 96 samples took 76 us, at 5 / 6 /
+// 7 CTAs 67 / 61 / 62; with the sort 110 us, 103 / 101 / 121.
 template <int E>
-__global__ void __launch_bounds__(256) sample_coarse_kernel(SampleParams p) {
+__global__ void __launch_bounds__(256, 6) sample_coarse_kernel(SampleParams p) {
   __shared__ float s_z[8][32 * E];
   __shared__ int s_i[8][32 * E];
   const int lane = lane_id(), w8 = threadIdx.x >> 5;
@@ -113,7 +116,7 @@ __global__ void __launch_bounds__(256) sort_rows_kernel(const float *__restrict_
 // node ids are written (8 bytes per sample, one coalesced pass).  Hit rows
 // may be compact (hit_count given) or -1 terminated (hit_count NULL).
 template <int E>
-__global__ void __launch_bounds__(256) sample_sorted_kernel(SampleParams p, const int *__restrict__ hit_count,
+__global__ void __launch_bounds__(256, 6) sample_sorted_kernel(SampleParams p, const int *__restrict__ hit_count,
                                                             float rand_const, float *out_z, int *out_idx) {
   __shared__ __align__(16) float s_z[8][32 * E];
   __shared__ int s_i[8][32 * E];
