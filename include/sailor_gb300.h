@@ -272,7 +272,8 @@ int sg_octree_nodes(const SgOctree *tree, int n_nodes, float *out,
  * order, each coarse node's entries in descent order, and neither limit
  * exists.  Rows wider than Wc / Wf keep their first entries and set
  * SG_FLAG_HIT_OVERFLOW; status->max_coarse / max_fine receive the largest
- * counts.  cnt_c / cnt_f [B,N] (nullable) receive the row counts. */
+ * counts.  cnt_c / cnt [B,N] receive the row counts (required: the rows'
+ * padding reads them). */
 int sg_octree_traversal(const SgOctree *tree, const float *ori,
                         const float *dir, int N, int start_level, int Wc,
                         int Wf, int th_early_stop, int opt_num, int *idx_c,
